@@ -114,7 +114,7 @@ def build_reference_checker(ref: Optional[str] = None) -> bool:
     GISSPA_REFERENCE environment variable) into oracle/_ref (test
     infrastructure) when they are present on this machine."""
     ref = ref or os.environ.get("GISSPA_REFERENCE")
-    if not ref or not os.path.isdir(ref):
+    if not ref or not os.path.isfile(os.path.join(ref, "main.cu")):
         return False
     _run(["make", "-C", os.path.join(ROOT, "oracle"), "ref", "ref-default", "REF=" + ref])
     return True
