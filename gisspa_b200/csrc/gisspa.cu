@@ -14,6 +14,7 @@
 #include "tccorr.cuh"
 #include "tccorr2.cuh"
 #include "refine.cuh"
+#include "seqsum.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -1060,20 +1061,22 @@ static int prep_micrograph(gs_ctx* ctx, const MicPlan& mp, float2* W) {
         d_mic = P<float>(ctx->in);
     }
     // ---- micrograph: init_d_image (main.cu:523-586) ----
-    TRY(ensure(ctx, ctx->q, sizeof(float) * 2 * npix));
+    const long long npix4 = (npix + 3) / 4 * 4;  // both quotient arrays 16-byte aligned
+    TRY(ensure(ctx, ctx->q, sizeof(float) * 2 * npix4));
     TRY(ensure(ctx, ctx->cimg, sizeof(float2) * npix));
     TRY(ensure(ctx, ctx->img, sizeof(float) * npix));
-    TRY(ensure(ctx, ctx->stats, sizeof(MicStats)));
+    TRY(ensure(ctx, ctx->stats, sizeof(float) * 2));
     const int ns = std::max(nx, ny) / 2;
     TRY(ensure(ctx, ctx->ra, sizeof(double) * ns));
     TRY(ensure(ctx, ctx->rb, sizeof(unsigned) * ns));
     float* q1 = P<float>(ctx->q);
-    float* q2 = q1 + npix;
+    float* q2 = q1 + npix4;
     k_mic_quot<<<blocks_for(npix, 256), 256, 0, ctx->stream>>>(d_mic, npix, nx, ny, q1, q2);
     ++ctx->counters.kernel_launches;
-    k_mic_seq<<<1, 1024, 0, ctx->stream>>>(q1, q2, npix, P<MicStats>(ctx->stats));
+    CK(cudaFuncSetAttribute(k_seq_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmem));
+    k_seq_sums<<<2, kSeqThreads, kSeqSmem, ctx->stream>>>(q1, npix4, npix, P<float>(ctx->stats));
     ++ctx->counters.kernel_launches;
-    k_mic_clamp<<<blocks_for(npix, 256), 256, 0, ctx->stream>>>(d_mic, npix, P<MicStats>(ctx->stats), p.invert,
+    k_mic_clamp<<<blocks_for(npix, 256), 256, 0, ctx->stream>>>(d_mic, npix, P<float>(ctx->stats), p.invert,
                                                                  P<float2>(ctx->cimg));
     ++ctx->counters.kernel_launches;
     CKL();

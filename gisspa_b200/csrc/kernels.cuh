@@ -203,76 +203,28 @@ __global__ void k_mic_quot(const float* __restrict__ img, long long n, int nx, i
     q2[i] = __fdiv_rn(__fdiv_rn(__fmul_rn(v, v), (float)nx), (float)ny);
 }
 
-// The two float32 running sums of main.cu:530-535 in their exact sequential
-// order (float addition is not associative, and the reference's clamp bounds
-// are integers cut from these sums, main.cu:536-543).  One CTA: thread 0 adds
-// the terms in order from a shared-memory chunk while warps 1.. stage the
-// next chunk (double buffer); the two sums are independent chains, so the
-// loop runs at about one add latency per term.
-constexpr int kSeqChunk = 2048;
-__global__ void __launch_bounds__(1024) k_mic_seq(const float* __restrict__ q1, const float* __restrict__ q2,
-                                                  long long n, MicStats* __restrict__ out) {
-    __shared__ __align__(16) float b1[2][kSeqChunk];
-    __shared__ __align__(16) float b2[2][kSeqChunk];
-    const int tid = threadIdx.x;
-    float s1 = 0.0f, s2 = 0.0f;
-    // stage chunk 0
-    for (int i = tid; i < kSeqChunk; i += blockDim.x) {
-        const long long g = i;
-        b1[0][i] = g < n ? q1[g] : 0.0f;
-        b2[0][i] = g < n ? q2[g] : 0.0f;
-    }
-    int buf = 0;
-    for (long long base = 0; base < n; base += kSeqChunk) {
-        __syncthreads();  // chunk `buf` is staged; chunk buf^1 is free
-        if (tid == 0) {
-            const int cnt = (int)min((long long)kSeqChunk, n - base);
-            const float4* v1 = reinterpret_cast<const float4*>(b1[buf]);
-            const float4* v2 = reinterpret_cast<const float4*>(b2[buf]);
-            int i = 0;
-            for (; i + 4 <= cnt; i += 4) {
-                const float4 a = v1[i >> 2], c = v2[i >> 2];
-                s1 = __fadd_rn(s1, a.x); s2 = __fadd_rn(s2, c.x);
-                s1 = __fadd_rn(s1, a.y); s2 = __fadd_rn(s2, c.y);
-                s1 = __fadd_rn(s1, a.z); s2 = __fadd_rn(s2, c.z);
-                s1 = __fadd_rn(s1, a.w); s2 = __fadd_rn(s2, c.w);
-            }
-            for (; i < cnt; ++i) {
-                s1 = __fadd_rn(s1, b1[buf][i]);
-                s2 = __fadd_rn(s2, b2[buf][i]);
-            }
-        } else if (tid >= 32) {
-            const long long nb = base + kSeqChunk;
-            for (int i = tid - 32; i < kSeqChunk; i += blockDim.x - 32) {
-                const long long g = nb + i;
-                b1[buf ^ 1][i] = g < n ? q1[g] : 0.0f;
-                b2[buf ^ 1][i] = g < n ? q2[g] : 0.0f;
-            }
-        }
-        buf ^= 1;
-    }
-    if (tid == 0) {
-        const float avg = s1;
-        const float aa = __fmul_rn(avg, avg);
-        const float var = __fsqrt_rn(__fsub_rn(s2, aa));
-        const float six = __fmul_rn(6.0f, var);
-        MicStats st;
-        st.avg = avg;
-        st.up = isnan(var) ? 0 : (int)__fadd_rn(avg, six);
-        st.low = isnan(var) ? 0 : (int)__fsub_rn(avg, six);
-        st.enabled = s2 > aa ? 1 : 0;
-        *out = st;
-    }
+// Clamp bounds from the two running sums (seqsum.cuh): main.cu:536-543.
+__device__ __forceinline__ MicStats mic_stats(float s1, float s2) {
+    const float avg = s1;
+    const float aa = __fmul_rn(avg, avg);
+    const float var = __fsqrt_rn(__fsub_rn(s2, aa));
+    const float six = __fmul_rn(6.0f, var);
+    MicStats st;
+    st.avg = avg;
+    st.up = isnan(var) ? 0 : (int)__fadd_rn(avg, six);
+    st.low = isnan(var) ? 0 : (int)__fsub_rn(avg, six);
+    st.enabled = s2 > aa ? 1 : 0;
+    return st;
 }
 
 // Hot-pixel clamp to the mean, optional inversion, real -> complex.
 // Reference: init_d_image host loops + float2Complex (main.cu:541-551).
-__global__ void k_mic_clamp(const float* __restrict__ img, long long n, const MicStats* __restrict__ st, int invert,
+__global__ void k_mic_clamp(const float* __restrict__ img, long long n, const float* __restrict__ sums, int invert,
                             float2* __restrict__ out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float v = img[i];
-    const MicStats s = *st;
+    const MicStats s = mic_stats(sums[0], sums[1]);
     if (s.enabled && (v > (float)s.up || v < (float)s.low)) v = s.avg;
     if (invert == 1) v = -v;
     out[i] = make_float2(v, 0.0f);
