@@ -16,6 +16,7 @@ import glob
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from typing import Optional
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -26,6 +27,8 @@ INCLUDE = os.path.join(ROOT, "include")
 LIB = os.path.join(LIBDIR, "libgisspa_b200.so")
 DRIVER = os.path.join(LIBDIR, "gisspa_main")
 MERGE = os.path.join(LIBDIR, "gisspa_merge")
+
+WIN_PARTS = 8  # win_ops in gisspa.cu names as many
 
 NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -46,16 +49,25 @@ def _run(cmd, cwd=None) -> None:
 
 def build_library(force: bool = False) -> str:
     srcs = sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))
-                  + glob.glob(os.path.join(CSRC, "*.cpp"))
+                  + glob.glob(os.path.join(CSRC, "*.cpp")) + glob.glob(os.path.join(CSRC, "*.hpp"))
                   + [os.path.join(INCLUDE, "gisspa.h")])
     if not force and _newer(LIB, srcs):
         return LIB
-    os.makedirs(LIBDIR, exist_ok=True)
-    _run([NVCC] + NVCC_FLAGS + ARCH + ["-shared", "-I" + INCLUDE, "-o", LIB,
-                                       os.path.join(CSRC, "gisspa.cu"),
-                                       os.path.join(CSRC, "noalloc.cu"),
-                                       os.path.join(CSRC, "merge.cu"),
-                                       os.path.join(CSRC, "hdf5io.cpp"), "-lz"])
+    objdir = os.path.join(LIBDIR, "_build")
+    os.makedirs(objdir, exist_ok=True)
+    # one compilation per unit, side by side; winops.cu in WIN_PARTS parts
+    jobs = [(os.path.join(CSRC, name), os.path.join(objdir, name + ".o"), [])
+            for name in ("gisspa.cu", "noalloc.cu", "merge.cu", "hdf5io.cpp")]
+    jobs += [(os.path.join(CSRC, "winops.cu"), os.path.join(objdir, "winops_%d.o" % k),
+              ["-DGS_WIN_PARTS=%d" % WIN_PARTS, "-DGS_WIN_PART=%d" % k]) for k in range(WIN_PARTS)]
+
+    def compile_one(job):
+        src, obj, extra = job
+        _run([NVCC] + NVCC_FLAGS + ARCH + extra + ["-I" + INCLUDE, "-c", "-o", obj, src])
+
+    with ThreadPoolExecutor(max(1, os.cpu_count() or 1)) as pool:
+        list(pool.map(compile_one, jobs))
+    _run([NVCC] + ARCH + ["-shared", "-o", LIB] + [obj for _, obj, _ in jobs] + ["-lz"])
     return LIB
 
 

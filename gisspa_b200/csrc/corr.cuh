@@ -133,7 +133,10 @@ struct CorrCfg {
     // the CTA finishes the current one.  Each was measured faster where used.
     static constexpr bool kWarpPub = (V * N2) % (16 * V) == 0;
     static constexpr int kDone = kWarpPub ? (V / 2) * T : T;  // completions that finish one pass of a unit
-    static constexpr int kCtasPerSm = 512 / kThreads;
+    // threads per SM: as many as the N2 complex values of a step-2 task leave
+    // registers for (64, 80 or 128 a thread)
+    static constexpr int kThreadsPerSm = N2 <= 16 ? 1024 : N2 <= 22 ? 768 : 512;
+    static constexpr int kCtasPerSm = kThreadsPerSm / kThreads;
     static_assert(V == 8 || V == 16, "tile width");
     static_assert(V == 2 * kWarps, "a row tile gives each warp two rows");
     // Odd N2 (l = 720 = 16 x 45): 16 and N2 are coprime, so both passes use

@@ -160,7 +160,7 @@ struct PfaCols {
 
 // In place, every row of `rows` rows of length L: to_physical moves
 // natural-order columns to the PfaCols order, otherwise back.
-__global__ void k_pfa_permute_rows(float2* __restrict__ data, long long rows, PfaCols pc, bool to_physical) {
+static __global__ void k_pfa_permute_rows(float2* __restrict__ data, long long rows, PfaCols pc, bool to_physical) {
     extern __shared__ float2 prow[];
     const int L = pc.L;
     for (long long r = blockIdx.x; r < rows; r += gridDim.x) {

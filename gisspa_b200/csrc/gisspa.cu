@@ -13,6 +13,7 @@
 #include "pixmax.cuh"
 #include "tccorr.cuh"
 #include "tccorr2.cuh"
+#include "winops.hpp"
 #include "refine.cuh"
 #include "seqsum.cuh"
 
@@ -27,6 +28,28 @@
 #include <vector>
 
 using namespace gs;
+
+namespace gs {
+
+// one table of kernels per compiled part of winops.cu
+const WinOps* win_ops_part0(int n2);
+const WinOps* win_ops_part1(int n2);
+const WinOps* win_ops_part2(int n2);
+const WinOps* win_ops_part3(int n2);
+const WinOps* win_ops_part4(int n2);
+const WinOps* win_ops_part5(int n2);
+const WinOps* win_ops_part6(int n2);
+const WinOps* win_ops_part7(int n2);
+
+const WinOps* win_ops(int l) {
+    if (l % 16) return nullptr;
+    using Part = const WinOps* (*)(int);
+    static const Part parts[8] = {win_ops_part0, win_ops_part1, win_ops_part2, win_ops_part3,
+                                  win_ops_part4, win_ops_part5, win_ops_part6, win_ops_part7};
+    return parts[(l / 16) % 8](l / 16);
+}
+
+}  // namespace gs
 
 namespace {
 
@@ -220,7 +243,8 @@ int run_fft(gs_ctx* ctx, int n, VecGeom g, int nimg, IO io, int max_tile = 16) {
     return GS_OK;
 }
 
-// Specialised l = 16 * N2 kernels (fastfft.cuh) exist for these sizes.
+// Windows whose two-pass, norm_type 1, per-pixel maximum and tensor-core
+// kernels are specialised too (winops.hpp has the others').
 bool fast_ok(const gs_ctx* ctx, int l) {
     if (ctx->generic_fft || l % 16) return false;
     const int n2 = l / 16;
@@ -255,35 +279,33 @@ int run_fast(gs_ctx* ctx, int l, int nimg, IO io) {
     }
 }
 
-template <int N2, int V>
-int launch_corr_nv(gs_ctx* ctx, const CorrArgs& a) {
-    using C = CorrCfg<N2, V>;
-    const size_t smem = CorrSmem<N2, V>::bytes;
-    auto kern = k_corr_persistent<N2, V>;
-    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0, nsm = 0, dev = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::kThreads, smem));
-    if (per_sm < 1) return set_err(ctx, GS_ERR_UNSUPPORTED, "persistent kernel does not fit on an SM");
-    if (ctx->corr_ctas_override > 0) per_sm = std::min(per_sm, ctx->corr_ctas_override);
-    const long long total_items = (long long)(a.nu + a.lag) * 2 * C::T;
-    const long long grid = std::min<long long>((long long)nsm * per_sm, total_items);
-    kern<<<(unsigned)grid, C::kThreads, smem, ctx->stream>>>(a);
+// The kernels specialised for this context's window (winops.hpp), or nullptr.
+const WinOps* win_of(const gs_ctx* ctx, int l) { return ctx->generic_fft ? nullptr : win_ops(l); }
+
+int win_status(gs_ctx* ctx, cudaError_t e, const char* what) {
+    if (e != cudaSuccess) return set_err(ctx, GS_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
     ++ctx->counters.kernel_launches;
-    CKL();
     return GS_OK;
+}
+
+// One transform of the specialised kernels over nimg images.
+template <class IO>
+int run_win(gs_ctx* ctx, int l, int nimg, cudaError_t (*launch)(const float2*, int, const IO&, cudaStream_t),
+            const IO& io) {
+    FftPlan* pl = nullptr;
+    TRY(get_plan(ctx, l, &pl));
+    if (nimg > 65535) return set_err(ctx, GS_ERR_UNSUPPORTED, "too many images in one FFT batch (%d)", nimg);
+    return win_status(ctx, launch(pl->tw, nimg, io, ctx->stream), "window transform");
 }
 
 // Persistent FP32 correlation with tiles of `tile` vectors (16 or 8).
 int launch_corr(gs_ctx* ctx, int l, int tile, const CorrArgs& a) {
-    const bool wide = tile != 8;
-    switch (l / 16) {
-        case 32: return wide ? launch_corr_nv<32, 16>(ctx, a) : launch_corr_nv<32, 8>(ctx, a);
-        case 45: return wide ? launch_corr_nv<45, 16>(ctx, a) : launch_corr_nv<45, 8>(ctx, a);
-        case 48: return wide ? launch_corr_nv<48, 16>(ctx, a) : launch_corr_nv<48, 8>(ctx, a);
-        default: return set_err(ctx, GS_ERR_UNSUPPORTED, "no persistent kernel for %d", l);
-    }
+    const WinOps* w = win_of(ctx, l);
+    if (!w) return set_err(ctx, GS_ERR_UNSUPPORTED, "no persistent kernel for %d", l);
+    bool fits = true;
+    const cudaError_t e = w->corr(a, tile, ctx->corr_ctas_override, ctx->stream, &fits);
+    if (!fits) return set_err(ctx, GS_ERR_UNSUPPORTED, "persistent kernel does not fit on an SM");
+    return win_status(ctx, e, "persistent correlation");
 }
 
 template <int N2, bool kBf16>
@@ -432,13 +454,13 @@ static int pair_spectra_n(gs_ctx* ctx, float e, const float2* cs, int nang, floa
                                                                 P<float4>(ctx->coef), nang);
     ++ctx->counters.kernel_launches;
     CKL();
-    if (fast_ok(ctx, l)) {
+    if (const WinOps* w = win_of(ctx, l)) {
         const F16PairNorm rows{TS, P<float4>(ctx->coef), l, l2};
         if (pfa)
-            TRY(run_fast<false, false>(ctx, l, nimg, F16PairNormPfa{rows, PfaCols::make(l)}));
+            TRY(run_win(ctx, l, nimg, w->pair_rows_pfa, F16PairNormPfa{rows, PfaCols::make(l)}));
         else
-            TRY(run_fast<false, false>(ctx, l, nimg, rows));
-        TRY(run_fast<false, true>(ctx, l, nimg, F16Complex<true>{TS, l, l2, (float)(1.0 / (double)l2)}));
+            TRY(run_win(ctx, l, nimg, w->pair_rows, rows));
+        TRY(run_win(ctx, l, nimg, w->cols, F16Complex<true>{TS, l, l2, (float)(1.0 / (double)l2)}));
     } else {
         TRY(run_fft<false>(ctx, l, rows_of(l, l), nimg, IoPairNorm{TS, P<float4>(ctx->coef), l2}));
         TRY(run_fft<false>(ctx, l, cols_of(l, l), nimg, IoComplex{TS, (float)(1.0 / (double)l2)}));
@@ -974,9 +996,10 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
             k_tmpl_pad_edge<<<nc, 256, 0, ctx->stream>>>(P<float>(raw), tx, ty, l, P<float2>(F));
             ++ctx->counters.kernel_launches;
             if (cudaGetLastError() != cudaSuccess) { st = set_err(ctx, GS_ERR_CUDA, "k_tmpl_pad_edge"); break; }
-            if (fast_ok(ctx, l)) {
-                if ((st = run_fast<false, false>(ctx, l, nc, F16Complex<false>{P<float2>(F), l, (long long)l2, 1.0f}))) break;
-                if ((st = run_fast<false, true>(ctx, l, nc, F16Complex<true>{P<float2>(F), l, (long long)l2, 1.0f / (float)l2}))) break;
+            const WinOps* w = win_of(ctx, l);
+            if (w) {
+                if ((st = run_win(ctx, l, nc, w->rows, F16Complex<false>{P<float2>(F), l, (long long)l2, 1.0f}))) break;
+                if ((st = run_win(ctx, l, nc, w->cols, F16Complex<true>{P<float2>(F), l, (long long)l2, 1.0f / (float)l2}))) break;
             } else {
                 if ((st = run_fft<false>(ctx, l, rows_of(l, l), nc, IoComplex{P<float2>(F), 1.0f}))) break;
                 if ((st = run_fft<false>(ctx, l, cols_of(l, l), nc, IoComplex{P<float2>(F), 1.0f / (float)l2}))) break;
@@ -1002,9 +1025,9 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
             k_inv_amp_norm<<<blocks_for(nc, 128), 128, 0, ctx->stream>>>(P<double>(sumsq), nc, P<double>(inv));
             ++ctx->counters.kernel_launches;
             if (cudaGetLastError() != cudaSuccess) { st = set_err(ctx, GS_ERR_CUDA, "template weighting"); break; }
-            if (fast_ok(ctx, l)) {
-                if ((st = run_fast<true, false>(ctx, l, nc, F16ScaleIn<false>{P<float2>(F), P<double>(inv), l, (long long)l2}))) break;
-                if ((st = run_fast<true, true>(ctx, l, nc, F16RealOut<true>{P<float2>(F), P<float>(ctx->tmpl) + (size_t)c0i * l2,
+            if (w) {
+                if ((st = run_win(ctx, l, nc, w->inv_rows, F16ScaleIn<false>{P<float2>(F), P<double>(inv), l, (long long)l2}))) break;
+                if ((st = run_win(ctx, l, nc, w->inv_cols, F16RealOut<true>{P<float2>(F), P<float>(ctx->tmpl) + (size_t)c0i * l2,
                                                                             l, (long long)l2}))) break;
             } else {
                 if ((st = run_fft<true>(ctx, l, rows_of(l, l), nc, IoScaleIn{P<float2>(F), P<double>(inv)}))) break;
@@ -1126,9 +1149,9 @@ static int prep_micrograph(gs_ctx* ctx, const MicPlan& mp, float2* W) {
         ++ctx->counters.kernel_launches;
         CKL();
     }
-    if (fast_ok(ctx, l)) {
-        TRY(run_fast<false, false>(ctx, l, nw, F16Complex<false>{Wm, l, l2, 1.0f}));
-        TRY(run_fast<false, true>(ctx, l, nw, F16Complex<true>{Wm, l, l2, (float)(1.0 / (double)l2)}));
+    if (const WinOps* w = win_of(ctx, l)) {
+        TRY(run_win(ctx, l, nw, w->rows, F16Complex<false>{Wm, l, l2, 1.0f}));
+        TRY(run_win(ctx, l, nw, w->cols, F16Complex<true>{Wm, l, l2, (float)(1.0 / (double)l2)}));
     } else {
         TRY(run_fft<false>(ctx, l, rows_of(l, l), nw, IoComplex{Wm, 1.0f}));
         TRY(run_fft<false>(ctx, l, cols_of(l, l), nw, IoComplex{Wm, (float)(1.0 / (double)l2)}));
@@ -1355,8 +1378,9 @@ static int prefetch_pair_spectra(gs_ctx* ctx, int NW, const std::vector<float>& 
     const int l = ctx->l, N = ctx->ntmpl, Np = (N + 1) / 2, na = (int)angles.size();
     const long long l2 = (long long)l * l;
     const bool tc2 = p.precision == GS_PREC_TC_FULL || p.precision == GS_PREC_TC_FULL_1P;
-    const bool persistent = fast_ok(ctx, l) && !ctx->two_pass;
+    const bool persistent = win_of(ctx, l) && !ctx->two_pass;
     if (!persistent || ctx->autotune || p.norm_type == 1 || na == 0 || (tc2 && l != 720)) return GS_OK;
+    if (p.precision != GS_PREC_FP32 && !fast_ok(ctx, l)) return GS_OK;  // the correlation refuses it
     const int nu = Np * NW;
     if (!units_fit(l, nu)) return GS_OK;  // the correlation reports it
     const bool pfa = (p.precision == GS_PREC_FP32 || tc2) && PfaCols::make(l).N2 != 0;
@@ -1403,14 +1427,14 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
     const int N = ctx->ntmpl, Np = (N + 1) / 2;
     const int na = (int)angles.size();
     const long long total_units = (long long)na * NW * N;
-    const bool persistent = fast_ok(ctx, l) && !ctx->two_pass;
+    const bool persistent = win_of(ctx, l) && !ctx->two_pass;
     // the FP32 persistent kernel at window 720 takes prime-factor transforms
     // and reads its spectra in PfaCols column order
     const bool tc2 = p.precision == GS_PREC_TC_FULL || p.precision == GS_PREC_TC_FULL_1P;
     if (tc2 && l != 720)
         return set_err(ctx, GS_ERR_UNSUPPORTED, "the all-tensor-core path takes window 720 (got %d)", l);
     const bool pfa = persistent && (p.precision == GS_PREC_FP32 || tc2) && PfaCols::make(l).N2 != 0;
-    if (p.precision != GS_PREC_FP32 && !persistent)
+    if (p.precision != GS_PREC_FP32 && !(persistent && fast_ok(ctx, l)))
         return set_err(ctx, GS_ERR_UNSUPPORTED,
                        "tensor-core precision needs window 512, 720 or 768 and the persistent path (window %d)", l);
     const int nu = Np * NW;
@@ -1454,6 +1478,23 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         }
         if (!ctx->window_block_set) tune.window_block = 8;
         if (!ctx->corr_tile_set) tune.tile = 8;
+    } else if (persistent && p.precision == GS_PREC_FP32 && !fast_ok(ctx, l)) {
+        // other windows: the smaller the window, the fewer tiles a unit has
+        // and the more units the resident CTAs hold at once, so the ring goes
+        // by them.  A unit's column tiles are queued 2.5 times as many items
+        // after its row tiles as there are CTAs (window 128: 12.5 ms against
+        // 56.9 with 0.6 times; 320: 11.6 against 36.3; 640: 27.8 against
+        // 78.3), and 2.2 slots per unit of lag leave the row tiles room
+        // (1.6: up to 1.8 times slower).  8-vector tiles win by 1 to 4 % up
+        // to window 576, 16-vector ones by 2 to 25 % above it.
+        if (!ctx->corr_tile_set) tune.tile = l <= 576 ? 8 : 16;
+        if (!ctx->corr_ring_set) {
+            int nsm = 0;
+            CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+            const int ctas = nsm * win_of(ctx, l)->threads_per_sm / (16 * tune.tile), tiles = l / tune.tile;
+            tune.lag = (5 * ctas + 4 * tiles - 1) / (4 * tiles);
+            tune.slots = (11 * tune.lag + 4) / 5;
+        }
     }
     // window spectra in PfaCols order for the duration of the correlation,
     // natural order again afterwards (on every return path)
@@ -1495,7 +1536,7 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         TRY(ensure(ctx, ctx->flags, sizeof(int) * 4));
         CK(cudaMemsetAsync(ctx->flags.p, 0, sizeof(int) * 4, ctx->stream));
         if (ctx->autotune) {
-            TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * 32));
+            TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * std::max(32, tune.slots)));
             TRY(pair_spectra(ctx, angles[0], TS, pfa));
             if (tc2) {
                 CK(cudaMemsetAsync(ctx->tc2_pmax.p, 0, sizeof(float) * Np, ctx->stream));

@@ -21,7 +21,7 @@ namespace gs {
 // (r-1)^2 <= d^2 <= (r+1)^2, r = l/2 - 2, around (l/2, l/2).
 // Reference: readAndPaddingTemplate + edgeNormalize (main.cu:182-223,
 // 311-385; kernels GPU_func.cu:3-94).  One CTA per template.
-__global__ void __launch_bounds__(256) k_tmpl_pad_edge(const float* __restrict__ raw, int tx, int ty, int l,
+static __global__ void __launch_bounds__(256) k_tmpl_pad_edge(const float* __restrict__ raw, int tx, int ty, int l,
                                                         float2* __restrict__ out) {
     __shared__ double red[4 * 32];
     const int J = blockIdx.x;
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(256) k_tmpl_pad_edge(const float* __restrict__
 // div[r] = sqrt(sum |F|^2 / count) for shells 0 <= r < l/2.
 // Reference: SQRSum_by_circle, mode 0 (GPU_func.cu:98-128).  One CTA per
 // template; shared memory holds the shell histogram (l/2 doubles + counts).
-__global__ void __launch_bounds__(256) k_tmpl_shells(const float2* __restrict__ F, int l, float* __restrict__ div) {
+static __global__ void __launch_bounds__(256) k_tmpl_shells(const float2* __restrict__ F, int l, float* __restrict__ div) {
     extern __shared__ double sh[];
     const int ns = l / 2;
     double* ra = sh;
@@ -104,7 +104,7 @@ struct WeightConsts {
 // Per-bin band-pass x |CTF| x Wiener factor of the template weighting,
 // identical for every template.  Reference: apply_weighting_function
 // (GPU_func.cu:249-290), CTF of the first micrograph.
-__global__ void k_weight_map(float* __restrict__ wmap, int l, WeightConsts wc, CtfDev c) {
+static __global__ void k_weight_map(float* __restrict__ wmap, int l, WeightConsts wc, CtfDev c) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= l * l) return;
     const int x = i % l, y = i / l;
@@ -124,7 +124,7 @@ __global__ void k_weight_map(float* __restrict__ wmap, int l, WeightConsts wc, C
 // The whitened template spectrum alone (F / shell RMS, no weight), written
 // to B: the base that the off-grid refinement re-weights with other CTF
 // parameters.  Same whitening as k_tmpl_apply (whiten_Tmp, GPU_func.cu:130-152).
-__global__ void __launch_bounds__(256) k_tmpl_whiten(const float2* __restrict__ F, int l, const float* __restrict__ div,
+static __global__ void __launch_bounds__(256) k_tmpl_whiten(const float2* __restrict__ F, int l, const float* __restrict__ div,
                                                      float2* __restrict__ B) {
     const int J = blockIdx.y;
     const int ns = l / 2;
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(256) k_tmpl_whiten(const float2* __restrict__ 
 // sum |F|^2 and the count over r < l/2, x <= l/2.
 // Reference: whiten_Tmp + apply_weighting_function + compute_area_sum_ofSQR
 // (GPU_func.cu:130-152, 249-290, 318-362).  Grid (pixel chunks, templates).
-__global__ void __launch_bounds__(256) k_tmpl_apply(float2* __restrict__ F, int l, const float* __restrict__ div,
+static __global__ void __launch_bounds__(256) k_tmpl_apply(float2* __restrict__ F, int l, const float* __restrict__ div,
                                                     const float* __restrict__ wmap, double* __restrict__ sumsq) {
     __shared__ double red[2 * 32];
     const int J = blockIdx.y;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256) k_tmpl_apply(float2* __restrict__ F, int 
 // 1 / m with m = sqrt(sum / count^2) (1 when m == 0).  Reference: the host
 // loop after compute_area_sum_ofSQR and `normalize` (main.cu:446-456,
 // GPU_func.cu:409-422).
-__global__ void k_inv_amp_norm(const double* __restrict__ sumsq, int n, double* __restrict__ inv) {
+static __global__ void k_inv_amp_norm(const double* __restrict__ sumsq, int n, double* __restrict__ inv) {
     const int J = blockIdx.x * blockDim.x + threadIdx.x;
     if (J >= n) return;
     const double c = sumsq[2 * J + 1];
@@ -194,7 +194,7 @@ struct MicStats {
 
 // Per-pixel quotients of the reference's host statistics loop
 // (main.cu:530-535): cur/nx/ny and cur*cur/nx/ny, IEEE float32 each.
-__global__ void k_mic_quot(const float* __restrict__ img, long long n, int nx, int ny, float* __restrict__ q1,
+static __global__ void k_mic_quot(const float* __restrict__ img, long long n, int nx, int ny, float* __restrict__ q1,
                            float* __restrict__ q2) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -219,7 +219,7 @@ __device__ __forceinline__ MicStats mic_stats(float s1, float s2) {
 
 // Hot-pixel clamp to the mean, optional inversion, real -> complex.
 // Reference: init_d_image host loops + float2Complex (main.cu:541-551).
-__global__ void k_mic_clamp(const float* __restrict__ img, long long n, const float* __restrict__ sums, int invert,
+static __global__ void k_mic_clamp(const float* __restrict__ img, long long n, const float* __restrict__ sums, int invert,
                             float2* __restrict__ out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -235,7 +235,7 @@ __global__ void k_mic_clamp(const float* __restrict__ img, long long n, const fl
 // nx != ny).  Reference: do_phase_flip + SQRSum_by_circle mode 1
 // (GPU_func.cu:785-796, 98-128).  Each CTA owns a row range and keeps its
 // histogram in shared memory.
-__global__ void __launch_bounds__(256) k_mic_flip_shells(float2* __restrict__ F, int nx, int ny, CtfDev c,
+static __global__ void __launch_bounds__(256) k_mic_flip_shells(float2* __restrict__ F, int nx, int ny, CtfDev c,
                                                          double* __restrict__ ra, unsigned* __restrict__ rb) {
     extern __shared__ double sh[];
     const int ns = max(nx, ny) / 2;
@@ -280,7 +280,7 @@ struct MicWhitenConsts {
 // beyond L*apix/6, band-pass, Wiener weight, then DC := 0.
 // Reference: whiten_filetr_weight_Img + set_0Hz_to_0_at_RI
 // (GPU_func.cu:155-227).
-__global__ void k_mic_whiten(float2* __restrict__ F, int nx, int ny, CtfDev c, MicWhitenConsts w,
+static __global__ void k_mic_whiten(float2* __restrict__ F, int nx, int ny, CtfDev c, MicWhitenConsts w,
                              const double* __restrict__ ra, const unsigned* __restrict__ rb) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)nx * ny) return;
@@ -307,11 +307,11 @@ __global__ void k_mic_whiten(float2* __restrict__ F, int nx, int ny, CtfDev c, M
     F[i] = (i == 0) ? make_float2(0.0f, 0.0f) : cscale(F[i], f);
 }
 
-__global__ void k_set_dc_zero(float2* F) { F[0] = make_float2(0.0f, 0.0f); }
+static __global__ void k_set_dc_zero(float2* F) { F[0] = make_float2(0.0f, 0.0f); }
 
 // Cut l x l windows (window w = i + j*bx at (offx[i], offy[j]); zero beyond
 // the image).  Reference: split_IMG (GPU_func.cu:564-581).
-__global__ void k_extract_windows(const float* __restrict__ img, int nx, int ny, const int* __restrict__ offx,
+static __global__ void k_extract_windows(const float* __restrict__ img, int nx, int ny, const int* __restrict__ offx,
                                   const int* __restrict__ offy, int bx, int l, float2* __restrict__ W) {
     const int w = blockIdx.y;
     const int i = w % bx, j = w / bx;
@@ -325,7 +325,7 @@ __global__ void k_extract_windows(const float* __restrict__ img, int nx, int ny,
 
 // Per-window sum |W|^2 and count over r < l/2, x <= l/2 (for the amplitude
 // normalisation of split_normalize_image, main.cu:617-653).
-__global__ void __launch_bounds__(256) k_win_sumsq(const float2* __restrict__ W, int l, double* __restrict__ out) {
+static __global__ void __launch_bounds__(256) k_win_sumsq(const float2* __restrict__ W, int l, double* __restrict__ out) {
     __shared__ double red[2 * 32];
     const int w = blockIdx.y;
     const float2* d = W + (size_t)w * l * l;
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(256) k_win_sumsq(const float2* __restrict__ W,
 }
 
 // Multiply image g by scale[g] (float).
-__global__ void k_scale_images(float2* __restrict__ d, long long per_img, const double* __restrict__ scale) {
+static __global__ void k_scale_images(float2* __restrict__ d, long long per_img, const double* __restrict__ scale) {
     const int g = blockIdx.y;
     const float s = (float)scale[g];
     float2* p = d + (size_t)g * per_img;
@@ -368,7 +368,7 @@ __global__ void k_scale_images(float2* __restrict__ d, long long per_img, const 
 // Several angles in one launch: with `cs` set, blockIdx.z selects angle z of
 // the group ((cos, sin) = cs[z]), its images start at out + z Np l^2 and its
 // sums at stats + 2 z ntmpl; without it, (cose, sine) and one angle.
-__global__ void __launch_bounds__(256) k_pair_rotate(const float* __restrict__ tmpl, int ntmpl, int l, float cose,
+static __global__ void __launch_bounds__(256) k_pair_rotate(const float* __restrict__ tmpl, int ntmpl, int l, float cose,
                                                      float sine, const float2* __restrict__ cs, float d_m,
                                                      float2* __restrict__ out, double* __restrict__ stats) {
     __shared__ double red[4 * 32];
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(256) k_pair_rotate(const float* __restrict__ t
 // substract_by_mean / divided_by_var (GPU_func.cu:424-443, main.cu:696-707).
 // `nang` angles one after the other: pair p of angle z at coef[z Np + p],
 // from stats + 2 z ntmpl.
-__global__ void k_pair_coef(const double* __restrict__ stats, int ntmpl, int l, float4* __restrict__ coef,
+static __global__ void k_pair_coef(const double* __restrict__ stats, int ntmpl, int l, float4* __restrict__ coef,
                             int nang) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int np = (ntmpl + 1) / 2;
@@ -577,7 +577,7 @@ struct UnitOut {
 
 // Score of each (window, template): peak = max(0, masked max), sigma of the
 // map without the peak (rc = l^2 - 1).  Reference: main.cu:869-876.
-__global__ void k_finalize(const UnitAcc* __restrict__ acc, int ntmpl, int l, UnitOut* __restrict__ out) {
+static __global__ void k_finalize(const UnitAcc* __restrict__ acc, int ntmpl, int l, UnitOut* __restrict__ out) {
     const int J = blockIdx.x * blockDim.x + threadIdx.x;
     if (J >= ntmpl) return;
     const UnitAcc a = acc[J];
@@ -609,7 +609,7 @@ struct PickDev {
 // The micrograph owns windows [w0, w0 + nw) of a units table laid out
 // [angle][NW windows][nt templates]; pick.unit is its local index
 // (angle, window, template), the reference's line order.
-__global__ void k_compact(const UnitOut* __restrict__ units, long long total, int nw, int nt, int bx,
+static __global__ void k_compact(const UnitOut* __restrict__ units, long long total, int nw, int nt, int bx,
                           const int* __restrict__ offx, const int* __restrict__ offy, int l, float d_m, int nx, int ny,
                           float thres, PickDev* __restrict__ picks, unsigned long long* __restrict__ count,
                           long long cap, int NW, int w0) {

@@ -2,7 +2,7 @@
 //
 // rfft<N, S, kInv, OFF>(a) transforms the N complex values a[OFF + n*S]
 // (n < N) of a register array in place.  N is split recursively as
-// N = P * Q with P a base radix (2, 3, 4, 5, 8).  When P and Q share a factor
+// N = P * Q with P a base radix (2, 3, 4, 5, 8, or a prime up to 23).  When P and Q share a factor
 // (Cooley-Tukey):
 //     X[k1 + P k2] = sum_{n2} W_Q^{n2 k2} W_N^{n2 k1} sum_{n1} x[n2 + Q n1] W_P^{n1 k1}
 // (P-point DFTs at stride Q, twiddles, Q-point DFTs on contiguous blocks).
@@ -76,10 +76,20 @@ __host__ __device__ __forceinline__ void static_for(F&& f) {
     StaticFor<0, N>::run(f);
 }
 
-constexpr bool is_base(int n) { return n == 2 || n == 3 || n == 4 || n == 5 || n == 8; }
+constexpr bool is_prime_base(int n) { return n == 7 || n == 11 || n == 13 || n == 17 || n == 19 || n == 23; }
+constexpr bool is_base(int n) { return n == 2 || n == 3 || n == 4 || n == 5 || n == 8 || is_prime_base(n); }
+// 8 where the rest is odd (24, 40: no twiddles then), else 4, 5, 3, 2; a
+// number without these factors is a prime base
 constexpr int first_factor(int n) {
-    return (n % 4 == 0 && n > 8) ? 4 : (n % 5 == 0 && n > 5) ? 5 : (n % 3 == 0 && n > 3) ? 3
-         : (n % 2 == 0 && n > 8) ? 2 : n;
+    return (n % 8 == 0 && n > 8 && (n / 8) % 2 == 1 && n < 48) ? 8
+         : (n % 4 == 0 && n > 8) ? 4 : (n % 5 == 0 && n > 5) ? 5 : (n % 3 == 0 && n > 3) ? 3
+         : (n % 2 == 0 && n > 2) ? 2 : n;
+}
+// whether rfft<n> exists: every prime factor is a base
+constexpr bool rfft_exists(int n) {
+    for (int p : {2, 3, 5, 7, 11, 13, 17, 19, 23})
+        while (n % p == 0) n /= p;
+    return n == 1;
 }
 constexpr int gcd_c(int a, int b) { return b == 0 ? a : gcd_c(b, a % b); }
 // prime-factor split of N = first_factor(N) x rest (coprime factors)
@@ -121,8 +131,43 @@ __host__ __device__ __forceinline__ float2 twiddle_mul(float2 a) {
     }
 }
 
+// DFT of an odd prime length by the symmetry of cos and sin: with s_j = a_j +
+// a_{R-j} and d_j = a_j - a_{R-j}, X_k and X_{R-k} are (a_0 + sum cos(2 pi jk/R) s_j)
+// -+ i sum sin(2 pi jk/R) d_j, j <= (R-1)/2: (R-1)^2 real multiply-adds.
+template <int R, int S, bool kInv, int OFF>
+__host__ __device__ __forceinline__ void dft_prime(float2* a) {
+    constexpr int H = (R - 1) / 2;
+    float2 s[H + 1], d[H + 1];
+    const float2 a0 = a[OFF];
+    float2 sum = a0;
+    static_for<H>([&](auto jc) {
+        constexpr int j = decltype(jc)::value + 1;
+        s[j] = cadd(a[OFF + j * S], a[OFF + (R - j) * S]);
+        d[j] = csub(a[OFF + j * S], a[OFF + (R - j) * S]);
+        sum = cadd(sum, s[j]);
+    });
+    a[OFF] = sum;
+    static_for<H>([&](auto kc) {
+        constexpr int k = decltype(kc)::value + 1;
+        float2 c = a0, e = make_float2(0.0f, 0.0f);
+        static_for<H>([&](auto jc) {
+            constexpr int j = decltype(jc)::value + 1;
+            constexpr float cj = (float)cos2pi(j * k, R), sj = (float)sin2pi(j * k, R);
+            c = make_float2(fmaf(cj, s[j].x, c.x), fmaf(cj, s[j].y, c.y));
+            e = j == 1 ? cscale(d[j], sj) : make_float2(fmaf(sj, d[j].x, e.x), fmaf(sj, d[j].y, e.y));
+        });
+        e = mul_mi<kInv>(e);
+        a[OFF + k * S] = cadd(c, e);
+        a[OFF + (R - k) * S] = csub(c, e);
+    });
+}
+
 template <int R, int S, bool kInv, int OFF>
 __host__ __device__ __forceinline__ void base_dft(float2* a) {
+    if constexpr (is_prime_base(R)) {
+        dft_prime<R, S, kInv, OFF>(a);
+        return;
+    }
     if constexpr (R == 2) {
         dft2<kInv>(a[OFF], a[OFF + S]);
     } else if constexpr (R == 3) {

@@ -305,8 +305,9 @@ int gs_set_kernel_timing(struct gs_ctx* ctx, int enable);
  * use the specialised l = 16*N2 kernels where they exist (default). */
 #define GS_OPT_GENERIC_FFT 1
 /* GS_OPT_TWO_PASS: 1 = run the correlation as separate row and column
- * launches per window, 0 = one persistent launch per angle where the
- * specialised kernels exist (default). */
+ * launches per window, 0 = persistent launches where the specialised
+ * kernels exist: windows l = 16 N2 with N2 from 6 to 48 whose prime factors
+ * are at most 23 (default). */
 #define GS_OPT_TWO_PASS 2
 /* GS_OPT_WINDOW_BLOCK: windows per block of the persistent launch's unit
  * order (reuse of window and pair spectra in L2); default 4 (8 for the FP32
@@ -315,7 +316,9 @@ int gs_set_kernel_timing(struct gs_ctx* ctx, int enable);
 /* GS_OPT_CORR_SLOTS / GS_OPT_CORR_LAG: scratch maps in the persistent
  * launch's ring (default 16) and how many units after its row tiles a unit's
  * column tiles are queued (default 6); slots must exceed lag.  The FP32
- * kernel at window 512 defaults to 32 slots and a lag of 10.  The
+ * kernel at window 512 defaults to 32 slots and a lag of 10, and at windows
+ * other than 512, 720 and 768 to a lag of 2.5 times the resident CTAs in items
+ * and 2.2 slots per unit of lag.  The
  * all-tensor-core modes keep more items in flight and default to 24 slots and
  * a lag of 12 unless either option was set; they need lag >= 1 and
  * slots >= lag + 2 (GS_ERR_UNSUPPORTED otherwise). */
@@ -335,8 +338,8 @@ int gs_set_kernel_timing(struct gs_ctx* ctx, int enable);
  * keep the fastest for this context (gs_get_tuning shows the choice). */
 #define GS_OPT_AUTOTUNE 8
 /* GS_OPT_CORR_TILE: vectors per tile of the FP32 persistent kernel: 16
- * (256-thread CTAs, two per SM; default) or 8 (128-thread CTAs, four per
- * SM; default at window 512).  The autotuner also tries both. */
+ * (256-thread CTAs, two or more per SM; default above window 576) or 8
+ * (128-thread CTAs, twice as many per SM; default up to it).  The autotuner also tries both. */
 #define GS_OPT_CORR_TILE 9
 /* GS_OPT_ANGLES_PER_LAUNCH: in-plane angles whose units one persistent
  * correlation launch covers (their pair spectra are computed first, all
