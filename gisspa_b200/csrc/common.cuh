@@ -11,9 +11,40 @@ namespace gs {
 // in the reference is formed with it, so the kernels use it too.
 constexpr double kPiRef = 3.141592654;
 
-__host__ __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__host__ __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__host__ __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+// Complex sums and products with real factors: one packed instruction for both
+// parts (FADD2, FMUL2, FFMA2).  The FP32 pipe does the same work either way;
+// what is saved is issue slots, which bound the transforms (see corr.cuh).
+// Sums with a factor +-i stay scalar (cadd_mi): a packed one would first have
+// to swap the parts.
+__host__ __device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+    return __fadd2_rn(a, b);
+#else
+    return make_float2(a.x + b.x, a.y + b.y);
+#endif
+}
+__host__ __device__ __forceinline__ float2 csub(float2 a, float2 b) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+    return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);
+#else
+    return make_float2(a.x - b.x, a.y - b.y);
+#endif
+}
+__host__ __device__ __forceinline__ float2 cscale(float2 a, float s) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+    return __fmul2_rn(a, make_float2(s, s));
+#else
+    return make_float2(a.x * s, a.y * s);
+#endif
+}
+// a s + b, s real
+__host__ __device__ __forceinline__ float2 cfma(float2 a, float s, float2 b) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+    return __ffma2_rn(a, make_float2(s, s), b);
+#else
+    return make_float2(fmaf(a.x, s, b.x), fmaf(a.y, s, b.y));
+#endif
+}
 __host__ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -25,6 +56,17 @@ __host__ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
 template <bool kInv>
 __host__ __device__ __forceinline__ float2 mul_mi(float2 a) {
     return kInv ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+}
+
+// a + b (-i) forward, a + b (+i) inverse
+template <bool kInv>
+__host__ __device__ __forceinline__ float2 cadd_mi(float2 a, float2 b) {
+    return kInv ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, a.y - b.x);
+}
+// the same with b scaled by a real s
+template <bool kInv>
+__host__ __device__ __forceinline__ float2 cfma_mi(float2 a, float2 b, float s) {
+    return kInv ? make_float2(fmaf(-s, b.y, a.x), fmaf(s, b.x, a.y)) : make_float2(fmaf(s, b.y, a.x), fmaf(-s, b.x, a.y));
 }
 
 // Radial shell index of the reference's whitening / band-pass code

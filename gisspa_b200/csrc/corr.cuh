@@ -16,16 +16,16 @@
 // Dependencies and why they cannot deadlock: a column tile of u waits until
 // all T row tiles of u are done; a row tile of u >= S waits until all
 // column tiles of u - S are done (its scratch slot is free).  Completion is
-// counted per tile or per warp (CorrCfg::kWarpPub).  Per tile: after the CTA
-// barrier that ends a tile, one thread (the publisher, the CTA's last thread,
-// which has the lightest share of step 1 when the tasks do not divide evenly)
-// increments the unit's counter, so a pass of a unit is done at T
-// increments, claims the CTA's next-but-one item (written into the CTA's
-// ring of claimed items just before the following barrier, so its warp does
-// not wait for the atomic), and each warp checks the dependency of its CTA's
-// next item itself before starting it.  Per warp: every warp counts its own share
-// before that barrier (a pass is done at warps x T increments), and thread 0
-// waits for the next item's dependency before it.  Both dependencies point at
+// counted per tile: after the CTA barrier that ends a tile, one thread (the
+// publisher, the CTA's last thread, which has the lightest share of step 1
+// when the tasks do not divide evenly) increments the unit's counter, so a
+// pass of a unit is done at T increments, claims the CTA's next-but-one item
+// (written into the CTA's ring of claimed items just before the following
+// barrier, so its warp does not wait for the atomic), and each warp checks the
+// dependency of its CTA's next item itself before starting it.  (Counting
+// every warp's share before the barrier instead costs each warp a release:
+// window 256 8.99 against 8.54 ms, 512 8.54 against 8.18, 768 22.2 against
+// 20.6, 20 to 35 k units.)  Both dependencies point at
 // items that come earlier in the claim order, and an item is claimed only by
 // a running CTA that finishes and publishes it before it waits for anything
 // later, so the earliest unpublished item can always proceed.  Every wait is
@@ -35,12 +35,12 @@
 //
 // Memory ordering: producers store the maps bypassing L1 (st.global with an
 // L2 cache hint) and add their accumulator atomics; the CTA barrier that ends
-// the tile (per warp: __syncwarp) orders every thread's stores before the
+// the tile orders every thread's stores before the
 // release increment (acquire-release for column tiles, whose last increment also
 // computes the unit's scores), which therefore makes all of them visible
-// (release is cumulative).  On the consumer side lane 0 of each warp (per
-// warp: thread 0) spins with ld.acquire.gpu and __syncwarp() (the barrier)
-// extends the acquire to its warp (CTA), whose threads read the maps with L1::no_allocate loads (L2, never a stale L1
+// (release is cumulative).  On the consumer side lane 0 of each warp spins with
+// ld.acquire.gpu and __syncwarp() extends the acquire to its warp, whose
+// threads read the maps with L1::no_allocate loads (L2, never a stale L1
 // line from an earlier occupant of the slot).  A column tile costs two CTA
 // barriers (step 1 -> step 2 of the FFT, whose vectors are columns spread
 // over all warps for coalesced loads, and the end-of-item barrier); a row
@@ -119,23 +119,18 @@ struct CorrCfg {
     static constexpr int L = 16 * N2;
     static constexpr int V = V_;
     static constexpr int BP = (N2 % 2) ? N2 : N2 + 1;  // odd block pitch
-    static constexpr int VP = 16 * BP + 1;             // vector pitch
+    // vector pitch, so that the column tile's stores (V vectors by 16 / V
+    // values of n2 in a half-warp) fall into 16 different bank pairs
+    static constexpr int VP = 16 * BP + 16 / V;
     static constexpr int kThreads = 16 * V;
     static constexpr int kWarps = kThreads / 32;
     static constexpr int T = L / V;
-    // Publication protocol.  When step 1's tasks do not divide evenly over
-    // the threads (odd N2), per tile: one thread publishes after the
-    // end-of-item barrier -- the CTA's last thread, whose step-1 share is the
-    // lightest, so the release fence it waits for costs no barrier time --
-    // and every warp checks its next item's dependency itself.  Otherwise
-    // (kWarpPub) per warp: lane 0 of every warp counts its own share before
-    // that barrier, and thread 0 waits for the next item's dependency while
-    // the CTA finishes the current one.  Each was measured faster where used.
-    static constexpr bool kWarpPub = (V * N2) % (16 * V) == 0;
-    static constexpr int kDone = kWarpPub ? (V / 2) * T : T;  // completions that finish one pass of a unit
-    // threads per SM: as many as the N2 complex values of a step-2 task leave
-    // registers for (64, 80 or 128 a thread)
-    static constexpr int kThreadsPerSm = N2 <= 16 ? 1024 : N2 <= 22 ? 768 : 512;
+    // Threads per SM (64, 80 or 128 registers each).  More of them hide more L2
+    // latency until the registers no longer hold a task's loads in flight:
+    // window 384 (N2 = 24) 241 Gpoint/s with 768 against 208 with 512 and 202
+    // with 896; 304 (19) 225 with 1024 against 218 with 768; 320 (20) 221 with
+    // 768 against 206 with 1024; 448 (28) 218 with 512 against 195 with 768.
+    static constexpr int kThreadsPerSm = N2 <= 19 ? 1024 : N2 <= 26 ? 768 : 512;
     static constexpr int kCtasPerSm = kThreadsPerSm / kThreads;
     static_assert(V == 8 || V == 16, "tile width");
     static_assert(V == 2 * kWarps, "a row tile gives each warp two rows");
@@ -170,8 +165,7 @@ struct CorrSmem {
     using C = CorrCfg<N2, V>;
     static constexpr size_t tile = (size_t)C::V * C::VP * sizeof(float2);
     static constexpr size_t tw = C::kPfa ? 0 : (size_t)16 * N2 * sizeof(float2);  // no twiddles with kPfa
-    static constexpr size_t red = 128 * sizeof(double);
-    static constexpr size_t bytes = tile + tw + red + 32;
+    static constexpr size_t bytes = tile + tw + 32;  // and the ring of claimed items
 };
 
 // L2 eviction-priority hints: scratch maps are stored "evict last" (they are
@@ -314,7 +308,7 @@ __device__ __forceinline__ void corr_col_tile(const CorrArgs& a, int u, int t, f
     // unit's scores are computed.
     float best1 = 0.0f, best2 = 0.0f;   // reference peak = max(0, masked max)
     int bk1 = -1, bk2 = -1;
-    float s2a = 0.f, s2b = 0.f;
+    float2 s2 = make_float2(0.0f, 0.0f);
     {
         float2 b[N2];
         const float2* src = tile + v * F::VP + k1 * F::BP;
@@ -331,35 +325,34 @@ __device__ __forceinline__ void corr_col_tile(const CorrArgs& a, int u, int t, f
             bk1 = g1 ? k2 : bk1;
             best2 = g2 ? v2 : best2;
             bk2 = g2 ? k2 : bk2;
-            s2a = fmaf(v1, v1, s2a);
-            s2b = fmaf(v2, v2, s2b);
+            s2 = __ffma2_rn(val, val, s2);
         });
     }
-    // keys: value bits high, ~flat index low (among equal values the smallest
-    // index wins across threads; within one thread, the first in k2 order)
+    // Warp reductions: the peaks by integer reductions of the value bits (the
+    // peaks are not negative) and then of the smallest map index that has
+    // the value (within one thread, the first in k2 order); the sums in double,
+    // each half of the warp taking one template's after one exchange.  Shuffles
+    // share the pipe of the shared-memory exchange, the tighter one here.
     const int X = x + h < L ? x + h : x - h;
-    unsigned long long ka = 0ull, kb = 0ull;
-    if (bk1 >= 0) {
-        const int y = F::map_coord(k1, bk1);
-        const int Y = y + h < L ? y + h : y - h;
-        ka = argmax_key(best1, Y * L + X);
-    }
-    if (bk2 >= 0) {
-        const int y = F::map_coord(k1, bk2);
-        const int Y = y + h < L ? y + h : y - h;
-        kb = argmax_key(best2, Y * L + X);
-    }
-    // warp-level reduction
-    const double d2a = warp_sum((double)s2a), d2b = warp_sum((double)s2b);
-    ka = warp_max_u64(ka);
-    kb = warp_max_u64(kb);
+    auto map_index = [&](int k2) {
+        const int y = F::map_coord(k1, k2);
+        return (unsigned)((y + h < L ? y + h : y - h) * L + X);
+    };
+    const unsigned m1 = __float_as_uint(best1), m2 = __float_as_uint(best2);
+    const unsigned p1 = __reduce_max_sync(0xffffffffu, m1), p2 = __reduce_max_sync(0xffffffffu, m2);
+    const unsigned i1 = __reduce_min_sync(0xffffffffu, bk1 >= 0 && m1 == p1 ? map_index(bk1) : 0xffffffffu);
+    const unsigned i2 = __reduce_min_sync(0xffffffffu, bk2 >= 0 && m2 == p2 ? map_index(bk2) : 0xffffffffu);
+    const int lane = threadIdx.x & 31;
+    const bool second = lane >= 16;
+    double d = (second ? (double)s2.y : (double)s2.x) + __shfl_xor_sync(0xffffffffu, second ? (double)s2.x : (double)s2.y, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
     // one set of atomics per warp (published with the tile)
-    if ((threadIdx.x & 31) == 0) {
-        UnitAcc* ac = a.acc + 2 * (long long)u;
-        if (ka) atomicMax(&ac[0].key, ka);
-        atomicAdd(&ac[0].s2, d2a);
-        if (kb) atomicMax(&ac[1].key, kb);
-        atomicAdd(&ac[1].s2, d2b);
+    if ((lane & 15) == 0) {
+        UnitAcc* ac = a.acc + 2 * (long long)u + (second ? 1 : 0);
+        const unsigned peak = second ? p2 : p1;
+        if (peak) atomicMax(&ac->key, ((unsigned long long)peak << 32) | (unsigned long long)(~(second ? i2 : i1)));
+        atomicAdd(&ac->s2, d);
     }
 }
 
@@ -380,7 +373,7 @@ __device__ __forceinline__ UnitOut unit_score(const UnitAcc& ac, double s1, int 
 }
 __device__ __forceinline__ UnitOut unit_score(const UnitAcc& ac, int l) { return unit_score(ac, ac.s1, l); }
 
-// The counter whose completions `item` waits for (kDone of them), or nullptr.
+// The counter whose completions `item` waits for (T of them), or nullptr.
 template <int N2, int V>
 __device__ __forceinline__ const int* corr_dep(const CorrArgs& a, int item) {
     using C = CorrCfg<N2, V>;
@@ -401,17 +394,16 @@ __device__ __forceinline__ int2 corr_item_wp(const CorrArgs& a, int item, int to
     return (j < C::T && s < a.nu) ? __ldg(a.unit_wp + s) : make_int2(0, 0);
 }
 
-// Per-tile protocol: each warp checks the dependency of `item` before
-// working on it.
+// Each warp checks the dependency of `item` before working on it.
 template <int N2, int V>
 __device__ __forceinline__ void corr_wait_for(const CorrArgs& a, int item) {
     using C = CorrCfg<N2, V>;
     const int* p = corr_dep<N2, V>(a, item);
-    if (p) wait_counter_warp(p, C::kDone, a.error);
+    if (p) wait_counter_warp(p, C::T, a.error);
 }
 
-// Count a finished tile (or one warp's share of it, kWarpPub); the last
-// count of a unit's column pass computes its two scores.
+// Count a finished tile; the last count of a unit's column pass computes its
+// two scores.
 template <int N2, int V>
 __device__ __forceinline__ void corr_publish(const CorrArgs& a, int item) {
     using F = CorrCfg<N2, V>;
@@ -424,7 +416,7 @@ __device__ __forceinline__ void corr_publish(const CorrArgs& a, int item) {
     if (u < 0 || u >= a.nu) return;
     int prev;
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(prev) : "l"(&a.done_cols[u]) : "memory");
-    if (prev != F::kDone - 1) return;
+    if (prev != F::T - 1) return;
     const int2 wp = a.unit_wp[u];
     const UnitAcc* ac = a.acc + 2 * (long long)u;
     // sum of the map c1 + i c2 = L^2 S(0, 0), S = W conj(P)
@@ -453,7 +445,7 @@ __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCta
     extern __shared__ __align__(16) unsigned char smc[];
     float2* tile = reinterpret_cast<float2*>(smc);
     float2* twt = reinterpret_cast<float2*>(smc + SM::tile);
-    int* ish = reinterpret_cast<int*>(smc + SM::tile + SM::tw + SM::red);  // ring of 4 claimed items
+    int* ish = reinterpret_cast<int*>(smc + SM::tile + SM::tw);  // ring of 4 claimed items
     // inverse twiddles W_L^{-n2 k1} = exp(+2 pi i n2 k1 / L), table [k1][n2]
     for (int i = threadIdx.x; i < (F::kPfa ? 0 : 16 * N2); i += F::kThreads) {
         const int k1 = i / N2, n2 = i - k1 * N2;
@@ -463,45 +455,7 @@ __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCta
     }
     const uint2 ymask = corr_row_mask<N2, V>(a.yb0, a.yb1);
     const int total = (a.nu + a.lag) * 2 * F::T;
-    if constexpr (F::kWarpPub) {
-        // per-warp protocol: thread 0 claims the next item while the CTA works
-        // on the current one and resolves its dependency before the barrier
-        // that ends the current one (each warp has counted its share by then,
-        // thread 0's own warp included, so nothing of this CTA is pending)
-        if (threadIdx.x == 0) {
-            const int first = atomicAdd(a.next_item, 1);
-            const int* p = first < total ? corr_dep<N2, V>(a, first) : nullptr;
-            if (p) wait_counter(p, F::kDone, a.error);
-            ish[0] = first;
-        }
-        __syncthreads();
-        int item = ish[0];
-        for (int iter = 1; item < total; ++iter) {
-            int nxt = 0;
-            if (threadIdx.x == 0) nxt = atomicAdd(a.next_item, 1);  // consumed after the tile
-            const int s = item / (2 * F::T), j = item - s * (2 * F::T);
-            if (j < F::T) {
-                if (s < a.nu) corr_row_tile<N2, V>(a, s, j, tile, twt, a.unit_wp[s]);
-            } else {
-                const int u = s - a.lag;
-                if (u >= 0 && u < a.nu) corr_col_tile<N2, V>(a, u, j - F::T, tile, twt, ymask);
-            }
-            __syncwarp();  // the warp's stores and atomics before its count
-            if ((threadIdx.x & 31) == 0) corr_publish<N2, V>(a, item);
-            if (threadIdx.x == 0) {
-                const int* p = nxt < total ? corr_dep<N2, V>(a, nxt) : nullptr;
-                if (p) wait_counter(p, F::kDone, a.error);
-                ish[iter & 3] = nxt;
-            }
-            // the tile buffer is free and the next item (dependency satisfied)
-            // published; slot iter & 3 is not rewritten before every thread has
-            // passed at least one more barrier
-            __syncthreads();
-            item = ish[iter & 3];
-        }
-        return;
-    }
-    // per-tile protocol: the CTA always holds its current item and the next one
+    // the CTA always holds its current item and the next one
     if (threadIdx.x == kPub) {
         ish[0] = atomicAdd(a.next_item, 1);
         ish[1] = atomicAdd(a.next_item, 1);
@@ -513,8 +467,8 @@ __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCta
         // the unit's (window, pair) is read-only in this launch: its load is
         // issued before the dependency wait and overlaps it
         const int2 wp = corr_item_wp<N2, V>(a, item, total);
-        corr_wait_for<N2, V>(a, item);
         const int s = item / (2 * F::T), j = item - s * (2 * F::T);
+        corr_wait_for<N2, V>(a, item);
         if (j < F::T) {
             if (s < a.nu) corr_row_tile<N2, V>(a, s, j, tile, twt, wp);
         } else {

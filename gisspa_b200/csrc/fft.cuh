@@ -47,23 +47,21 @@ __host__ __device__ __forceinline__ void dft2(float2& a0, float2& a1) {
 template <bool kInv>
 __host__ __device__ __forceinline__ void dft3(float2& a0, float2& a1, float2& a2) {
     const float s = 0.86602540378443864676f;
-    float2 t1 = cadd(a1, a2);
-    float2 t2 = make_float2(a0.x - 0.5f * t1.x, a0.y - 0.5f * t1.y);
-    float2 d = csub(a1, a2);
-    float2 rot = cscale(mul_mi<kInv>(d), s);
+    const float2 t1 = cadd(a1, a2), d = csub(a1, a2);
+    const float2 t2 = cfma(t1, -0.5f, a0);
     a0 = cadd(a0, t1);
-    a1 = cadd(t2, rot);
-    a2 = csub(t2, rot);
+    a1 = cfma_mi<kInv>(t2, d, s);
+    a2 = cfma_mi<!kInv>(t2, d, s);
 }
 
 template <bool kInv>
 __host__ __device__ __forceinline__ void dft4(float2& a0, float2& a1, float2& a2, float2& a3) {
-    float2 s02 = cadd(a0, a2), d02 = csub(a0, a2);
-    float2 s13 = cadd(a1, a3), d13 = mul_mi<kInv>(csub(a1, a3));
+    const float2 s02 = cadd(a0, a2), d02 = csub(a0, a2);
+    const float2 s13 = cadd(a1, a3), d13 = csub(a1, a3);
     a0 = cadd(s02, s13);
     a2 = csub(s02, s13);
-    a1 = cadd(d02, d13);
-    a3 = csub(d02, d13);
+    a1 = cadd_mi<kInv>(d02, d13);
+    a3 = cadd_mi<!kInv>(d02, d13);
 }
 
 template <bool kInv>
@@ -72,20 +70,18 @@ __host__ __device__ __forceinline__ void dft5(float2& a0, float2& a1, float2& a2
     const float c2 = -0.80901699437494742410f;  // cos(4 pi / 5)
     const float s1 = 0.95105651629515357212f;   // sin(2 pi / 5)
     const float s2 = 0.58778525229247312917f;   // sin(4 pi / 5)
-    float2 p14 = cadd(a1, a4), m14 = csub(a1, a4);
-    float2 p23 = cadd(a2, a3), m23 = csub(a2, a3);
-    float2 b1 = make_float2(a0.x + c1 * p14.x + c2 * p23.x, a0.y + c1 * p14.y + c2 * p23.y);
-    float2 b2 = make_float2(a0.x + c2 * p14.x + c1 * p23.x, a0.y + c2 * p14.y + c1 * p23.y);
+    const float2 p14 = cadd(a1, a4), m14 = csub(a1, a4);
+    const float2 p23 = cadd(a2, a3), m23 = csub(a2, a3);
+    const float2 b1 = cfma(p23, c2, cfma(p14, c1, a0));
+    const float2 b2 = cfma(p23, c1, cfma(p14, c2, a0));
     // forward: X1 = b1 - i(s1 m14 + s2 m23), X2 = b2 - i(s2 m14 - s1 m23)
-    float2 e1 = make_float2(s1 * m14.x + s2 * m23.x, s1 * m14.y + s2 * m23.y);
-    float2 e2 = make_float2(s2 * m14.x - s1 * m23.x, s2 * m14.y - s1 * m23.y);
-    e1 = mul_mi<kInv>(e1);
-    e2 = mul_mi<kInv>(e2);
+    const float2 e1 = cfma(m23, s2, cscale(m14, s1));
+    const float2 e2 = cfma(m23, -s1, cscale(m14, s2));
     a0 = cadd(a0, cadd(p14, p23));
-    a1 = cadd(b1, e1);
-    a4 = csub(b1, e1);
-    a2 = cadd(b2, e2);
-    a3 = csub(b2, e2);
+    a1 = cadd_mi<kInv>(b1, e1);
+    a4 = cadd_mi<!kInv>(b1, e1);
+    a2 = cadd_mi<kInv>(b2, e2);
+    a3 = cadd_mi<!kInv>(b2, e2);
 }
 
 template <bool kInv>
@@ -96,20 +92,16 @@ __host__ __device__ __forceinline__ void dft8(float2* a) {
     float2 o0 = a[1], o1 = a[3], o2 = a[5], o3 = a[7];
     dft4<kInv>(e0, e1, e2, e3);
     dft4<kInv>(o0, o1, o2, o3);
-    // w8^1 = h(1 -+ i), w8^2 = -+i, w8^3 = h(-1 -+ i)
-    float2 w1o1 = kInv ? make_float2(h * (o1.x - o1.y), h * (o1.x + o1.y))
-                       : make_float2(h * (o1.x + o1.y), h * (o1.y - o1.x));
-    float2 w2o2 = mul_mi<kInv>(o2);
-    float2 w3o3 = kInv ? make_float2(-h * (o3.x + o3.y), h * (o3.x - o3.y))
-                       : make_float2(h * (o3.y - o3.x), -h * (o3.x + o3.y));
+    // w8^1 = h(1 -+ i), w8^2 = -+i, w8^3 = -h(1 +- i)
+    const float2 u1 = cadd_mi<kInv>(o1, o1), u3 = cadd_mi<!kInv>(o3, o3);
     a[0] = cadd(e0, o0);
     a[4] = csub(e0, o0);
-    a[1] = cadd(e1, w1o1);
-    a[5] = csub(e1, w1o1);
-    a[2] = cadd(e2, w2o2);
-    a[6] = csub(e2, w2o2);
-    a[3] = cadd(e3, w3o3);
-    a[7] = csub(e3, w3o3);
+    a[1] = cfma(u1, h, e1);
+    a[5] = cfma(u1, -h, e1);
+    a[2] = cadd_mi<kInv>(e2, o2);
+    a[6] = cadd_mi<!kInv>(e2, o2);
+    a[3] = cfma(u3, -h, e3);
+    a[7] = cfma(u3, h, e3);
 }
 
 // One Stockham stage of radix R for butterfly j of one vector.

@@ -153,12 +153,11 @@ __host__ __device__ __forceinline__ void dft_prime(float2* a) {
         static_for<H>([&](auto jc) {
             constexpr int j = decltype(jc)::value + 1;
             constexpr float cj = (float)cos2pi(j * k, R), sj = (float)sin2pi(j * k, R);
-            c = make_float2(fmaf(cj, s[j].x, c.x), fmaf(cj, s[j].y, c.y));
-            e = j == 1 ? cscale(d[j], sj) : make_float2(fmaf(sj, d[j].x, e.x), fmaf(sj, d[j].y, e.y));
+            c = cfma(s[j], cj, c);
+            e = j == 1 ? cscale(d[j], sj) : cfma(d[j], sj, e);
         });
-        e = mul_mi<kInv>(e);
-        a[OFF + k * S] = cadd(c, e);
-        a[OFF + (R - k) * S] = csub(c, e);
+        a[OFF + k * S] = cadd_mi<kInv>(c, e);
+        a[OFF + (R - k) * S] = cadd_mi<!kInv>(c, e);
     });
 }
 
