@@ -67,7 +67,16 @@ struct CorrArgs {
     int yb0, yb1;            // border interval of unshifted indices (both axes)
     int pairs;               // template pairs per angle
     long long out_stride;    // results per angle (windows x templates)
+    // norm_type 1 (kCorrMoments, kCorrBlocks) instead of acc and out:
+    float2* moments;           // per window and map pixel: sums, then (mean, 1 / deviation)
+    unsigned long long* keys;  // per angle, window, template: nblk block maxima
+    int nblk, nw;
+    float inv_l2;
 };
+
+// What the column tiles do with the maps: score them; add them into the
+// per-pixel moments; z-score them and keep every 1024-element block's maximum.
+enum CorrEpi { kCorrScore, kCorrMoments, kCorrBlocks };
 
 // Results slot of template q (0, 1) of pair index y = angle x pairs + pair
 // for window w, or -1 when the pair has no second template (odd count).
@@ -263,7 +272,89 @@ __device__ __forceinline__ uint2 corr_row_mask(int yb0, int yb1) {
     return m;
 }
 
+// norm_type 1, sweep 1: cc / l^2 and its square of both templates added into
+// the window's per-pixel sums (add_CCG_to_sum, GPU_func.cu:617-633), one 8-byte
+// reduction per pixel.  b: the thread's map column x, rows map_coord(k1, k2).
 template <int N2, int V>
+__device__ __forceinline__ void corr_moments(const CorrArgs& a, int u, int x, int k1, const float2 (&b)[N2]) {
+    using F = CorrCfg<N2, V>;
+    constexpr int L = F::L, h = L / 2;
+    const int2 wp = __ldg(a.unit_wp + u);
+    const bool two = 2 * (wp.y % a.pairs) + 1 < a.ntmpl;
+    const float s = ((L / 2) % 2 == 0) ? a.inv_l2 : -a.inv_l2;
+    float2* mom = a.moments + (long long)wp.x * a.L2 + (x + h < L ? x + h : x - h);
+    rf::static_for<N2>([&](auto kc) {
+        constexpr int k2 = decltype(kc)::value;
+        const float2 c = cscale(b[rf::rpos<N2>(k2)], s);
+        const int y = F::map_coord(k1, k2), Y = y + h < L ? y + h : y - h;
+        atomicAdd(mom + (long long)Y * L, two ? make_float2(c.x + c.y, fmaf(c.y, c.y, c.x * c.x)) : make_float2(c.x, c.x * c.x));
+    });
+}
+
+// norm_type 1, sweep 2: z-scores against the window's per-pixel (mean, 1 /
+// deviation) and the maximum of every 1024-element block of the flat map
+// (update_CCG + get_peak_pos, GPU_func.cu:648-662, 711-745).  The tile's z go
+// through the tile buffer (l rows of 16, both templates), so that a thread
+// takes a whole 16-column run of one row, which lies inside one block (l is a
+// multiple of 32); runs of one block in neighbouring lanes are combined before
+// the one atomic.  One atomic per map value instead cost 173 us per
+// 12 pairs at window 512.  The 16-byte pieces of a row are rotated by its
+// index to keep both sides free of bank conflicts.
+template <int N2, int V>
+__device__ __forceinline__ void corr_blocks(const CorrArgs& a, int u, int v, int x, int k1, const float2 (&b)[N2],
+                                            float* z) {
+    using F = CorrCfg<N2, V>;
+    static_assert(V == 16 && !F::kPfa, "16-column runs in natural order");
+    constexpr int L = F::L, h = L / 2;
+    const int2 wp = __ldg(a.unit_wp + u);
+    const int an = wp.y / a.pairs, p = wp.y - an * a.pairs;
+    const float s = ((L / 2) % 2 == 0) ? a.inv_l2 : -a.inv_l2;
+    const int X = x + h < L ? x + h : x - h;
+    const float2* mom = a.moments + (long long)wp.x * a.L2 + X;
+    __syncthreads();  // every read of the tile's columns is done
+    rf::static_for<N2>([&](auto kc) {
+        constexpr int k2 = decltype(kc)::value;
+        const int y = k1 + 16 * k2, Y = y + h < L ? y + h : y - h;
+        const float2 m = __ldg(mom + (long long)Y * L);
+        const float2 c = cscale(b[rf::rpos<N2>(k2)], s);
+        float* o = z + Y * 16 + (((v >> 2) ^ ((Y >> 1) & 3)) << 2) + (v & 3);
+        o[0] = (c.x - m.x) * m.y;
+        o[L * 16] = (c.y - m.x) * m.y;
+    });
+    __syncthreads();
+    const int X0 = X & ~15;  // V = 16: the tile's columns start at a multiple of 16
+    for (int r = threadIdx.x; r < 2 * L; r += F::kThreads) {  // L is a multiple of 32: no partial warps
+        const int q = r >= L, Y = q ? r - L : r, J = 2 * p + q;
+        const float4* row = reinterpret_cast<const float4*>(z + (q * L + Y) * 16);
+        float best = __int_as_float(0xff800000);  // -inf
+        int at = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float4 w = row[c ^ ((Y >> 1) & 3)];
+            if (w.x > best) { best = w.x; at = 4 * c; }
+            if (w.y > best) { best = w.y; at = 4 * c + 1; }
+            if (w.z > best) { best = w.z; at = 4 * c + 2; }
+            if (w.w > best) { best = w.w; at = 4 * c + 3; }
+        }
+        const int pos = Y * L + X0 + at, blk = (Y * L + X0) >> 10;
+        const unsigned bits = __float_as_uint(best);
+        unsigned long long key =
+            ((unsigned long long)((bits & 0x80000000u) ? ~bits : bits | 0x80000000u) << 32) | (unsigned)~pos;
+        // rows of one block sit in neighbouring lanes (a warp holds rows of one template)
+#pragma unroll
+        for (int o = 1; o < 32; o *= 2) {
+            if (o * L >= 1024) break;
+            const unsigned long long k = __shfl_down_sync(0xffffffffu, key, o);
+            const int kb = __shfl_down_sync(0xffffffffu, blk, o);
+            if ((threadIdx.x & 31) + o < 32 && kb == blk) key = k > key ? k : key;
+        }
+        const int before = __shfl_up_sync(0xffffffffu, blk, 1);
+        if (J < a.ntmpl && ((threadIdx.x & 31) == 0 || before != blk))
+            atomicMax(a.keys + (((long long)an * a.nw + wp.x) * a.ntmpl + J) * a.nblk + blk, key);
+    }
+}
+
+template <int N2, int V, CorrEpi kEpi>
 __device__ __forceinline__ void corr_col_tile(const CorrArgs& a, int u, int t, float2* tile, const float2* twt,
                                               uint2 ymask) {
     using F = CorrCfg<N2, V>;
@@ -302,6 +393,16 @@ __device__ __forceinline__ void corr_col_tile(const CorrArgs& a, int u, int t, f
     const int x = F::kPfa ? F::map_coord((c0 + v) & 15, (c0 + v) >> 4) : c0 + v;
     // column outside the border: the rows of ymask count, else none
     if ((unsigned)(x - a.yb0) <= (unsigned)(a.yb1 - a.yb0)) ymask = make_uint2(0u, 0u);
+    if constexpr (kEpi != kCorrScore) {
+        float2 b[N2];
+        const float2* src = tile + v * F::VP + k1 * F::BP;
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) b[n2] = src[n2];
+        rf::rfft<N2, 1, true>(b);
+        if constexpr (kEpi == kCorrMoments) corr_moments<N2, V>(a, u, x, k1, b);
+        else corr_blocks<N2, V>(a, u, v, x, k1, b, reinterpret_cast<float*>(tile));
+        return;
+    }
     constexpr float sgn = ((L / 2) % 2 == 0) ? 1.0f : -1.0f;
     // Per point the border-masked maximum with its k2 and the sum of squares;
     // the map's plain sum is L^2 times its spectrum's DC term, taken when the
@@ -404,7 +505,7 @@ __device__ __forceinline__ void corr_wait_for(const CorrArgs& a, int item) {
 
 // Count a finished tile; the last count of a unit's column pass computes its
 // two scores.
-template <int N2, int V>
+template <int N2, int V, CorrEpi kEpi>
 __device__ __forceinline__ void corr_publish(const CorrArgs& a, int item) {
     using F = CorrCfg<N2, V>;
     const int s = item / (2 * F::T), j = item - s * (2 * F::T);
@@ -414,6 +515,10 @@ __device__ __forceinline__ void corr_publish(const CorrArgs& a, int item) {
     }
     const int u = s - a.lag;
     if (u < 0 || u >= a.nu) return;
+    if constexpr (kEpi != kCorrScore) {
+        asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(&a.done_cols[u]) : "memory");
+        return;
+    }
     int prev;
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(prev) : "l"(&a.done_cols[u]) : "memory");
     if (prev != F::T - 1) return;
@@ -437,7 +542,7 @@ __device__ __forceinline__ void corr_publish(const CorrArgs& a, int item) {
     }
 }
 
-template <int N2, int V>
+template <int N2, int V, CorrEpi kEpi = kCorrScore>
 __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCtasPerSm) k_corr_persistent(CorrArgs a) {
     using F = CorrCfg<N2, V>;
     using SM = CorrSmem<N2, V>;
@@ -473,7 +578,7 @@ __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCta
             if (s < a.nu) corr_row_tile<N2, V>(a, s, j, tile, twt, wp);
         } else {
             const int u = s - a.lag;
-            if (u >= 0 && u < a.nu) corr_col_tile<N2, V>(a, u, j - F::T, tile, twt, ymask);
+            if (u >= 0 && u < a.nu) corr_col_tile<N2, V, kEpi>(a, u, j - F::T, tile, twt, ymask);
         }
         // the claim made after the previous barrier enters the ring only now,
         // so the publisher's warp did not wait for the atomic's return
@@ -485,7 +590,7 @@ __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCta
         __syncthreads();
         const int next = ish[(iter + 1) & 3];
         if (threadIdx.x == kPub) {
-            corr_publish<N2, V>(a, item);
+            corr_publish<N2, V, kEpi>(a, item);
             claimed = atomicAdd(a.next_item, 1);  // for slot (iter + 2) & 3
         }
         item = next;

@@ -298,12 +298,17 @@ int run_win(gs_ctx* ctx, int l, int nimg, cudaError_t (*launch)(const float2*, i
     return win_status(ctx, launch(pl->tw, nimg, io, ctx->stream), "window transform");
 }
 
-// Persistent FP32 correlation with tiles of `tile` vectors (16 or 8).
-int launch_corr(gs_ctx* ctx, int l, int tile, const CorrArgs& a) {
+// Persistent FP32 correlation with tiles of `tile` vectors (16 or 8; the
+// norm_type 1 epilogues: 16).
+int launch_corr(gs_ctx* ctx, int l, int tile, const CorrArgs& a, CorrEpi epi = kCorrScore) {
     const WinOps* w = win_of(ctx, l);
-    if (!w) return set_err(ctx, GS_ERR_UNSUPPORTED, "no persistent kernel for %d", l);
+    if (!w || (epi != kCorrScore && !w->corr_moments))
+        return set_err(ctx, GS_ERR_UNSUPPORTED, "no persistent kernel for %d", l);
     bool fits = true;
-    const cudaError_t e = w->corr(a, tile, ctx->corr_ctas_override, ctx->stream, &fits);
+    const int ctas = ctx->corr_ctas_override;
+    const cudaError_t e = epi == kCorrScore ? w->corr(a, tile, ctas, ctx->stream, &fits)
+                          : epi == kCorrMoments ? w->corr_moments(a, ctas, ctx->stream, &fits)
+                                                : w->corr_blocks(a, ctas, ctx->stream, &fits);
     if (!fits) return set_err(ctx, GS_ERR_UNSUPPORTED, "persistent kernel does not fit on an SM");
     return win_status(ctx, e, "persistent correlation");
 }
@@ -484,8 +489,6 @@ static int corr_rows(gs_ctx* ctx, const float2* Ww, const float2* TS, float2* R)
 template <class Epi>
 static int corr_cols(gs_ctx* ctx, const float2* R, const Epi& epi) {
     const int l = ctx->l, Np = (ctx->ntmpl + 1) / 2;
-    const long long l2 = (long long)l * l;
-    if (fast_ok(ctx, l)) return run_fast<true, true>(ctx, l, Np, F16Norm1<Epi>{R, epi, l, l2});
     return run_fft<true>(ctx, l, cols_of(l, l), Np, IoNorm1<Epi>{R, epi});
 }
 
@@ -496,9 +499,55 @@ static int corr_cols(gs_ctx* ctx, const float2* R, const Epi& epi) {
 // and reports the maximum of every 1024-element block (main.cu:770-820).
 // Picks come out in the reference's order: angle, window row, window
 // column, template, block.
-static int search_norm1(gs_ctx* ctx, const float2* W, int nx, int ny, const std::vector<int>& offx,
-                        const std::vector<int>& offy, const std::vector<float>& angles, float* ms_spec,
-                        float* ms_corr, std::vector<gs_pick>* out) {
+static void norm1_picks(std::vector<BlockPickDev>& hp, const std::vector<float>& angles, int N, int nw, int bx, int nblk,
+                        std::vector<gs_pick>* out) {
+    std::sort(hp.begin(), hp.end(), [](const BlockPickDev& a, const BlockPickDev& b) { return a.key < b.key; });
+    out->resize(hp.size());
+    for (size_t k = 0; k < hp.size(); ++k) {
+        const long long u = hp[k].key / nblk;
+        const int J = (int)(u % N);
+        const int w = (int)((u / N) % nw);
+        const int ai = (int)(u / ((long long)N * nw));
+        gs_pick& o = (*out)[k];
+        o.angle_index = ai;
+        o.phi = printed_phi(angles[ai]);
+        o.window_x = w % bx;
+        o.window_y = w / bx;
+        o.template_index = J;
+        o.center_x = hp[k].cx;
+        o.center_y = hp[k].cy;
+        o.score = hp[k].score;
+    }
+}
+
+// ctx->off: the window offsets of nx, then of ny (prep_micrograph uploaded them)
+static int norm1_compact(gs_ctx* ctx, long long nkeys, int nblk, int bx, int by, int nx, int ny, long long key0,
+                         std::vector<BlockPickDev>* hp) {
+    CK(cudaMemsetAsync(ctx->count.p, 0, sizeof(unsigned long long), ctx->stream));
+    k_norm1_compact<<<blocks_for(nkeys, 256), 256, 0, ctx->stream>>>(
+        P<unsigned long long>(ctx->units), nkeys, ctx->ntmpl, nblk, bx * by, bx, ctx->l, P<int>(ctx->off),
+        P<int>(ctx->off) + bx, ctx->p.d_m, nx, ny, ctx->p.thres, key0, P<BlockPickDev>(ctx->picks),
+        P<unsigned long long>(ctx->count));
+    ++ctx->counters.kernel_launches;
+    CKL();
+    unsigned long long cnt = 0;
+    CK(cudaMemcpyAsync(&cnt, ctx->count.p, sizeof cnt, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (cnt) {
+        const size_t o = hp->size();
+        hp->resize(o + cnt);
+        CK(cudaMemcpyAsync(hp->data() + o, ctx->picks.p, sizeof(BlockPickDev) * cnt, cudaMemcpyDeviceToHost,
+                           ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+    }
+    return GS_OK;
+}
+
+// Without the persistent kernel (other windows, GS_OPT_TWO_PASS,
+// GS_OPT_GENERIC_FFT): row and column launches per (angle, window).
+static int search_norm1_passes(gs_ctx* ctx, const float2* W, int nx, int ny, const std::vector<int>& offx,
+                               const std::vector<int>& offy, const std::vector<float>& angles, float* ms_spec,
+                               float* ms_corr, std::vector<gs_pick>* out) {
     const int l = ctx->l, N = ctx->ntmpl;
     const long long l2 = (long long)l * l;
     const int bx = (int)offx.size(), nw = bx * (int)offy.size(), na = (int)angles.size();
@@ -555,46 +604,17 @@ static int search_norm1(gs_ctx* ctx, const float2* W, int nx, int ny, const std:
         TRY(pair_spectra(ctx, angles[ai], TS));
         CK(cudaEventRecord(eb, ctx->stream));
         CK(cudaMemsetAsync(keys, 0, sizeof(unsigned long long) * nkeys * nw, ctx->stream));
-        CK(cudaMemsetAsync(ctx->count.p, 0, sizeof(unsigned long long), ctx->stream));
         for (int w = 0; w < nw; ++w) {
             TRY(corr_rows(ctx, W + (size_t)w * l2, TS, R));
             Norm1Blocks e{s1 + (size_t)w * l2, s2 + (size_t)w * l2, keys + (size_t)w * nkeys, l, N, nblk,
                           (float)l, sgn};
             TRY(corr_cols(ctx, R, e));
-            k_norm1_compact<<<blocks_for(nkeys, 256), 256, 0, ctx->stream>>>(
-                keys + (size_t)w * nkeys, N, nblk, l, offx[w % bx], offy[w / bx], ctx->p.d_m, nx, ny, ctx->p.thres,
-                ((long long)ai * nw + w) * nkeys, P<BlockPickDev>(ctx->picks), P<unsigned long long>(ctx->count),
-                nkeys * nw);
-            ++ctx->counters.kernel_launches;
-            CKL();
         }
         CK(cudaEventRecord(ec, ctx->stream));
+        TRY(norm1_compact(ctx, nkeys * nw, nblk, bx, (int)offy.size(), nx, ny, (long long)ai * nw * nkeys, &hp));
         TRY(elapsed());
-        unsigned long long cnt = 0;
-        CK(cudaMemcpy(&cnt, ctx->count.p, sizeof cnt, cudaMemcpyDeviceToHost));
-        if (cnt) {
-            const size_t o = hp.size();
-            hp.resize(o + cnt);
-            CK(cudaMemcpy(hp.data() + o, ctx->picks.p, sizeof(BlockPickDev) * cnt, cudaMemcpyDeviceToHost));
-        }
     }
-    std::sort(hp.begin(), hp.end(), [](const BlockPickDev& a, const BlockPickDev& b) { return a.key < b.key; });
-    out->resize(hp.size());
-    for (size_t k = 0; k < hp.size(); ++k) {
-        const long long u = hp[k].key / nblk;
-        const int J = (int)(u % N);
-        const int w = (int)((u / N) % nw);
-        const int ai = (int)(u / ((long long)N * nw));
-        gs_pick& o = (*out)[k];
-        o.angle_index = ai;
-        o.phi = printed_phi(angles[ai]);
-        o.window_x = w % bx;
-        o.window_y = w / bx;
-        o.template_index = J;
-        o.center_x = hp[k].cx;
-        o.center_y = hp[k].cy;
-        o.score = hp[k].score;
-    }
+    norm1_picks(hp, angles, N, nw, bx, nblk, out);
     return GS_OK;
 }
 
@@ -1179,6 +1199,52 @@ struct CorrTuning {
     int slots, lag, window_block, ctas, tile;
 };
 
+// Scheduling of the persistent correlation before any tuning: the options
+// that were set, else by window and precision.
+static int default_tuning(gs_ctx* ctx, bool tc2, CorrTuning* out) {
+    const gs_params& p = ctx->p;
+    const int l = ctx->l;
+    CorrTuning& tune = *out;
+    tune = CorrTuning{ctx->corr_slots, ctx->corr_lag, ctx->window_block, ctx->corr_ctas, ctx->corr_tile};
+    // the all-tensor-core kernel keeps about twice as many items in flight
+    // (five pipelines per SM, items claimed in pairs): its own defaults
+    // unless the caller set the ring explicitly
+    if (tc2 && !ctx->corr_ring_set) {
+        tune.slots = 24;
+        tune.lag = 12;
+    }
+    // window 512, FP32 kernel: the autotuner's choice on both measured
+    // workloads there (the reference's 1024^2 case, 34.6 against 32.6
+    // micrographs/s, and the 32-micrograph batch): 8-vector tiles, a deeper
+    // ring and blocks of 8 windows, unless the caller set them
+    if (l == 512 && p.precision == GS_PREC_FP32) {
+        if (!ctx->corr_ring_set) {
+            tune.slots = 32;
+            tune.lag = 10;
+        }
+        if (!ctx->window_block_set) tune.window_block = 8;
+        if (!ctx->corr_tile_set) tune.tile = 8;
+    } else if (win_of(ctx, l) && p.precision == GS_PREC_FP32 && !fast_ok(ctx, l)) {
+        // other windows: the smaller the window, the fewer tiles a unit has
+        // and the more units the resident CTAs hold at once, so the ring goes
+        // by them.  A unit's column tiles are queued 2.5 times as many items
+        // after its row tiles as there are CTAs (window 128: 12.5 ms against
+        // 56.9 with 0.6 times; 320: 11.6 against 36.3; 640: 27.8 against
+        // 78.3), and 2.2 slots per unit of lag leave the row tiles room
+        // (1.6: up to 1.8 times slower).  8-vector tiles win by 1 to 4 % up
+        // to window 576, 16-vector ones by 2 to 25 % above it.
+        if (!ctx->corr_tile_set) tune.tile = l <= 576 ? 8 : 16;
+        if (!ctx->corr_ring_set) {
+            int nsm = 0;
+            CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+            const int ctas = nsm * win_of(ctx, l)->threads_per_sm / (16 * tune.tile), tiles = l / tune.tile;
+            tune.lag = (5 * ctas + 4 * tiles - 1) / (4 * tiles);
+            tune.slots = (11 * tune.lag + 4) / 5;
+        }
+    }
+    return GS_OK;
+}
+
 // Unit order: angle-major over the launch's `angles` angles (pair index
 // angle x Np + pair); within an angle blocks of window_block windows, inside
 // a block pair-major.
@@ -1198,17 +1264,25 @@ static int upload_unit_order(gs_ctx* ctx, int NW, int Np, int wbk, int limit, in
     return GS_OK;
 }
 
+// A norm_type 1 launch: sweep 1 (keys null) adds into the moments, sweep 2
+// takes block maxima.
+struct Norm1Launch {
+    float2* moments;
+    unsigned long long* keys;
+    int nblk, nw;
+};
+
 // One persistent correlation launch over the first nu units (the template-pair
 // spectra of the launch's angles already in TS, angle after angle), results
 // to out, out_stride results per angle.
 static int corr_launch(gs_ctx* ctx, const float2* W, const float2* TS, int nu, const CorrTuning& t, UnitOut* out,
-                       long long out_stride = 0) {
+                       long long out_stride = 0, const Norm1Launch* norm1 = nullptr) {
     const int l = ctx->l;
     const long long l2 = (long long)l * l;
     int* cnt = P<int>(ctx->dep_counters);
     CK(cudaMemsetAsync(cnt, 0, sizeof(int) * (2 * (size_t)nu + 4), ctx->stream));
-    CK(cudaMemsetAsync(ctx->pacc.p, 0, sizeof(UnitAcc) * 2 * (size_t)nu, ctx->stream));
-    CorrArgs ca;
+    if (!norm1) CK(cudaMemsetAsync(ctx->pacc.p, 0, sizeof(UnitAcc) * 2 * (size_t)nu, ctx->stream));
+    CorrArgs ca{};
     ca.W = W; ca.P = TS; ca.R = P<float2>(ctx->scratch);
     ca.unit_wp = P<int2>(ctx->unit_wp);
     ca.done_rows = cnt; ca.done_cols = cnt + nu;
@@ -1230,6 +1304,14 @@ static int corr_launch(gs_ctx* ctx, const float2* W, const float2* TS, int nu, c
         if (ca.yb1 < ca.yb0) { ca.yb0 = 1; ca.yb1 = 0; }
     }
     ctx->corr_ctas_override = t.ctas;
+    if (norm1) {
+        ca.moments = norm1->moments;
+        ca.keys = norm1->keys;
+        ca.nblk = norm1->nblk;
+        ca.nw = norm1->nw;
+        ca.inv_l2 = (float)(1.0 / (double)l2);
+        return launch_corr(ctx, l, 16, ca, norm1->keys ? kCorrBlocks : kCorrMoments);
+    }
     if (ctx->p.precision == GS_PREC_FP32) return launch_corr(ctx, l, t.tile, ca);
     if (ctx->p.precision == GS_PREC_TC_FULL || ctx->p.precision == GS_PREC_TC_FULL_1P) {
         if (l != 720) return set_err(ctx, GS_ERR_UNSUPPORTED, "the all-tensor-core path takes window 720 (got %d)", l);
@@ -1329,7 +1411,7 @@ static int autotune(gs_ctx* ctx, const float2* W, const float2* TS, int NW, Corr
 
 // Item indices of one persistent launch over n units (2 x l/8 tiles per
 // unit) must fit an int.
-static bool units_fit(int l, long long n) { return (n + 64) * 2 * (l / 8) < (1ll << 31); }
+static bool units_fit(int l, long long n) { return n < (1ll << 31) && (n + 64) * 2 * (l / 8) < (1ll << 31); }
 
 // In-plane angles per persistent launch before any tuning: the option's
 // count, else enough angles for about kUnitsPerLaunch units (a launch's
@@ -1363,6 +1445,93 @@ static int upload_rotations(gs_ctx* ctx, const std::vector<float>& angles) {
     for (int i = 0; i < na; ++i) cs[i] = rotation_cs(angles[i]);
     TRY(ensure(ctx, ctx->rot_cs, sizeof(float2) * cs.size()));
     CK(cudaMemcpy(ctx->rot_cs.p, cs.data(), sizeof(float2) * na, cudaMemcpyHostToDevice));
+    return GS_OK;
+}
+
+// norm_type 1 on the persistent kernel: both sweeps run over groups of angles
+// like the norm_type 0 search, their column tiles doing the per-pixel sums and
+// the block maxima.
+static int search_norm1(gs_ctx* ctx, const float2* W, int nx, int ny, const std::vector<int>& offx,
+                        const std::vector<int>& offy, const std::vector<float>& angles, float* ms_spec,
+                        float* ms_corr, std::vector<gs_pick>* out) {
+    const int l = ctx->l, N = ctx->ntmpl, Np = (N + 1) / 2;
+    const long long l2 = (long long)l * l;
+    const int bx = (int)offx.size(), by = (int)offy.size(), nw = bx * by, na = (int)angles.size();
+    const int nblk = (int)(l2 / 1024);
+    const long long per_angle = (long long)nw * N * nblk;  // block maxima
+    const long long nu = (long long)Np * nw;
+    const WinOps* ops = win_of(ctx, l);
+    if (ctx->two_pass || !ops || !ops->corr_moments || !units_fit(l, nu)) {
+        TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np));
+        TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * Np));
+        TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N));
+        TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np));
+        return search_norm1_passes(ctx, W, nx, ny, offx, offy, angles, ms_spec, ms_corr, out);
+    }
+    // angles per launch as in the norm_type 0 search, with the block maxima and
+    // their picks within 2 GiB
+    int A = launch_angles(ctx, (int)nu, na, false);
+    const long long key_bytes = (long long)(sizeof(unsigned long long) + sizeof(BlockPickDev)) * per_angle;
+    A = (int)std::max<long long>(1, std::min<long long>(A, (2ll << 30) / std::max(1ll, key_bytes)));
+    CorrTuning tune;
+    TRY(default_tuning(ctx, false, &tune));
+    tune.tile = 16;
+    TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np * A));
+    TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N * A));
+    TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np * A));
+    TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * tune.slots));
+    TRY(ensure(ctx, ctx->dep_counters, sizeof(int) * (2 * (size_t)nu * A + 4)));
+    TRY(ensure(ctx, ctx->flags, sizeof(int) * 4));
+    TRY(ensure(ctx, ctx->pacc, sizeof(float2) * l2 * nw));  // per-pixel moments
+    TRY(ensure(ctx, ctx->units, sizeof(unsigned long long) * per_angle * A));
+    TRY(ensure(ctx, ctx->picks, sizeof(BlockPickDev) * per_angle * A));
+    TRY(ensure(ctx, ctx->count, sizeof(unsigned long long)));
+    TRY(upload_rotations(ctx, angles));
+    TRY(upload_unit_order(ctx, nw, Np, tune.window_block, (int)(nu * A), A));
+    CK(cudaMemsetAsync(ctx->flags.p, 0, sizeof(int) * 4, ctx->stream));
+    CK(cudaMemsetAsync(ctx->pacc.p, 0, sizeof(float2) * l2 * nw, ctx->stream));
+    float2* TS = P<float2>(ctx->tspec);
+    Norm1Launch job{P<float2>(ctx->pacc), nullptr, nblk, nw};
+    cudaEvent_t ev[3];
+    for (auto& e : ev) CK(cudaEventCreate(&e));
+    struct EvGuard { cudaEvent_t* e; ~EvGuard() { for (int i = 0; i < 3; ++i) cudaEventDestroy(e[i]); } } guard{ev};
+    std::vector<BlockPickDev> hp;
+    constexpr int kImgs = 32768;
+    const int per = std::max(1, kImgs / Np);
+    for (int sweep = 0; sweep < 2; ++sweep) {
+        for (int a0 = 0; a0 < na; a0 += A) {
+            const int ag = std::min(A, na - a0);
+            CK(cudaEventRecord(ev[0], ctx->stream));
+            // one group holds all angles: sweep 1's spectra are still there
+            for (int k = 0; k < ag && !(sweep && ag == na); k += per)
+                TRY(pair_spectra_n(ctx, angles[a0 + k], P<float2>(ctx->rot_cs) + a0 + k, std::min(per, ag - k),
+                                   TS + (size_t)k * Np * l2, false));
+            CK(cudaEventRecord(ev[1], ctx->stream));
+            if (sweep) {
+                job.keys = P<unsigned long long>(ctx->units);
+                CK(cudaMemsetAsync(job.keys, 0, sizeof(unsigned long long) * per_angle * ag, ctx->stream));
+            }
+            TRY(corr_launch(ctx, W, TS, (int)(nu * ag), tune, nullptr, 0, &job));
+            CK(cudaEventRecord(ev[2], ctx->stream));
+            if (sweep) TRY(norm1_compact(ctx, per_angle * ag, nblk, bx, by, nx, ny, (long long)a0 * per_angle, &hp));
+            CK(cudaEventSynchronize(ev[2]));
+            float t1 = 0, t2 = 0;
+            cudaEventElapsedTime(&t1, ev[0], ev[1]);
+            cudaEventElapsedTime(&t2, ev[1], ev[2]);
+            *ms_spec += t1;
+            *ms_corr += t2;
+        }
+        if (!sweep) {
+            k_norm1_moments2<<<blocks_for(l2 * nw, 256), 256, 0, ctx->stream>>>(job.moments, l2 * nw, (float)N * (float)na);
+            ++ctx->counters.kernel_launches;
+            CKL();
+        }
+    }
+    int flag = 0;
+    CK(cudaMemcpyAsync(&flag, ctx->flags.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (flag) return set_err(ctx, GS_ERR_TIMEOUT, "correlation kernel: a bounded dependency wait gave up");
+    norm1_picks(hp, angles, N, nw, bx, nblk, out);
     return GS_OK;
 }
 
@@ -1459,43 +1628,8 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
     UnitOut* units = P<UnitOut>(ctx->units);
     FftPlan* plan = nullptr;
     TRY(get_plan(ctx, l, &plan));  // before any capture: plan creation copies synchronously
-    CorrTuning tune{ctx->corr_slots, ctx->corr_lag, ctx->window_block, ctx->corr_ctas, ctx->corr_tile};
-    // the all-tensor-core kernel keeps about twice as many items in flight
-    // (five pipelines per SM, items claimed in pairs): its own defaults
-    // unless the caller set the ring explicitly
-    if (tc2 && !ctx->corr_ring_set) {
-        tune.slots = 24;
-        tune.lag = 12;
-    }
-    // window 512, FP32 kernel: the autotuner's choice on both measured
-    // workloads there (the reference's 1024^2 case, 34.6 against 32.6
-    // micrographs/s, and the 32-micrograph batch): 8-vector tiles, a deeper
-    // ring and blocks of 8 windows, unless the caller set them
-    if (l == 512 && p.precision == GS_PREC_FP32) {
-        if (!ctx->corr_ring_set) {
-            tune.slots = 32;
-            tune.lag = 10;
-        }
-        if (!ctx->window_block_set) tune.window_block = 8;
-        if (!ctx->corr_tile_set) tune.tile = 8;
-    } else if (persistent && p.precision == GS_PREC_FP32 && !fast_ok(ctx, l)) {
-        // other windows: the smaller the window, the fewer tiles a unit has
-        // and the more units the resident CTAs hold at once, so the ring goes
-        // by them.  A unit's column tiles are queued 2.5 times as many items
-        // after its row tiles as there are CTAs (window 128: 12.5 ms against
-        // 56.9 with 0.6 times; 320: 11.6 against 36.3; 640: 27.8 against
-        // 78.3), and 2.2 slots per unit of lag leave the row tiles room
-        // (1.6: up to 1.8 times slower).  8-vector tiles win by 1 to 4 % up
-        // to window 576, 16-vector ones by 2 to 25 % above it.
-        if (!ctx->corr_tile_set) tune.tile = l <= 576 ? 8 : 16;
-        if (!ctx->corr_ring_set) {
-            int nsm = 0;
-            CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
-            const int ctas = nsm * win_of(ctx, l)->threads_per_sm / (16 * tune.tile), tiles = l / tune.tile;
-            tune.lag = (5 * ctas + 4 * tiles - 1) / (4 * tiles);
-            tune.slots = (11 * tune.lag + 4) / 5;
-        }
-    }
+    CorrTuning tune;
+    TRY(default_tuning(ctx, tc2, &tune));
     // window spectra in PfaCols order for the duration of the correlation,
     // natural order again afterwards (on every return path)
     struct PfaWindows {
@@ -1843,11 +1977,6 @@ static int search_many(gs_ctx* ctx, std::vector<MicPlan>& mics, std::vector<std:
     float t_spec = 0.0f, t_corr = 0.0f, kt[4] = {0, 0, 0, 0};
     res->assign(mics.size(), std::vector<gs_pick>());
     if (p.norm_type == 1) {
-        const int Np = (N + 1) / 2;
-        TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np));
-        TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * Np));
-        TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N));
-        TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np));
         const MicPlan& mp = mics[0];
         TRY(search_norm1(ctx, W, mp.nx, mp.ny, mp.offx, mp.offy, angles, &t_spec, &t_corr, &(*res)[0]));
     } else {

@@ -2,6 +2,10 @@
 // templates and angles (reference main.cu:718-821, 1170-1229;
 // GPU_func.cu:617-662, 711-745).
 //
+// Where the persistent correlation kernel exists its column tiles do both
+// sweeps (corr_moments, corr_blocks in corr.cuh); otherwise the per-window
+// passes with the epilogues below.
+//
 // Sweep 1 accumulates, per window pixel, sum and sum of squares of cc / l^2
 // over every template and angle (column-pass epilogue, float atomics like
 // the reference's float CCG_sum).  k_norm1_moments turns them into mean and
@@ -111,37 +115,46 @@ __global__ void k_norm1_moments(float* s1, float* s2, long long n, float total) 
     s2[i] = var;
 }
 
+// The same for the persistent kernel's interleaved sums: (mean, 1 / standard
+// deviation), 0 where the deviation is not positive (z = 0 there).
+__global__ void k_norm1_moments2(float2* mom, long long n, float total) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float2 s = mom[i];
+    const float avg = s.x / total;
+    const float sd = sqrtf(s.y / total - avg * avg);
+    mom[i] = make_float2(avg, sd > 0.0f ? 1.0f / sd : 0.0f);
+}
+
 struct BlockPickDev {
     long long key;  // ((angle * nw + window) * ntmpl + template) * nblk + block
     float cx, cy, score;
     int pad;
 };
 
-// Threshold + centre test of every (template, block) of one window
-// (main.cu:800-817).
-__global__ void k_norm1_compact(const unsigned long long* __restrict__ keys, int ntmpl, int nblk, int L,
-                                int offx, int offy, float d_m, int nx, int ny, float thres, long long key0,
-                                BlockPickDev* __restrict__ picks, unsigned long long* __restrict__ count,
-                                long long cap) {
+// Threshold + centre test of every (angle, window, template, block) key
+// (main.cu:800-817); the first key is key0 in the order of the picks.
+__global__ void k_norm1_compact(const unsigned long long* __restrict__ keys, long long nkeys, int ntmpl, int nblk,
+                                int nw, int bx, int L, const int* __restrict__ offx, const int* __restrict__ offy,
+                                float d_m, int nx, int ny, float thres, long long key0,
+                                BlockPickDev* __restrict__ picks, unsigned long long* __restrict__ count) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)ntmpl * nblk) return;
+    if (t >= nkeys) return;
     const unsigned long long k = keys[t];
     if (!k) return;
     const float z = float_unorder((unsigned)(k >> 32));
     if (!(z >= thres)) return;
+    const int w = (int)(t / ((long long)ntmpl * nblk) % nw);
     const int pos = (int)(~(unsigned)(k & 0xffffffffull));
-    const float cx = (float)(offx + pos % L), cy = (float)(offy + pos / L);
+    const float cx = (float)(offx[w % bx] + pos % L), cy = (float)(offy[w / bx] + pos / L);
     if (cx >= d_m && cx < (float)nx - d_m && cy >= d_m && cy < (float)ny - d_m) {
-        const unsigned long long slot = atomicAdd(count, 1ull);
-        if ((long long)slot < cap) {
-            BlockPickDev pk;
-            pk.key = key0 + t;
-            pk.cx = cx;
-            pk.cy = cy;
-            pk.score = z;
-            pk.pad = 0;
-            picks[slot] = pk;
-        }
+        BlockPickDev pk;
+        pk.key = key0 + t;
+        pk.cx = cx;
+        pk.cy = cy;
+        pk.score = z;
+        pk.pad = 0;
+        picks[atomicAdd(count, 1ull)] = pk;  // at most one per key: the array has nkeys places
     }
 }
 

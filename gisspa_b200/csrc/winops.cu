@@ -21,11 +21,11 @@ cudaError_t fft_launch(const float2* tw, int nimg, const IO& io, cudaStream_t st
     return cudaGetLastError();
 }
 
-template <int N2, int V>
+template <int N2, int V, CorrEpi kEpi = kCorrScore>
 cudaError_t corr_launch_v(const CorrArgs& a, int ctas, cudaStream_t st, bool* fits) {
     using C = CorrCfg<N2, V>;
     constexpr size_t smem = CorrSmem<N2, V>::bytes;
-    auto kern = k_corr_persistent<N2, V>;
+    auto kern = k_corr_persistent<N2, V, kEpi>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per_sm = 0, nsm = 0, dev = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
@@ -55,6 +55,10 @@ struct Ops {
                 WinOps o{};
                 o.threads_per_sm = CorrCfg<N2, 16>::kThreadsPerSm;
                 o.corr = corr_launch<N2>;
+                if constexpr (N2 % 2 == 0) {
+                    o.corr_moments = corr_launch_v<N2, 16, kCorrMoments>;
+                    o.corr_blocks = corr_launch_v<N2, 16, kCorrBlocks>;
+                }
                 if constexpr (N2 % 2 == 1) o.pair_rows_pfa = fft_launch<N2, false, false, F16PairNormPfa>;
                 o.pair_rows = fft_launch<N2, false, false, F16PairNorm>;
                 o.rows = fft_launch<N2, false, false, F16Complex<false>>;

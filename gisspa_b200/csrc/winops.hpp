@@ -13,6 +13,10 @@ struct WinOps {
     // most `ctas` resident CTAs per SM when ctas > 0; *fits = false (nothing
     // launched) when it does not fit on an SM
     cudaError_t (*corr)(const CorrArgs& a, int tile, int ctas, cudaStream_t st, bool* fits);
+    // the same with a norm_type 1 epilogue and 16-vector tiles; nullptr for odd
+    // N2 (norm_type 1 takes windows that are multiples of 32)
+    cudaError_t (*corr_moments)(const CorrArgs& a, int ctas, cudaStream_t st, bool* fits);
+    cudaError_t (*corr_blocks)(const CorrArgs& a, int ctas, cudaStream_t st, bool* fits);
     // forward transforms along rows: template pairs (natural or PfaCols column
     // order) and complex images in place
     cudaError_t (*pair_rows)(const float2* tw, int nimg, const F16PairNorm& io, cudaStream_t st);
