@@ -10,6 +10,7 @@
 #include "fastfft.cuh"
 #include "kernels.cuh"
 #include "norm1.cuh"
+#include "planfft.cuh"
 #include "pixmax.cuh"
 #include "tccorr.cuh"
 #include "tccorr2.cuh"
@@ -55,6 +56,7 @@ namespace {
 
 struct FftPlan {
     FftDesc d;
+    PlanDesc plan;  // of the in-place kernel (A = 0: none)
     float2* tw = nullptr;
 };
 
@@ -213,6 +215,14 @@ int get_plan(gs_ctx* ctx, int n, FftPlan** out) {
     CK(cudaMalloc(&pl.tw, sizeof(float2) * n));
     CK(cudaMemcpy(pl.tw, tw.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
     pl.d.tw = pl.tw;
+    bool dense = false;
+    if (plan_factors(n, &pl.plan.A, &pl.plan.B, &pl.plan.C, &dense)) {
+        pl.plan.n = n;
+        pl.plan.dense = dense ? 1 : 0;
+        pl.plan.tw = pl.tw;
+    } else {
+        pl.plan.A = 0;
+    }
     auto res = ctx->plans.emplace(n, pl);
     *out = &res.first->second;
     return GS_OK;
@@ -222,10 +232,40 @@ constexpr int kFftThreads = 256;
 constexpr size_t kFftSmemBudget = 96 * 1024;
 constexpr size_t kMaxSmem = 227 * 1024;
 
+// Vectors per CTA of the in-place kernel: three CTAs to an SM where that takes
+// 16 vectors, down to four (a 32-byte sector of neighbouring columns) with
+// fewer CTAs, and whatever fits beyond that.
+int plan_tile(PlanDesc* d, int nvec, bool columns) {
+    const size_t budgets[3] = {72 * 1024, 110 * 1024, 220 * 1024};
+    const int least[3] = {columns ? 8 : 1, columns ? 4 : 1, 1};
+    for (int i = 0; i < 3; ++i)
+        for (int t = 16; t >= least[i]; t /= 2) {
+            plan_layout(d, t);
+            if (plan_smem_bytes(*d, t) <= budgets[i]) return std::min(t, std::max(1, nvec));
+        }
+    return 0;
+}
+
 template <bool kInv, class IO>
 int run_fft(gs_ctx* ctx, int n, VecGeom g, int nimg, IO io, int max_tile = 16) {
     FftPlan* pl = nullptr;
     TRY(get_plan(ctx, n, &pl));
+    if (pl->plan.A && !ctx->generic_fft && nimg <= 65535) {
+        PlanDesc d = pl->plan;
+        int tile = plan_tile(&d, g.nvec, g.elem_stride != 1);
+        if (tile) {
+            tile = std::min(tile, max_tile);
+            plan_layout(&d, tile);
+            const size_t smem = plan_smem_bytes(d, tile);
+            auto kern = fft_plan_kernel<kInv, IO>;
+            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            kern<<<dim3((unsigned)((g.nvec + tile - 1) / tile), (unsigned)nimg), kFftThreads, smem, ctx->stream>>>(
+                d, g, tile, io);
+            ++ctx->counters.kernel_launches;
+            CKL();
+            return GS_OK;
+        }
+    }
     const size_t per = 2 * (size_t)(n + 1) * sizeof(float2);
     size_t tile = std::max<size_t>(1, kFftSmemBudget / per);
     if (per > kFftSmemBudget) tile = 1;
