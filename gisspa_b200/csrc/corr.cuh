@@ -78,14 +78,6 @@ struct CorrArgs {
 // per-pixel moments; z-score them and keep every 1024-element block's maximum.
 enum CorrEpi { kCorrScore, kCorrMoments, kCorrBlocks };
 
-// Results slot of template q (0, 1) of pair index y = angle x pairs + pair
-// for window w, or -1 when the pair has no second template (odd count).
-__device__ __forceinline__ long long unit_out_index(int y, int q, int w, int pairs, int ntmpl,
-                                                    long long out_stride) {
-    const int an = y / pairs, J = 2 * (y - an * pairs) + q;
-    return J < ntmpl ? an * out_stride + (long long)w * ntmpl + J : -1;
-}
-
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     int v;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -1624,6 +1624,10 @@ static int prefetch_pair_spectra(gs_ctx* ctx, int NW, const std::vector<float>& 
     return GS_OK;
 }
 
+// Row-pass maps of one chunked launch (correlate_all): enough units for many
+// CTAs per SM (window 300: 186 units, 3534 CTAs) while the maps stay in L2.
+constexpr long long kChunkBytes = 128ll << 20;
+
 // Correlation of every window with every template over all angles (the
 // angle loop of main.cu:1232-1257): per angle the template-pair spectra, then
 // either one persistent launch over all (window, pair) units or per-window
@@ -1649,7 +1653,11 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
     const int nu = Np * NW;
     if (!units_fit(l, nu))
         return set_err(ctx, GS_ERR_UNSUPPORTED, "too many (window, template pair) units in one search (%d)", nu);
-    int A = persistent ? launch_angles(ctx, nu, na, tc2) : 1;
+    // windows without a persistent kernel: row and column launches over chunks
+    // of units, unless one of the cross-check options asks for the per-window ones
+    const bool chunked = !persistent && !ctx->two_pass && !ctx->generic_fft;
+    const int chunk = (int)std::max<long long>(1, std::min<long long>(65535, kChunkBytes / (l2 * (long long)sizeof(float2))));
+    int A = persistent || chunked ? launch_angles(ctx, nu, na, tc2) : 1;
     // pair spectra of the first launch already enqueued on the side stream
     // (prefetch_pair_spectra): used when the group matches, else awaited
     // and recomputed
@@ -1725,6 +1733,10 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         // angle-major: a launch of fewer angles takes a prefix of this order
         TRY(upload_unit_order(ctx, NW, Np, tune.window_block, nu * A, A));
         TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * tune.slots));
+    } else if (chunked) {
+        TRY(upload_unit_order(ctx, NW, Np, tune.window_block, nu * A, A));
+        TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * std::min<long long>(chunk, (long long)nu * A)));
+        TRY(ensure(ctx, ctx->pacc, sizeof(UnitAcc) * 2 * (size_t)nu * A));
     } else {
         TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * Np));
     }
@@ -1739,8 +1751,10 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
     const float q_hi = (float)l - q_lo;
     const float sgn = ((l / 2) % 2 == 0) ? 1.0f : -1.0f;
     const bool timing = ctx->kernel_timing && !ctx->use_graph;
-    if (timing && (int)ctx->kev.size() < 4 * NW) {
-        while ((int)ctx->kev.size() < 4 * NW) {
+    // pairs of events per group of angles: one per window, or one per chunk
+    const int nev = chunked ? (int)(((long long)nu * A + chunk - 1) / chunk) : NW;
+    if (timing && (int)ctx->kev.size() < 4 * nev) {
+        while ((int)ctx->kev.size() < 4 * nev) {
             cudaEvent_t e;
             CK(cudaEventCreate(&e));
             ctx->kev.push_back(e);
@@ -1755,8 +1769,8 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
     long long k1n = 0, k2n = 0;
 
     bool capturing = false;  // enqueue_group is being captured into the graph
-    // the work of angles a0 .. a0 + ag - 1 (ag = 1 without the persistent
-    // kernel), enqueued on the context's stream: their pair spectra one
+    // the work of angles a0 .. a0 + ag - 1 (ag = 1 with the per-window launches),
+    // enqueued on the context's stream: their pair spectra one
     // after the other in TS, then one correlation launch over all their units
     auto enqueue_group = [&](int a0, int ag, bool rec) -> int {
         if (rec) CK(cudaEventRecord(ea, ctx->stream));
@@ -1789,6 +1803,29 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
             if (timing) CK(cudaEventRecord(ctx->kev[0], ctx->stream));
             TRY(corr_launch(ctx, W, TS, nu * ag, tune, units + (size_t)a0 * NW * N, (long long)NW * N));
             if (timing) CK(cudaEventRecord(ctx->kev[1], ctx->stream));
+            return GS_OK;
+        }
+        if (chunked) {
+            const int n = nu * ag;
+            UnitAcc* ua = P<UnitAcc>(ctx->pacc);
+            CK(cudaMemsetAsync(ua, 0, sizeof(UnitAcc) * 2 * (size_t)n, ctx->stream));
+            for (int u0 = 0, c = 0; u0 < n; u0 += chunk, ++c) {
+                const int nc = std::min(chunk, n - u0);
+                const int2* wp = P<int2>(ctx->unit_wp) + u0;
+                if (timing) CK(cudaEventRecord(ctx->kev[4 * c + 0], ctx->stream));
+                TRY(run_fft<true>(ctx, l, rows_of(l, l), nc, IoPass1Units{W, TS, R, wp, l2}));
+                if (timing) CK(cudaEventRecord(ctx->kev[4 * c + 1], ctx->stream));
+                if (timing) CK(cudaEventRecord(ctx->kev[4 * c + 2], ctx->stream));
+                IoPass2 io2;
+                io2.R = R; io2.acc = ua + 2 * (size_t)u0; io2.l = l; io2.ntmpl = 2 * nc;
+                io2.q_lo = q_lo; io2.q_hi = q_hi; io2.sgn = sgn;
+                TRY(run_fft<true>(ctx, l, cols_of(l, l), nc, io2));
+                if (timing) CK(cudaEventRecord(ctx->kev[4 * c + 3], ctx->stream));
+            }
+            k_finalize_units<<<blocks_for(2ll * n, 128), 128, 0, ctx->stream>>>(
+                ua, P<int2>(ctx->unit_wp), n, Np, N, (long long)NW * N, l, units + (size_t)a0 * NW * N);
+            ++ctx->counters.kernel_launches;
+            CKL();
             return GS_OK;
         }
         const int ai = a0;
@@ -1895,15 +1932,16 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
                 k1ms += a;
                 k1n += 1;
             } else if (timing) {
-                for (int w = 0; w < NW; ++w) {
+                const int n = chunked ? (int)(((long long)nu * std::min(A, na - ai) + chunk - 1) / chunk) : NW;
+                for (int w = 0; w < n; ++w) {
                     float a = 0, b = 0;
                     cudaEventElapsedTime(&a, ctx->kev[4 * w + 0], ctx->kev[4 * w + 1]);
                     cudaEventElapsedTime(&b, ctx->kev[4 * w + 2], ctx->kev[4 * w + 3]);
                     k1ms += a;
                     k2ms += b;
                 }
-                k1n += NW;
-                k2n += NW;
+                k1n += n;
+                k2n += n;
             }
         }
     }

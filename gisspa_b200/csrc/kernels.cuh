@@ -497,6 +497,23 @@ struct IoPass1 {
     __device__ void finish(double*, int, int) const {}
 };
 
+// The same over a chunk of (window, pair) units: image i is unit u0 + i of the
+// unit order, its pair's spectra counted over the launch's angles.
+struct IoPass1Units {
+    const float2* W;
+    const float2* P;
+    float2* R;
+    const int2* unit_wp;
+    long long l2;
+    __device__ float2 load(int img, int, int, long long a) const {
+        const int2 wp = __ldg(unit_wp + img);
+        const long long off = a - (long long)img * l2;
+        return cmulc(__ldg(W + (long long)wp.x * l2 + off), __ldg(P + (long long)wp.y * l2 + off));
+    }
+    __device__ void store(int, int, int, long long a, float2 v) const { R[a] = v; }
+    __device__ void finish(double*, int, int) const {}
+};
+
 // Per (window, template) accumulators of the column pass.
 struct UnitAcc {
     unsigned long long key;  // argmax_key of the border-masked max
@@ -577,12 +594,8 @@ struct UnitOut {
 
 // Score of each (window, template): peak = max(0, masked max), sigma of the
 // map without the peak (rc = l^2 - 1).  Reference: main.cu:869-876.
-static __global__ void k_finalize(const UnitAcc* __restrict__ acc, int ntmpl, int l, UnitOut* __restrict__ out) {
-    const int J = blockIdx.x * blockDim.x + threadIdx.x;
-    if (J >= ntmpl) return;
-    const UnitAcc a = acc[J];
+__device__ __forceinline__ UnitOut unit_result(const UnitAcc& a, int l) {
     const float peak = key_value(a.key);
-    const int pos = key_index(a.key);
     const double ra = a.s1 - peak;
     const double rb = a.s2 - (double)peak * peak;
     const double rc = (double)l * l - 1.0;
@@ -590,10 +603,33 @@ static __global__ void k_finalize(const UnitAcc* __restrict__ acc, int ntmpl, in
     const double sd = sqrt(var);  // NaN for var < 0, as sqrt in the reference
     UnitOut u;
     u.peak = peak;
-    u.pos = pos;
+    u.pos = key_index(a.key);
     u.sigma = (float)sd;
     u.score = sd > 0.0 ? (float)(peak / sd) : __int_as_float(0x7fc00000);
-    out[J] = u;
+    return u;
+}
+static __global__ void k_finalize(const UnitAcc* __restrict__ acc, int ntmpl, int l, UnitOut* __restrict__ out) {
+    const int J = blockIdx.x * blockDim.x + threadIdx.x;
+    if (J < ntmpl) out[J] = unit_result(acc[J], l);
+}
+
+// Results slot of template q (0, 1) of pair index y = angle x pairs + pair
+// for window w, or -1 when the pair has no second template (odd count).
+__device__ __forceinline__ long long unit_out_index(int y, int q, int w, int pairs, int ntmpl,
+                                                    long long out_stride) {
+    const int an = y / pairs, J = 2 * (y - an * pairs) + q;
+    return J < ntmpl ? an * out_stride + (long long)w * ntmpl + J : -1;
+}
+
+// k_finalize over the chunk of units unit_wp[0 .. nu): acc[2 u + q] of template
+// q of unit u's pair.
+static __global__ void k_finalize_units(const UnitAcc* __restrict__ acc, const int2* __restrict__ unit_wp, int nu,
+                                        int pairs, int ntmpl, long long out_stride, int l, UnitOut* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 2 * nu) return;
+    const int2 wp = unit_wp[i >> 1];
+    const long long o = unit_out_index(wp.y, i & 1, wp.x, pairs, ntmpl, out_stride);
+    if (o >= 0) out[o] = unit_result(acc[i], l);
 }
 
 struct PickDev {

@@ -260,7 +260,7 @@ static __device__ __noinline__ float2* plan_block_fft(float2* buf, float2* alt, 
 // Batched FFT through a plan: the grid, the IO functors and their calls are
 // those of fft_batched_kernel.
 template <bool kInv, class IO>
-__global__ void __launch_bounds__(256) fft_plan_kernel(const __grid_constant__ PlanDesc D, VecGeom g, int tile,
+__global__ void __launch_bounds__(256, 3) fft_plan_kernel(const __grid_constant__ PlanDesc D, VecGeom g, int tile,
                                                        IO io_param) {
     extern __shared__ float2 smem_plan[];
     IO io = io_param;

@@ -224,7 +224,8 @@ void gs_picks_free(gs_pick* picks);
  *  [6] column-pass kernel ms (sum)    [7] column-pass launches
  * With the persistent correlation kernel, [4]/[5] hold its time and launches
  * (one launch covers gs_get_tuning's [5] angles, the last launch the
- * remainder) and [6]/[7] are zero.  Entries 4-7 are filled only while per-kernel timing
+ * remainder) and [6]/[7] are zero; without it a row or column launch covers
+ * one window, or a chunk of units (GS_OPT_TWO_PASS).  Entries 4-7 are filled only while per-kernel timing
  * is enabled. */
 #define GS_TIMING_COUNT 8
 int gs_get_timings(struct gs_ctx* ctx, float* out, int n);
@@ -306,8 +307,9 @@ int gs_set_kernel_timing(struct gs_ctx* ctx, int enable);
 #define GS_OPT_GENERIC_FFT 1
 /* GS_OPT_TWO_PASS: 1 = run the correlation as separate row and column
  * launches per window, 0 = persistent launches where the specialised
- * kernels exist: windows l = 16 N2 with N2 from 6 to 48 whose prime factors
- * are at most 23 (default). */
+ * kernels exist (windows l = 16 N2 with N2 from 6 to 48 whose prime factors
+ * are at most 23), row and column launches over chunks of (window, pair)
+ * units at other windows (default). */
 #define GS_OPT_TWO_PASS 2
 /* GS_OPT_WINDOW_BLOCK: windows per block of the persistent launch's unit
  * order (reuse of window and pair spectra in L2); default 4 (8 for the FP32
