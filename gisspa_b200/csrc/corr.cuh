@@ -1,8 +1,10 @@
 // Persistent correlation kernel: the row pass and the column pass of every
 // (window, template pair) unit of one in-plane angle in a single launch.
 //
-// Work items, claimed in increasing order from one atomic counter:
-//   slot s (0 <= s < Nu + lag) = [T row tiles of unit s] [T column tiles of unit s - lag]
+// Work items, claimed in increasing order from one atomic counter (lag <= Nu):
+//   the row tiles of units 0 .. lag - 1, then for every later unit s
+//   [T row tiles of unit s] [T column tiles of unit s - lag], then the column
+//   tiles of the last lag units
 // with T = l / V tiles of V vectors (V = 16 or 8, CorrCfg).  A row tile takes V
 // spectrum rows of unit u: S = W_w conj(P_p), inverse FFT along x (the
 // four-step l = 16 N2 transform of fastfft.cuh), written to scratch map slot
@@ -55,6 +57,7 @@ struct CorrArgs {
     const float2* W;         // window spectra, Nw x L2
     const float2* P;         // template-pair spectra of the launch's angles, (angles x pairs) x L2
     float2* R;               // scratch ring, S x L2
+    const float2* tw;        // exp(-2 pi i k / l), k < l (even N2 only)
     const int2* unit_wp;     // unit -> (window, angle x pairs + pair)
     int* done_rows;          // per unit, row tiles finished
     int* done_cols;          // per unit, column tiles finished
@@ -73,6 +76,20 @@ struct CorrArgs {
     int nblk, nw;
     float inv_l2;
 };
+
+// Border interval of unshifted indices: X = (x + l/2) mod l is masked when X <
+// d_m/4 or X > l - d_m/4 (GPU_func.cu:681).
+inline void corr_border(CorrArgs* a, float d_m, int l) {
+    const float q_lo = d_m / 4.0f, q_hi = (float)l - q_lo;
+    const int h = l / 2;
+    a->yb0 = (int)floorf(q_hi) - h + 1;
+    a->yb1 = (int)ceilf(q_lo) + h - 1;
+    if (a->yb1 < a->yb0) { a->yb0 = 1; a->yb1 = 0; }
+}
+
+// Lag of the column tiles in units for `ctas` resident CTAs and units of `tiles`
+// tiles a pass: 2.5 times as many items as CTAs.
+inline int corr_lag(int ctas, int tiles) { return (5 * ctas + 4 * tiles - 1) / (4 * tiles); }
 
 // What the column tiles do with the maps: score them; add them into the
 // per-pixel moments; z-score them and keep every 1024-element block's maximum.
@@ -466,47 +483,41 @@ __device__ __forceinline__ UnitOut unit_score(const UnitAcc& ac, double s1, int 
 }
 __device__ __forceinline__ UnitOut unit_score(const UnitAcc& ac, int l) { return unit_score(ac, ac.s1, l); }
 
-// The counter whose completions `item` waits for (T of them), or nullptr.
-template <int N2, int V>
-__device__ __forceinline__ const int* corr_dep(const CorrArgs& a, int item) {
-    using C = CorrCfg<N2, V>;
-    const int s = item / (2 * C::T), j = item - s * (2 * C::T);
-    if (j < C::T) return (s < a.nu && s >= a.S) ? a.done_cols + (s - a.S) : nullptr;
-    const int u = s - a.lag;
-    return (u >= 0 && u < a.nu) ? a.done_rows + u : nullptr;
+// What a claimed item is.
+struct CorrItem {
+    int u, j;  // unit, tile
+    bool row;
+};
+
+template <int T>
+__device__ __forceinline__ CorrItem corr_item(const CorrArgs& a, int item) {
+    const int head = a.lag * T;
+    if (item < head) return CorrItem{item / T, item % T, true};
+    const int i = item - head, s = i / (2 * T), j = i - s * (2 * T);
+    if (s < a.nu - a.lag) return j < T ? CorrItem{a.lag + s, j, true} : CorrItem{s, j - T, false};
+    const int c = i - (a.nu - a.lag) * (2 * T);
+    return CorrItem{a.nu - a.lag + c / T, c % T, false};
 }
 
-// (window, pair) of the unit whose row tile `item` is ({0, 0} for column
-// tiles and the padding items past the last unit).  unit_wp is written by the
-// host before the launch, so this load needs no ordering.
-template <int N2, int V>
-__device__ __forceinline__ int2 corr_item_wp(const CorrArgs& a, int item, int total) {
-    using C = CorrCfg<N2, V>;
-    if (item >= total) return make_int2(0, 0);
-    const int s = item / (2 * C::T), j = item - s * (2 * C::T);
-    return (j < C::T && s < a.nu) ? __ldg(a.unit_wp + s) : make_int2(0, 0);
-}
-
-// Each warp checks the dependency of `item` before working on it.
-template <int N2, int V>
-__device__ __forceinline__ void corr_wait_for(const CorrArgs& a, int item) {
-    using C = CorrCfg<N2, V>;
-    const int* p = corr_dep<N2, V>(a, item);
-    if (p) wait_counter_warp(p, C::T, a.error);
+// Each warp waits for what an item depends on before working on it: a row
+// tile for its slot's previous unit's column tiles, a column tile for its
+// unit's row tiles.
+template <int T>
+__device__ __forceinline__ void corr_wait_for(const CorrArgs& a, const CorrItem& it) {
+    if (!it.row) wait_counter_warp(a.done_rows + it.u, T, a.error);
+    else if (it.u >= a.S) wait_counter_warp(a.done_cols + (it.u - a.S), T, a.error);
 }
 
 // Count a finished tile; the last count of a unit's column pass computes its
 // two scores.
 template <int N2, int V, CorrEpi kEpi>
-__device__ __forceinline__ void corr_publish(const CorrArgs& a, int item) {
+__device__ __forceinline__ void corr_publish(const CorrArgs& a, const CorrItem& it) {
     using F = CorrCfg<N2, V>;
-    const int s = item / (2 * F::T), j = item - s * (2 * F::T);
-    if (j < F::T) {
-        if (s < a.nu) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(&a.done_rows[s]) : "memory");
+    const int u = it.u;
+    if (it.row) {
+        asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(&a.done_rows[u]) : "memory");
         return;
     }
-    const int u = s - a.lag;
-    if (u < 0 || u >= a.nu) return;
     if constexpr (kEpi != kCorrScore) {
         asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(&a.done_cols[u]) : "memory");
         return;
@@ -546,12 +557,10 @@ __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCta
     // inverse twiddles W_L^{-n2 k1} = exp(+2 pi i n2 k1 / L), table [k1][n2]
     for (int i = threadIdx.x; i < (F::kPfa ? 0 : 16 * N2); i += F::kThreads) {
         const int k1 = i / N2, n2 = i - k1 * N2;
-        double sn, cs;
-        sincospi(2.0 * (double)((n2 * k1) % F::L) / (double)F::L, &sn, &cs);
-        twt[i] = make_float2((float)cs, (float)sn);
+        twt[i] = twiddle(a.tw, n2 * k1, true);
     }
     const uint2 ymask = corr_row_mask<N2, V>(a.yb0, a.yb1);
-    const int total = (a.nu + a.lag) * 2 * F::T;
+    const int total = a.nu * 2 * F::T;
     // the CTA always holds its current item and the next one
     if (threadIdx.x == kPub) {
         ish[0] = atomicAdd(a.next_item, 1);
@@ -563,15 +572,11 @@ __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCta
     for (int iter = 0; item < total; ++iter) {
         // the unit's (window, pair) is read-only in this launch: its load is
         // issued before the dependency wait and overlaps it
-        const int2 wp = corr_item_wp<N2, V>(a, item, total);
-        const int s = item / (2 * F::T), j = item - s * (2 * F::T);
-        corr_wait_for<N2, V>(a, item);
-        if (j < F::T) {
-            if (s < a.nu) corr_row_tile<N2, V>(a, s, j, tile, twt, wp);
-        } else {
-            const int u = s - a.lag;
-            if (u >= 0 && u < a.nu) corr_col_tile<N2, V, kEpi>(a, u, j - F::T, tile, twt, ymask);
-        }
+        const CorrItem it = corr_item<F::T>(a, item);
+        const int2 wp = it.row ? __ldg(a.unit_wp + it.u) : make_int2(0, 0);
+        corr_wait_for<F::T>(a, it);
+        if (it.row) corr_row_tile<N2, V>(a, it.u, it.j, tile, twt, wp);
+        else corr_col_tile<N2, V, kEpi>(a, it.u, it.j, tile, twt, ymask);
         // the claim made after the previous barrier enters the ring only now,
         // so the publisher's warp did not wait for the atomic's return
         if (threadIdx.x == kPub && iter > 0) ish[(iter + 1) & 3] = claimed;
@@ -582,7 +587,7 @@ __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCta
         __syncthreads();
         const int next = ish[(iter + 1) & 3];
         if (threadIdx.x == kPub) {
-            corr_publish<N2, V, kEpi>(a, item);
+            corr_publish<N2, V, kEpi>(a, it);
             claimed = atomicAdd(a.next_item, 1);  // for slot (iter + 2) & 3
         }
         item = next;

@@ -339,8 +339,9 @@ int run_win(gs_ctx* ctx, int l, int nimg, cudaError_t (*launch)(const float2*, i
 }
 
 // Persistent FP32 correlation with tiles of `tile` vectors (16 or 8; the
-// norm_type 1 epilogues: 16).
-int launch_corr(gs_ctx* ctx, int l, int tile, const CorrArgs& a, CorrEpi epi = kCorrScore) {
+// norm_type 1 epilogues: 16).  The ring needs no more lag than there are units.
+int launch_corr(gs_ctx* ctx, int l, int tile, CorrArgs a, CorrEpi epi = kCorrScore) {
+    a.lag = std::min(a.lag, a.nu);
     const WinOps* w = win_of(ctx, l);
     if (!w || (epi != kCorrScore && !w->corr_moments))
         return set_err(ctx, GS_ERR_UNSUPPORTED, "no persistent kernel for %d", l);
@@ -1278,7 +1279,7 @@ static int default_tuning(gs_ctx* ctx, bool tc2, CorrTuning* out) {
             int nsm = 0;
             CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
             const int ctas = nsm * win_of(ctx, l)->threads_per_sm / (16 * tune.tile), tiles = l / tune.tile;
-            tune.lag = (5 * ctas + 4 * tiles - 1) / (4 * tiles);
+            tune.lag = corr_lag(ctas, tiles);
             tune.slots = (11 * tune.lag + 4) / 5;
         }
     }
@@ -1333,16 +1334,10 @@ static int corr_launch(gs_ctx* ctx, const float2* W, const float2* TS, int nu, c
     ca.nu = nu; ca.ntmpl = ctx->ntmpl; ca.S = t.slots; ca.lag = t.lag; ca.L2 = l2;
     ca.pairs = (ctx->ntmpl + 1) / 2;
     ca.out_stride = out_stride;
-    // border interval of unshifted indices: X = (x + l/2) mod l is masked
-    // when X < d_m/4 or X > l - d_m/4 (GPU_func.cu:681)
-    {
-        const float q_lo = ctx->p.d_m / 4.0f, q_hi = (float)l - q_lo;
-        const int h = l / 2;
-        const int ya = (int)ceilf(q_lo), yb = (int)floorf(q_hi);
-        ca.yb0 = yb - h + 1;
-        ca.yb1 = ya + h - 1;
-        if (ca.yb1 < ca.yb0) { ca.yb0 = 1; ca.yb1 = 0; }
-    }
+    corr_border(&ca, ctx->p.d_m, l);
+    FftPlan* plan = nullptr;
+    TRY(get_plan(ctx, l, &plan));  // there since before any capture
+    ca.tw = plan->tw;
     ctx->corr_ctas_override = t.ctas;
     if (norm1) {
         ca.moments = norm1->moments;

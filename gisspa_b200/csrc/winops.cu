@@ -35,7 +35,7 @@ cudaError_t corr_launch_v(const CorrArgs& a, int ctas, cudaStream_t st, bool* fi
     *fits = per_sm >= 1;
     if (!*fits) return cudaSuccess;
     if (ctas > 0 && ctas < per_sm) per_sm = ctas;
-    const long long items = (long long)(a.nu + a.lag) * 2 * C::T;
+    const long long items = (long long)a.nu * 2 * C::T;
     const long long grid = (long long)nsm * per_sm < items ? (long long)nsm * per_sm : items;
     kern<<<(unsigned)grid, C::kThreads, smem, st>>>(a);
     return cudaGetLastError();
