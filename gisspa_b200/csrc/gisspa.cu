@@ -124,6 +124,10 @@ struct gs_ctx {
     DBuf tc2_wmax, tc2_pmax;  // per window / per pair max |spectrum| (all-tensor-core path)
     DBuf tc2_w16, tc2_p16;    // their FP16 copies, scaled by powers of two
     DBuf rot_cs;              // (cos, sin) of every in-plane angle of the search
+    // template preparation, kept for the next set: raw templates, shell RMS,
+    // double sums (edge, shells, amplitudes), weight map (the spectra use tspec
+    // and scratch)
+    DBuf tp_raw, tp_div, tp_sums, tp_wmap;
     // off-grid refinement (refine.cuh): per-pick chunk buffers
     DBuf rf_pk, rf_acc, rf_B, rf_F1, rf_T, rf_TM, rf_F, rf_G, rf_TB, rf_mask;
     std::vector<cudaEvent_t> kev;  // pool of events for per-kernel timing
@@ -970,7 +974,7 @@ int gs_ctx_destroy(gs_ctx* ctx) {
                     &ctx->dep_counters, &ctx->pacc, &ctx->flags, &ctx->tbase, &ctx->rf_pk, &ctx->rf_acc,
                     &ctx->rf_B, &ctx->rf_F1, &ctx->rf_T, &ctx->rf_TM, &ctx->rf_F, &ctx->rf_G, &ctx->rf_TB,
                     &ctx->rf_mask, &ctx->pix_keys, &ctx->pix_pairs, &ctx->pix_R, &ctx->tc2_wmax,
-                    &ctx->tc2_pmax, &ctx->tc2_w16, &ctx->tc2_p16, &ctx->rot_cs};
+                    &ctx->tc2_pmax, &ctx->tc2_w16, &ctx->tc2_p16, &ctx->rot_cs, &ctx->tp_raw, &ctx->tp_div, &ctx->tp_sums, &ctx->tp_wmap};
     for (DBuf* b : bufs) free_buf(*b);
     for (cudaEvent_t e : ctx->kev) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->side_ev) cudaEventDestroy(e);
@@ -1025,17 +1029,27 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
     const size_t l2 = (size_t)l * l;
     TRY(ensure(ctx, ctx->tmpl, sizeof(float) * l2 * n));
     TRY(ensure(ctx, ctx->tbase, sizeof(float) * l2 * n));
-    const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)n, (size_t)(1u << 30) / (l2 * 8)));
-    DBuf raw, F, div, sumsq, inv, wmap, Fb;
+    // templates per pass: spectra of 256 MiB keep every kernel busy for tens of
+    // microseconds
+    const int chunk = (int)std::max<size_t>(1, std::min<size_t>(std::min(n, 65535), (size_t)(256u << 20) / (l2 * 8)));
+    DBuf &raw = ctx->tp_raw, &F = ctx->tspec, &Fb = ctx->scratch, &div = ctx->tp_div, &wmap = ctx->tp_wmap;
+    const int ns = l / 2;
     int st = GS_OK;
     do {
+        // doubles: edge sums [4], amplitude sums [2] and their inverses [1] per
+        // template, shell sums [ns] per template, shell counts
+        const size_t sums_bytes = sizeof(double) * (size_t)chunk * (7 + ns) + sizeof(unsigned) * ns;
         if ((st = ensure(ctx, raw, sizeof(float) * (size_t)tx * ty * chunk))) break;
         if ((st = ensure(ctx, F, sizeof(float2) * l2 * chunk))) break;
-        if ((st = ensure(ctx, div, sizeof(float) * (size_t)(l / 2) * chunk))) break;
-        if ((st = ensure(ctx, sumsq, sizeof(double) * 2 * chunk))) break;
-        if ((st = ensure(ctx, inv, sizeof(double) * chunk))) break;
+        if ((st = ensure(ctx, div, sizeof(float) * (size_t)ns * chunk))) break;
+        if ((st = ensure(ctx, ctx->tp_sums, sums_bytes))) break;
         if ((st = ensure(ctx, wmap, sizeof(float) * l2))) break;
         if ((st = ensure(ctx, Fb, sizeof(float2) * l2 * chunk))) break;
+        double* edge = P<double>(ctx->tp_sums);
+        double* sumsq = edge + 4 * (size_t)chunk;
+        double* inv = sumsq + 2 * (size_t)chunk;
+        double* shells = inv + chunk;
+        unsigned* shell_count = reinterpret_cast<unsigned*>(shells + (size_t)chunk * ns);
         // weight map with the FIRST micrograph's CTF; ds from the configured
         // window size (main.cu:155 runs before main.cu:1116 adjusts it)
         float ds = 0.0f;
@@ -1054,9 +1068,13 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
             cudaError_t e = cudaMemcpyAsync(P<float>(raw), host_templates + (size_t)c0i * tx * ty,
                                             sizeof(float) * (size_t)tx * ty * nc, cudaMemcpyHostToDevice, ctx->stream);
             if (e != cudaSuccess) { st = set_err(ctx, GS_ERR_CUDA, "template upload: %s", cudaGetErrorString(e)); break; }
-            k_tmpl_pad_edge<<<nc, 256, 0, ctx->stream>>>(P<float>(raw), tx, ty, l, P<float2>(F));
-            ++ctx->counters.kernel_launches;
-            if (cudaGetLastError() != cudaSuccess) { st = set_err(ctx, GS_ERR_CUDA, "k_tmpl_pad_edge"); break; }
+            if (cudaMemsetAsync(ctx->tp_sums.p, 0, sums_bytes, ctx->stream) != cudaSuccess) { st = set_err(ctx, GS_ERR_CUDA, "template sums"); break; }
+            const TmplPad pad = tmpl_pad(tx, ty, l);
+            const dim3 gp(blocks_for((long long)l2, 1024, 64), nc);
+            k_tmpl_edge_sums<<<gp, 256, 0, ctx->stream>>>(P<float>(raw), pad, edge);
+            k_tmpl_pad<<<gp, 256, 0, ctx->stream>>>(P<float>(raw), pad, edge, P<float2>(F));
+            ctx->counters.kernel_launches += 2;
+            if (cudaGetLastError() != cudaSuccess) { st = set_err(ctx, GS_ERR_CUDA, "template padding"); break; }
             const WinOps* w = win_of(ctx, l);
             if (w) {
                 if ((st = run_win(ctx, l, nc, w->rows, F16Complex<false>{P<float2>(F), l, (long long)l2, 1.0f}))) break;
@@ -1065,33 +1083,36 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
                 if ((st = run_fft<false>(ctx, l, rows_of(l, l), nc, IoComplex{P<float2>(F), 1.0f}))) break;
                 if ((st = run_fft<false>(ctx, l, cols_of(l, l), nc, IoComplex{P<float2>(F), 1.0f / (float)l2}))) break;
             }
-            const size_t shs = (size_t)(l / 2) * (sizeof(double) + sizeof(unsigned));
+            const size_t shs = (size_t)ns * (sizeof(double) + sizeof(unsigned));
             if (shs > kMaxSmem) { st = set_err(ctx, GS_ERR_UNSUPPORTED, "window too large"); break; }
             cudaFuncSetAttribute(k_tmpl_shells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shs);
-            k_tmpl_shells<<<nc, 256, shs, ctx->stream>>>(P<float2>(F), l, P<float>(div));
-            ++ctx->counters.kernel_launches;
-            {
-                // whitened base (before the weight), kept for the refinement
-                dim3 gb(blocks_for((long long)l2, 256, 64), nc);
-                k_tmpl_whiten<<<gb, 256, 0, ctx->stream>>>(P<float2>(F), l, P<float>(div), P<float2>(Fb));
-                ++ctx->counters.kernel_launches;
-                if ((st = run_fft<true>(ctx, l, rows_of(l, l), nc, IoComplex{P<float2>(Fb), 1.0f}))) break;
-                if ((st = run_fft<true>(ctx, l, cols_of(l, l), nc,
-                                        IoRealOut{P<float2>(Fb), P<float>(ctx->tbase) + (size_t)c0i * l2, 1.0f}))) break;
-            }
-            cudaMemsetAsync(P<double>(sumsq), 0, sizeof(double) * 2 * nc, ctx->stream);
+            k_tmpl_shells<<<dim3(blocks_for((long long)l2 / 2, 2048, 32), nc), 256, shs, ctx->stream>>>(
+                P<float2>(F), l, shells, shell_count);
+            k_tmpl_shell_rms<<<blocks_for((long long)nc * ns, 256), 256, 0, ctx->stream>>>(shells, shell_count, ns, nc,
+                                                                                         P<float>(div), inv);
+            ctx->counters.kernel_launches += 2;
+            // weighted spectra, and the whitened base (before the weight), kept for
+            // the refinement
             dim3 g(blocks_for((long long)l2, 256, 64), nc);
-            k_tmpl_apply<<<g, 256, 0, ctx->stream>>>(P<float2>(F), l, P<float>(div), P<float>(wmap), P<double>(sumsq));
+            k_tmpl_apply<<<g, 256, 0, ctx->stream>>>(P<float2>(F), l, P<float>(div), P<float>(wmap), sumsq, P<float2>(Fb));
             ++ctx->counters.kernel_launches;
-            k_inv_amp_norm<<<blocks_for(nc, 128), 128, 0, ctx->stream>>>(P<double>(sumsq), nc, P<double>(inv));
+            float* base = P<float>(ctx->tbase) + (size_t)c0i * l2;
+            if (w) {
+                if ((st = run_win(ctx, l, nc, w->inv_rows, F16ScaleIn<false>{P<float2>(Fb), inv, l, (long long)l2}))) break;
+                if ((st = run_win(ctx, l, nc, w->inv_cols, F16RealOut<true>{P<float2>(Fb), base, l, (long long)l2}))) break;
+            } else {
+                if ((st = run_fft<true>(ctx, l, rows_of(l, l), nc, IoComplex{P<float2>(Fb), 1.0f}))) break;
+                if ((st = run_fft<true>(ctx, l, cols_of(l, l), nc, IoRealOut{P<float2>(Fb), base, 1.0f}))) break;
+            }
+            k_inv_amp_norm<<<blocks_for(nc, 128), 128, 0, ctx->stream>>>(sumsq, nc, inv);
             ++ctx->counters.kernel_launches;
             if (cudaGetLastError() != cudaSuccess) { st = set_err(ctx, GS_ERR_CUDA, "template weighting"); break; }
             if (w) {
-                if ((st = run_win(ctx, l, nc, w->inv_rows, F16ScaleIn<false>{P<float2>(F), P<double>(inv), l, (long long)l2}))) break;
+                if ((st = run_win(ctx, l, nc, w->inv_rows, F16ScaleIn<false>{P<float2>(F), inv, l, (long long)l2}))) break;
                 if ((st = run_win(ctx, l, nc, w->inv_cols, F16RealOut<true>{P<float2>(F), P<float>(ctx->tmpl) + (size_t)c0i * l2,
                                                                             l, (long long)l2}))) break;
             } else {
-                if ((st = run_fft<true>(ctx, l, rows_of(l, l), nc, IoScaleIn{P<float2>(F), P<double>(inv)}))) break;
+                if ((st = run_fft<true>(ctx, l, rows_of(l, l), nc, IoScaleIn{P<float2>(F), inv}))) break;
                 if ((st = run_fft<true>(ctx, l, cols_of(l, l), nc,
                                         IoRealOut{P<float2>(F), P<float>(ctx->tmpl) + (size_t)c0i * l2, 1.0f}))) break;
             }
@@ -1101,7 +1122,6 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
         if (e != cudaSuccess) st = set_err(ctx, GS_ERR_CUDA, "template preprocessing: %s", cudaGetErrorString(e));
     } while (0);
     cudaStreamSynchronize(ctx->stream);
-    free_buf(raw); free_buf(F); free_buf(div); free_buf(sumsq); free_buf(inv); free_buf(wmap); free_buf(Fb);
     if (st == GS_OK) ctx->have_tmpl = true;
     return st;
 }

@@ -20,29 +20,34 @@ namespace gs {
 // it: (t - ring mean) / std(full l x l frame), the ring being the 1-px annulus
 // (r-1)^2 <= d^2 <= (r+1)^2, r = l/2 - 2, around (l/2, l/2).
 // Reference: readAndPaddingTemplate + edgeNormalize (main.cu:182-223,
-// 311-385; kernels GPU_func.cu:3-94).  One CTA per template.
-static __global__ void __launch_bounds__(256) k_tmpl_pad_edge(const float* __restrict__ raw, int tx, int ty, int l,
-                                                        float2* __restrict__ out) {
-    __shared__ double red[4 * 32];
-    const int J = blockIdx.x;
-    const float* src = raw + (size_t)J * tx * ty;
-    float2* dst = out + (size_t)J * l * l;
-    const int sx = (l - tx) / 2, sy = (l - ty) / 2;
+// 311-385; kernels GPU_func.cu:3-94).  Two launches of many CTAs per template
+// (sums, then the padded frame): one CTA per template took 1.09 ms for 100
+// templates at window 720.
+struct TmplPad {
+    int tx, ty, l, sx, sy;
+    float low, up;  // the ring's squared radii
+};
+inline TmplPad tmpl_pad(int tx, int ty, int l) {
     const float r = (float)l / 2.0f - 2.0f;
-    float up = 0.0f, low = 0.0f;
-    if (r > 1.0f) {
-        up = (r + 1.0f) * (r + 1.0f);
-        low = (r - 1.0f) * (r - 1.0f);
-    }
-    const int h = l / 2;
-    const int npix = l * l;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};  // ring sum, ring count, sum, sum of squares
-    for (int i = threadIdx.x; i < npix; i += blockDim.x) {
-        const int x = i % l, y = i / l;
-        float v = 0.0f;
-        if (x >= sx && x < sx + tx && y >= sy && y < sy + ty) v = src[(y - sy) * tx + (x - sx)];
+    return TmplPad{tx, ty, l, (l - tx) / 2, (l - ty) / 2, r > 1.0f ? (r - 1.0f) * (r - 1.0f) : 0.0f,
+                   r > 1.0f ? (r + 1.0f) * (r + 1.0f) : 0.0f};
+}
+__device__ __forceinline__ float tmpl_padded(const float* src, const TmplPad& d, int x, int y) {
+    return x >= d.sx && x < d.sx + d.tx && y >= d.sy && y < d.sy + d.ty ? src[(y - d.sy) * d.tx + (x - d.sx)] : 0.0f;
+}
+
+// sums[4 J ..]: ring sum, ring count, sum, sum of squares of padded template J.
+static __global__ void __launch_bounds__(256) k_tmpl_edge_sums(const float* __restrict__ raw, TmplPad d,
+                                                               double* __restrict__ sums) {
+    __shared__ double red[4 * 32];
+    const int J = blockIdx.y, h = d.l / 2, npix = d.l * d.l;
+    const float* src = raw + (size_t)J * d.tx * d.ty;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
+        const int y = i / d.l, x = i - y * d.l;
+        const float v = tmpl_padded(src, d, x, y);
         const float rr = (float)((x - h) * (x - h) + (y - h) * (y - h));
-        if (rr >= low && rr <= up) {
+        if (rr >= d.low && rr <= d.up) {
             acc[0] += v;
             acc[1] += 1.0;
         }
@@ -50,49 +55,66 @@ static __global__ void __launch_bounds__(256) k_tmpl_pad_edge(const float* __res
         acc[3] += (double)v * v;
     }
     block_sum<4>(acc, red);
-    const double em = acc[1] > 0 ? acc[0] / acc[1] : 0.0;
-    const double mean = acc[2] / npix;
-    double sigma = sqrt(acc[3] / npix - mean * mean);
+    if (threadIdx.x < 4) atomicAdd(&sums[4 * J + threadIdx.x], acc[threadIdx.x]);
+}
+
+static __global__ void __launch_bounds__(256) k_tmpl_pad(const float* __restrict__ raw, TmplPad d,
+                                                         const double* __restrict__ sums, float2* __restrict__ out) {
+    const int J = blockIdx.y, npix = d.l * d.l;
+    const float* src = raw + (size_t)J * d.tx * d.ty;
+    const double* a = sums + 4 * J;
+    const double em = a[1] > 0 ? a[0] / a[1] : 0.0;
+    const double mean = a[2] / npix;
+    double sigma = sqrt(a[3] / npix - mean * mean);
     if (!(sigma >= 0.0) || !isfinite(sigma)) sigma = 0.0;
     const bool scale = fabs(sigma) >= 1e-8;  // EPS of GPU_func.cuh:28
-    for (int i = threadIdx.x; i < npix; i += blockDim.x) {
-        const int x = i % l, y = i / l;
-        float v = 0.0f;
-        if (x >= sx && x < sx + tx && y >= sy && y < sy + ty) v = src[(y - sy) * tx + (x - sx)];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
+        const int y = i / d.l, x = i - y * d.l;
+        float v = tmpl_padded(src, d, x, y);
         if (scale) v = (float)(((double)v - em) / sigma);
-        dst[i] = make_float2(v, 0.0f);
+        out[(size_t)J * npix + i] = make_float2(v, 0.0f);
     }
 }
 
-// Radial-shell RMS of one template spectrum over the half plane x <= l/2:
-// div[r] = sqrt(sum |F|^2 / count) for shells 0 <= r < l/2.
-// Reference: SQRSum_by_circle, mode 0 (GPU_func.cu:98-128).  One CTA per
-// template; shared memory holds the shell histogram (l/2 doubles + counts).
-static __global__ void __launch_bounds__(256) k_tmpl_shells(const float2* __restrict__ F, int l, float* __restrict__ div) {
+// Radial-shell sums of one template spectrum over the half plane x <= l/2:
+// sum[J ns + r] += |F|^2 and, for template 0, count[r], shells 0 <= r < ns = l/2.
+// Reference: SQRSum_by_circle, mode 0 (GPU_func.cu:98-128).  Each CTA keeps its
+// rows' histogram in shared memory (l/2 doubles + counts).
+static __global__ void __launch_bounds__(256) k_tmpl_shells(const float2* __restrict__ F, int l,
+                                                            double* __restrict__ sum, unsigned* __restrict__ count) {
     extern __shared__ double sh[];
     const int ns = l / 2;
-    double* ra = sh;
     unsigned* rb = reinterpret_cast<unsigned*>(sh + ns);
     for (int r = threadIdx.x; r < ns; r += blockDim.x) {
-        ra[r] = 0.0;
+        sh[r] = 0.0;
         rb[r] = 0u;
     }
     __syncthreads();
-    const int J = blockIdx.x;
+    const int J = blockIdx.y;
     const float2* src = F + (size_t)J * l * l;
     const int hw = l / 2 + 1;  // x <= l/2
-    for (int i = threadIdx.x; i < hw * l; i += blockDim.x) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < hw * l; i += gridDim.x * blockDim.x) {
         const int y = i / hw, x = i % hw;
         const int r = shell_index(x, y, l, l);
         if (r >= 0 && r < ns) {
             const float2 v = src[y * l + x];
-            atomicAdd(&ra[r], (double)v.x * v.x + (double)v.y * v.y);
-            atomicAdd(&rb[r], 1u);
+            atomicAdd(&sh[r], (double)v.x * v.x + (double)v.y * v.y);
+            if (J == 0) atomicAdd(&rb[r], 1u);
         }
     }
     __syncthreads();
-    for (int r = threadIdx.x; r < ns; r += blockDim.x)
-        div[(size_t)J * ns + r] = (float)sqrt(ra[r] / (double)rb[r]);
+    for (int r = threadIdx.x; r < ns; r += blockDim.x) {
+        if (sh[r] != 0.0) atomicAdd(&sum[(size_t)J * ns + r], sh[r]);
+        if (J == 0 && rb[r]) atomicAdd(&count[r], rb[r]);
+    }
+}
+
+// div[J ns + r]: the shell's RMS; one[J] = 1 (the base's scale).
+static __global__ void k_tmpl_shell_rms(const double* __restrict__ sum, const unsigned* __restrict__ count, int ns,
+                                        int n, float* __restrict__ div, double* __restrict__ one) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n * ns) div[i] = (float)sqrt(sum[i] / (double)count[i % ns]);
+    if (i < n) one[i] = 1.0;
 }
 
 struct WeightConsts {
@@ -121,31 +143,15 @@ static __global__ void k_weight_map(float* __restrict__ wmap, int l, WeightConst
     wmap[i] = f;
 }
 
-// The whitened template spectrum alone (F / shell RMS, no weight), written
-// to B: the base that the off-grid refinement re-weights with other CTF
-// parameters.  Same whitening as k_tmpl_apply (whiten_Tmp, GPU_func.cu:130-152).
-static __global__ void __launch_bounds__(256) k_tmpl_whiten(const float2* __restrict__ F, int l, const float* __restrict__ div,
-                                                     float2* __restrict__ B) {
-    const int J = blockIdx.y;
-    const int ns = l / 2;
-    const float2* d = F + (size_t)J * l * l;
-    const float* dv = div + (size_t)J * ns;
-    const int npix = l * l;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
-        const int x = i % l, y = i / l;
-        const int r = shell_index(x, y, l, l);
-        float2 v = d[i];
-        if (r >= 0 && r < ns) v = cscale(v, 1.0f / dv[r]);
-        B[(size_t)J * l * l + i] = v;
-    }
-}
-
 // Whiten by the shell RMS, apply the weight map, and accumulate per template
-// sum |F|^2 and the count over r < l/2, x <= l/2.
+// sum |F|^2 and the count over r < l/2, x <= l/2.  The whitened spectrum without
+// the weight goes to B: the base that the off-grid refinement re-weights with
+// other CTF parameters.
 // Reference: whiten_Tmp + apply_weighting_function + compute_area_sum_ofSQR
 // (GPU_func.cu:130-152, 249-290, 318-362).  Grid (pixel chunks, templates).
 static __global__ void __launch_bounds__(256) k_tmpl_apply(float2* __restrict__ F, int l, const float* __restrict__ div,
-                                                    const float* __restrict__ wmap, double* __restrict__ sumsq) {
+                                                    const float* __restrict__ wmap, double* __restrict__ sumsq,
+                                                    float2* __restrict__ B) {
     __shared__ double red[2 * 32];
     const int J = blockIdx.y;
     const int ns = l / 2;
@@ -158,6 +164,7 @@ static __global__ void __launch_bounds__(256) k_tmpl_apply(float2* __restrict__ 
         const int r = shell_index(x, y, l, l);
         float2 v = d[i];
         if (r >= 0 && r < ns) v = cscale(v, 1.0f / dv[r]);
+        B[(size_t)J * npix + i] = v;
         v = cscale(v, wmap[i]);
         d[i] = v;
         if (r >= 0 && r < ns && x <= l / 2) {
