@@ -1169,18 +1169,25 @@ static int prep_micrograph(gs_ctx* ctx, const MicPlan& mp, float2* W) {
     TRY(ensure(ctx, ctx->q, sizeof(float) * 2 * npix4));
     TRY(ensure(ctx, ctx->cimg, sizeof(float2) * npix));
     TRY(ensure(ctx, ctx->img, sizeof(float) * npix));
-    TRY(ensure(ctx, ctx->stats, sizeof(float) * 2));
+    // running sums: block sums (double), block runs, the two sums
+    static_assert(kQuotBlock == kSeqBlock, "one block of terms");
+    const int nblk = (int)((npix + kSeqBlock - 1) / kSeqBlock);
+    const size_t b_exact = sizeof(double) * 2 * nblk, b_runs = (sizeof(SeqBlock) * 2 * nblk + 7) / 8 * 8;
+    TRY(ensure(ctx, ctx->stats, b_exact + b_runs + sizeof(float) * 2));
+    double* exact = P<double>(ctx->stats);
+    SeqBlock* seq_runs = reinterpret_cast<SeqBlock*>(exact + 2 * nblk);
+    float* seq_sums = reinterpret_cast<float*>(reinterpret_cast<char*>(seq_runs) + b_runs);
     const int ns = std::max(nx, ny) / 2;
     TRY(ensure(ctx, ctx->ra, sizeof(double) * ns));
     TRY(ensure(ctx, ctx->rb, sizeof(unsigned) * ns));
     float* q1 = P<float>(ctx->q);
     float* q2 = q1 + npix4;
-    k_mic_quot<<<blocks_for(npix, 256), 256, 0, ctx->stream>>>(d_mic, npix, nx, ny, q1, q2);
-    ++ctx->counters.kernel_launches;
-    CK(cudaFuncSetAttribute(k_seq_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmem));
-    k_seq_sums<<<2, kSeqThreads, kSeqSmem, ctx->stream>>>(q1, npix4, npix, P<float>(ctx->stats));
-    ++ctx->counters.kernel_launches;
-    k_mic_clamp<<<blocks_for(npix, 256), 256, 0, ctx->stream>>>(d_mic, npix, P<float>(ctx->stats), p.invert,
+    k_mic_quot<<<nblk, 256, 0, ctx->stream>>>(d_mic, npix, nx, ny, q1, q2, exact);
+    k_seq_runs<<<dim3(nblk, 2), kSeqThreads, 0, ctx->stream>>>(q1, npix4, npix, exact, seq_runs);
+    CK(cudaFuncSetAttribute(k_seq_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmem));
+    k_seq_apply<<<2, kSeqThreads, kSeqSmem, ctx->stream>>>(q1, npix4, npix, seq_runs, nblk, seq_sums);
+    ctx->counters.kernel_launches += 3;
+    k_mic_clamp<<<blocks_for(npix, 256), 256, 0, ctx->stream>>>(d_mic, npix, seq_sums, p.invert,
                                                                  P<float2>(ctx->cimg));
     ++ctx->counters.kernel_launches;
     CKL();

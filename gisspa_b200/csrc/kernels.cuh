@@ -200,14 +200,27 @@ struct MicStats {
 };
 
 // Per-pixel quotients of the reference's host statistics loop
-// (main.cu:530-535): cur/nx/ny and cur*cur/nx/ny, IEEE float32 each.
-static __global__ void k_mic_quot(const float* __restrict__ img, long long n, int nx, int ny, float* __restrict__ q1,
-                           float* __restrict__ q2) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float v = img[i];
-    q1[i] = __fdiv_rn(__fdiv_rn(v, (float)nx), (float)ny);
-    q2[i] = __fdiv_rn(__fdiv_rn(__fmul_rn(v, v), (float)nx), (float)ny);
+// (main.cu:530-535): cur/nx/ny and cur*cur/nx/ny, IEEE float32 each, and their
+// sums in double over the CTA's kQuotBlock pixels at sums[blockIdx.x] and
+// sums[gridDim.x + blockIdx.x].
+constexpr int kQuotBlock = 16384;
+static __global__ void __launch_bounds__(256) k_mic_quot(const float* __restrict__ img, long long n, int nx, int ny,
+                                                         float* __restrict__ q1, float* __restrict__ q2,
+                                                         double* __restrict__ sums) {
+    __shared__ double red[2 * 32];
+    const long long end = min(n, (long long)(blockIdx.x + 1) * kQuotBlock);
+    double s[2] = {0.0, 0.0};
+    for (long long i = (long long)blockIdx.x * kQuotBlock + threadIdx.x; i < end; i += blockDim.x) {
+        const float v = img[i];
+        const float a = __fdiv_rn(__fdiv_rn(v, (float)nx), (float)ny);
+        const float b = __fdiv_rn(__fdiv_rn(__fmul_rn(v, v), (float)nx), (float)ny);
+        q1[i] = a;
+        q2[i] = b;
+        s[0] += a;
+        s[1] += b;
+    }
+    block_sum<2>(s, red);
+    if (threadIdx.x < 2) sums[threadIdx.x * gridDim.x + blockIdx.x] = s[threadIdx.x];
 }
 
 // Clamp bounds from the two running sums (seqsum.cuh): main.cu:536-543.

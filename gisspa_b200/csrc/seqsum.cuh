@@ -4,7 +4,8 @@
 // taken pixel by pixel (main.cu:530-535); float addition is not associative,
 // so the order is part of the result.  One dependent addition per pixel costs
 // 4 cycles of latency: 73.4 ms for 5760 x 4092 pixels when a single thread does
-// it, with the rest of the GPU waiting; this way it is 6.7 ms.
+// it, with the rest of the GPU waiting; this way it is 1.7 ms (0.5 where the mean
+// is not 0).
 //
 // While the running sum s stays inside one binade [2^e, 2^(e+1)) it is k u with
 // u = 2^(e-23) and an integer k, and rounding to nearest even makes adding q
@@ -66,44 +67,56 @@ __host__ __device__ __forceinline__ float seq_scale(unsigned binade) {
     return seq_float(((binade >> 8) << 31) | ((277u - e) << 23));
 }
 
-// The run of N terms.  Terms of 2^22 units and more (and NaN) make it fail.
+// The run of N terms (N even).  The change of k is summed in floats, exact
+// integers below 2^24; on the way k moves by no more than the terms' absolute
+// sum and their rounding.  Runs whose absolute sum reaches 2^22 units (or is
+// NaN) fail.
 template <int N>
 __host__ __device__ __forceinline__ SeqRun seq_run(const float (&q)[N], float scale) {
     constexpr float kMagic = 12582912.0f;  // 1.5 x 2^23: adding it rounds to an integer
-    int acc = 0, o = 0, mn = 0, mx = 0;
-    float big = 0.0f;
+    float2 acc = make_float2(0.0f, 0.0f);  // of the even and the odd terms
+    float size = 0.0f;
+    int o = 0;
 #ifdef __CUDA_ARCH__
 #pragma unroll
 #endif
-    for (int i = 0; i < N; ++i) {
-        const float x = q[i] * scale;
+    for (int i = 0; i < N; i += 2) {
 #ifdef __CUDA_ARCH__
-        asm("max.NaN.f32 %0, %0, %1;" : "+f"(big) : "f"(fabsf(x)));
-        const float y = __fadd_rn(x, kMagic);
-        const float r = __fsub_rn(y, kMagic);
-        const float f = __fsub_rn(x, r);
+        const float2 x = cscale(make_float2(q[i], q[i + 1]), scale);
+        const float2 y = cadd(x, make_float2(kMagic, kMagic));
+        float2 r = cadd(y, make_float2(-kMagic, -kMagic));
+        const float2 f = csub(x, r);
 #else
-        if (!(fabsf(x) <= big) && big == big) big = fabsf(x);  // keeps a NaN
-        volatile float yv = x + kMagic;
-        const float y = yv;
-        volatile float rv = y - kMagic;
-        const float r = rv, f = x - r;
+        const float2 x = make_float2(q[i] * scale, q[i + 1] * scale);
+        volatile float y0 = x.x + kMagic, y1 = x.y + kMagic;
+        float2 r = make_float2(y0 - kMagic, y1 - kMagic);
+        const float2 f = make_float2(x.x - r.x, x.y - r.y);
 #endif
-        int step = (int)(seq_bits(y) - 0x4b400000u);
-        if (fabsf(f) == 0.5f) {
-            // halfway: `step` is the even neighbour, the other one makes an odd k even
-            const int other = step + (f > 0.0f ? 1 : -1);
-            const int se = (acc & 1) ? other : step;
-            const int so = ((acc + o) & 1) ? step : other;  // k odd at the start
-            o += so - se;
-            step = se;
+        size += fabsf(x.x) + fabsf(x.y);
+        if (fabsf(f.x) == 0.5f || fabsf(f.y) == 0.5f) {
+            // halfway: r is the even neighbour, the other one makes an odd k even
+            int k = (int)(acc.x + acc.y);
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+            for (int t = 0; t < 2; ++t) {
+                const float g = t ? f.y : f.x, v = t ? r.y : r.x;
+                const int even = (int)v, other = even + (g > 0.0f ? 1 : -1);
+                int step = even;
+                if (fabsf(g) == 0.5f) {
+                    step = (k & 1) ? other : even;
+                    o += (((k + o) & 1) ? even : other) - step;  // k odd at the start
+                }
+                k += step;
+                if (t) r.y = (float)step;
+                else r.x = (float)step;
+            }
         }
-        acc += step;
-        mn = acc < mn ? acc : mn;
-        mx = acc > mx ? acc : mx;
+        acc = cadd(acc, r);
     }
-    if (!(big < 4194304.0f) || mn < -kSeqRange || mx > kSeqRange) return SeqRun{0, 0, 0, kSeqFail};
-    return SeqRun{acc, o, mn, mx};
+    if (!(size < 4194304.0f)) return SeqRun{0, 0, 0, kSeqFail};
+    const int far = (int)(size * 1.0001f) + N;
+    return SeqRun{(int)(acc.x + acc.y), o, -far, far};
 }
 
 // Run a, then run b.
@@ -133,34 +146,31 @@ __host__ __device__ __forceinline__ bool seq_apply(float& s, unsigned binade, co
     return true;
 }
 
-// sums[b] = ((0 + q_b[0]) + q_b[1]) + ... for the two arrays q_0 = q and
-// q_1 = q + stride (16-byte aligned), one CTA each.
-//
-// Bound by the FP32 and integer issue rate of the one SM each sum runs on
-// (about 11 instructions a term).  A block of 16384 terms (16 a thread) is
-// staged by cp.async while the one before it is summed; each warp's 512-term
-// run, composed by shuffles, is a unit that is either applied or added term
-// by term by one thread.  Chunks of 20 floats keep both the 16-byte copies
-// aligned and a thread's 16-byte reads free of bank conflicts.
+// Three launches over blocks of kSeqBlock terms:
+//   the terms' kernel (k_mic_quot) also leaves the blocks' sums in double;
+//   k_seq_runs, one CTA per block, predicts the binade at the block's start from
+//   those sums and composes the block's run for it (threads 16 terms, then
+//   warps, then the CTA), all blocks at once;
+//   k_seq_apply, one CTA per sum, applies the blocks' runs in order, about 40
+//   cycles each.  A block whose binade was predicted wrongly (float sums drift
+//   from the exact ones) or that comes too close to its edges is staged in
+//   shared memory and done 512 terms at a time by one warp: by a run where that
+//   applies, term by term (4 cycles each) where it does not.
+// The last kernel is what is left: its time goes with the number of blocks in
+// which the sum passes a power of two, 12 of 1438 for a mean that is not 0 and
+// 136 for 5760 x 4092 pixels of coloured noise around 0.
 constexpr int kSeqThreads = 1024;
-constexpr int kSeqTerms = 16;                         // per thread
-constexpr int kSeqPitch = kSeqTerms + 4;
+constexpr int kSeqTerms = 16;  // per thread
 constexpr int kSeqBlock = kSeqThreads * kSeqTerms;
-constexpr size_t kSeqSmem = 2 * (size_t)kSeqThreads * kSeqPitch * sizeof(float);
+// chunks of 20 floats: 16-byte copies stay aligned and a lane's 16-byte reads
+// free of bank conflicts
+constexpr int kSeqPitch = kSeqTerms + 4;
+constexpr size_t kSeqSmem = (size_t)kSeqThreads * kSeqPitch * sizeof(float);
 
-__device__ __forceinline__ void seq_stage(float* buf, const float* __restrict__ q, long long base, long long n) {
-#pragma unroll
-    for (int j = 0; j < kSeqTerms / 4; ++j) {
-        const int i4 = j * kSeqThreads + threadIdx.x;  // 16-byte piece
-        const long long g = base + 4ll * i4;
-        const long long left = n - g;
-        const int bytes = left >= 4 ? 16 : left > 0 ? (int)left * 4 : 0;  // the rest is zero filled: s + 0 = s
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + (i4 >> 2) * kSeqPitch + (i4 & 3) * 4);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(q + (bytes ? g : 0)), "r"(bytes)
-                     : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
+struct SeqBlock {
+    SeqRun run;
+    unsigned binade;  // it was composed for; 0: none
+};
 
 __device__ __forceinline__ SeqRun seq_shfl_down(const SeqRun& r, int off) {
     SeqRun v;
@@ -171,71 +181,166 @@ __device__ __forceinline__ SeqRun seq_shfl_down(const SeqRun& r, int off) {
     return v;
 }
 
-// Lane 0 gets the composition of all 32 lanes' runs in lane order.
+// The composition of all 32 lanes' runs in lane order, in lane 0 at least.
+// Without ties and failed runs a prefix sum and two reductions do.
 __device__ __forceinline__ SeqRun seq_warp(SeqRun r) {
+    if (!__any_sync(0xffffffffu, r.o != 0 || r.mx >= kSeqFail)) {
+        const int lane = threadIdx.x & 31;
+        int sum = r.d;
+#pragma unroll
+        for (int off = 1; off < 32; off *= 2) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, off);
+            if (lane >= off) sum += v;
+        }
+        const int before = sum - r.d;
+        const int mn = __reduce_min_sync(0xffffffffu, before + r.mn), mx = __reduce_max_sync(0xffffffffu, before + r.mx);
+        const int d = __shfl_sync(0xffffffffu, sum, 31);
+        return mn < -kSeqRange || mx > kSeqRange ? SeqRun{0, 0, 0, kSeqFail} : SeqRun{d, 0, mn, mx};
+    }
 #pragma unroll
     for (int off = 1; off < 32; off *= 2) r = seq_then(r, seq_shfl_down(r, off));
     return r;
 }
 
-__global__ void __launch_bounds__(kSeqThreads) k_seq_sums(const float* __restrict__ q, long long stride, long long n,
-                                                          float* __restrict__ sums) {
+// Blocks of the array q + blockIdx.y stride (16-byte aligned), their exact sums at
+// exact + blockIdx.y gridDim.x; results at out + blockIdx.y gridDim.x.
+__global__ void __launch_bounds__(kSeqThreads) k_seq_runs(const float* __restrict__ q, long long stride, long long n,
+                                                          const double* __restrict__ exact, SeqBlock* __restrict__ out) {
+    __shared__ SeqRun runs[32];
+    __shared__ double red[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b = blockIdx.x;
+    q += blockIdx.y * stride;
+    exact += (size_t)blockIdx.y * gridDim.x;
+    float t[kSeqTerms];
+    const long long base = (long long)b * kSeqBlock + threadIdx.x * kSeqTerms;
+#pragma unroll
+    for (int j = 0; j < kSeqTerms; j += 4) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // behind the end: s + 0 = s
+        if (base + j + 3 < n) {
+            v = *reinterpret_cast<const float4*>(q + base + j);
+        } else {
+            if (base + j < n) v.x = q[base + j];
+            if (base + j + 1 < n) v.y = q[base + j + 1];
+            if (base + j + 2 < n) v.z = q[base + j + 2];
+        }
+        t[j] = v.x; t[j + 1] = v.y; t[j + 2] = v.z; t[j + 3] = v.w;
+    }
+    double before[1] = {0.0};
+    for (int i = threadIdx.x; i < b; i += kSeqThreads) before[0] += exact[i];
+    block_sum<1>(before, red);
+    const unsigned binade = seq_binade((float)before[0]);
+    SeqRun r = seq_identity();
+    if (binade) r = seq_warp(seq_run(t, seq_scale(binade)));
+    if (lane == 0) runs[warp] = r;
+    __syncthreads();
+    if (warp == 0) {
+        r = seq_warp(runs[lane]);
+        if (lane == 0) out[(size_t)blockIdx.y * gridDim.x + b] = SeqBlock{r, binade};
+    }
+}
+
+// One block of terms into buf, zeros behind the end.
+__device__ __forceinline__ void seq_stage(float* buf, const float* __restrict__ q, long long base, long long n) {
+#pragma unroll
+    for (int j = 0; j < kSeqTerms / 4; ++j) {
+        const int i4 = j * kSeqThreads + threadIdx.x;  // 16-byte piece
+        const long long g = base + 4ll * i4;
+        const long long left = n - g;
+        const int bytes = left >= 4 ? 16 : left > 0 ? (int)left * 4 : 0;
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + (i4 >> 2) * kSeqPitch + (i4 & 3) * 4);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(q + (bytes ? g : 0)), "r"(bytes)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// sums[b] = ((0 + q_b[0]) + q_b[1]) + ... for q_b = q + b stride, b = blockIdx.x.
+__global__ void __launch_bounds__(kSeqThreads) k_seq_apply(const float* __restrict__ q, long long stride, long long n,
+                                                           const SeqBlock* __restrict__ blocks, int nblocks,
+                                                           float* __restrict__ sums) {
     extern __shared__ __align__(16) float seq_buf[];
     __shared__ SeqRun runs[32];
     __shared__ float sh_s;
-    __shared__ int sh_w;
+    __shared__ int sh_b;
     q += blockIdx.x * stride;
+    blocks += (size_t)blockIdx.x * nblocks;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) sh_s = 0.0f;
-    seq_stage(seq_buf, q, 0, n);
-    int cur = 0;
-    for (long long base = 0; base < n; base += kSeqBlock, cur ^= 1) {
-        const float* buf = seq_buf + cur * kSeqThreads * kSeqPitch;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();  // the block is staged, and the other buffer free
-        if (base + kSeqBlock < n) seq_stage(seq_buf + (cur ^ 1) * kSeqThreads * kSeqPitch, q, base + kSeqBlock, n);
-        float t[kSeqTerms];
-#pragma unroll
-        for (int j = 0; j < kSeqTerms / 4; ++j) {
-            const float4 v = *reinterpret_cast<const float4*>(buf + threadIdx.x * kSeqPitch + 4 * j);
-            t[4 * j] = v.x; t[4 * j + 1] = v.y; t[4 * j + 2] = v.z; t[4 * j + 3] = v.w;
-        }
-        int w0 = 0;  // warps before it are in the sum
-        do {
-            const unsigned binade = seq_binade(sh_s);
-            SeqRun r = seq_identity();
-            if (warp >= w0 && binade) r = seq_warp(seq_run(t, seq_scale(binade)));
-            if (lane == 0) runs[warp] = r;
-            __syncthreads();
-            if (warp == 0) {
-                const SeqRun all = seq_warp(runs[lane]);
-                if (lane == 0) {
-                    float s = sh_s;
-                    int w = 32;
-                    if (!seq_apply(s, binade, all)) {
-                        for (w = w0; w < 32; ++w) {
-                            if (seq_apply(s, binade, runs[w])) continue;
-                            const float4* v = reinterpret_cast<const float4*>(buf + w * 32 * kSeqPitch);
-#pragma unroll 4
-                            for (int c = 0; c < 32; ++c)
-#pragma unroll
-                                for (int j = 0; j < kSeqTerms / 4; ++j) {
-                                    const float4 a = v[c * (kSeqPitch / 4) + j];
-                                    s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a.x), a.y), a.z), a.w);
-                                }
-                            if (seq_binade(s) != binade) {  // the later warps' runs need another unit
-                                ++w;
-                                break;
-                            }
-                        }
-                    }
-                    sh_s = s;
-                    sh_w = w;
+    int b = 0;
+    for (;;) {
+        if (warp == 0) {
+            __syncwarp();
+            float s = sh_s;
+            bool ok = true;
+            while (ok && b < nblocks) {
+                const SeqBlock mine = b + lane < nblocks ? blocks[b + lane] : SeqBlock{seq_identity(), 0u};
+                const int m = min(32, nblocks - b);
+                int i = 0;
+                for (; i < m; ++i) {
+                    SeqRun r;
+                    r.d = __shfl_sync(0xffffffffu, mine.run.d, i);
+                    r.o = __shfl_sync(0xffffffffu, mine.run.o, i);
+                    r.mn = __shfl_sync(0xffffffffu, mine.run.mn, i);
+                    r.mx = __shfl_sync(0xffffffffu, mine.run.mx, i);
+                    ok = seq_apply(s, __shfl_sync(0xffffffffu, mine.binade, i), r);
+                    if (!ok) break;
                 }
+                b += i;
             }
-            __syncthreads();
-            w0 = sh_w;
-        } while (w0 < 32);
+            if (lane == 0) {
+                sh_s = s;
+                sh_b = b;
+            }
+        }
+        __syncthreads();
+        b = sh_b;
+        if (b >= nblocks) break;
+        // block b by its parts
+        seq_stage(seq_buf, q, (long long)b * kSeqBlock, n);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const unsigned binade = seq_binade(sh_s);
+        auto part = [&](int w, unsigned bin) {  // the run of warp w's 512 terms, by the calling warp
+            float t[kSeqTerms];
+#pragma unroll
+            for (int j = 0; j < kSeqTerms; j += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(seq_buf + (w * 32 + lane) * kSeqPitch + j);
+                t[j] = v.x; t[j + 1] = v.y; t[j + 2] = v.z; t[j + 3] = v.w;
+            }
+            return seq_warp(seq_run(t, seq_scale(bin)));
+        };
+        SeqRun r = seq_identity();
+        if (binade) r = part(warp, binade);
+        if (lane == 0) runs[warp] = r;
+        __syncthreads();
+        if (warp == 0) {
+            float s = sh_s;
+            for (int w = 0; w < 32; ++w) {
+                const unsigned now = seq_binade(s);
+                // (only lane 0 of a warp holds its composition)
+                bool ok = false;
+                if (now && now == binade) {
+                    ok = seq_apply(s, now, runs[w]);
+                } else if (now) {
+                    const SeqRun p = part(w, now);
+                    if (lane == 0) ok = seq_apply(s, now, p);
+                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                    s = __shfl_sync(0xffffffffu, s, 0);
+                }
+                if (ok) continue;
+                const float4* v = reinterpret_cast<const float4*>(seq_buf + w * 32 * kSeqPitch);
+#pragma unroll 4
+                for (int c = 0; c < 32; ++c)
+#pragma unroll
+                    for (int j = 0; j < kSeqTerms / 4; ++j) {
+                        const float4 a = v[c * (kSeqPitch / 4) + j];
+                        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a.x), a.y), a.z), a.w);
+                    }
+            }
+            if (lane == 0) sh_s = s;
+        }
+        ++b;
+        __syncthreads();
     }
     if (threadIdx.x == 0) sums[blockIdx.x] = sh_s;
 }

@@ -98,18 +98,37 @@ int main(int argc, char** argv) {
         other.resize(n, 0.0f);
         memcpy(two.data(), cs[c].data(), 4 * n);
         memcpy(two.data() + n4, other.data(), 4 * n);
-        float *d = nullptr, *ds = nullptr, got[2] = {0, 0};
-        if (cudaMalloc(&d, 8 * n4) || cudaMalloc(&ds, 8)) return 2;
-        cudaMemcpy(d, two.data(), 8 * n4, cudaMemcpyHostToDevice);
-        cudaFuncSetAttribute(k_seq_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmem);
-        k_seq_sums<<<2, kSeqThreads, kSeqSmem>>>(d, (long long)n4, (long long)n, ds);
-        if (cudaMemcpy(got, ds, 8, cudaMemcpyDeviceToHost) != cudaSuccess) { printf("%s\n", cudaGetErrorString(cudaGetLastError())); return 2; }
-        cudaFree(d);
-        cudaFree(ds);
-        const float want2 = plain(other);
-        if (!same(got[0], want) || !same(got[1], want2)) {
-            printf("case %zu (n %zu): %.9g %.9g, plain %.9g %.9g\n", c, n, got[0], got[1], want, want2);
-            bad = 1;
+        const int nblk = (int)((n + kSeqBlock - 1) / kSeqBlock);
+        std::vector<double> exact(2 * nblk, 0.0);
+        for (size_t i = 0; i < n; ++i) {
+            exact[i / kSeqBlock] += two[i];
+            exact[nblk + i / kSeqBlock] += two[n4 + i];
+        }
+        // the second time with predictions that are no good: only the route may change
+        for (int bad_guess = 0; bad_guess < 2; ++bad_guess) {
+            if (bad_guess)
+                for (double& e : exact) e *= 0.37;
+            float *d = nullptr, *ds = nullptr, got[2] = {0, 0};
+            double* de = nullptr;
+            SeqBlock* db = nullptr;
+            if (cudaMalloc(&d, 8 * n4) || cudaMalloc(&ds, 8) || cudaMalloc(&de, 16 * nblk) ||
+                cudaMalloc(&db, 2 * nblk * sizeof(SeqBlock)))
+                return 2;
+            cudaMemcpy(d, two.data(), 8 * n4, cudaMemcpyHostToDevice);
+            cudaMemcpy(de, exact.data(), 16 * nblk, cudaMemcpyHostToDevice);
+            cudaFuncSetAttribute(k_seq_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmem);
+            k_seq_runs<<<dim3(nblk, 2), kSeqThreads>>>(d, (long long)n4, (long long)n, de, db);
+            k_seq_apply<<<2, kSeqThreads, kSeqSmem>>>(d, (long long)n4, (long long)n, db, nblk, ds);
+            if (cudaMemcpy(got, ds, 8, cudaMemcpyDeviceToHost) != cudaSuccess) { printf("%s\n", cudaGetErrorString(cudaGetLastError())); return 2; }
+            cudaFree(d);
+            cudaFree(ds);
+            cudaFree(de);
+            cudaFree(db);
+            const float want2 = plain(other);
+            if (!same(got[0], want) || !same(got[1], want2)) {
+                printf("case %zu (n %zu): %.9g %.9g, plain %.9g %.9g\n", c, n, got[0], got[1], want, want2);
+                bad = 1;
+            }
         }
     }
     if (!gpu && applied < 1000) { printf("only %lld runs applied\n", applied); bad = 1; }
