@@ -217,19 +217,22 @@ struct F16RealOut {
     __device__ void finish(double*) const {}
 };
 
-// Rows of the template-pair images: z = t1n - i t2n with per-template
-// (mean, 1/sd) normalisation on load (see IoPairNorm), in place.
+// Rows of the template-pair images: z = (t1 - i t2) with the per-template 1/sd
+// on load (see IoPairNorm), in place, from image row row0 on (a multiple of 16).
 struct F16PairNorm {
     float2* data;
     const float4* coef;
     int L;
     long long L2;
+    int row0;
     __device__ float2 load(int img, int v, int k) const {
         const float4 c = coef[img];
-        const float2 z = data[f16_addr<false>(L, L2, img, v, k)];
-        return make_float2((z.x - c.x) * c.y, -(z.y - c.z) * c.w);
+        const float2 z = data[f16_addr<false>(L, L2, img, v + row0, k)];
+        return make_float2(z.x * c.y, -z.y * c.w);
     }
-    __device__ void store(int img, int v, int k, float2 x) const { data[f16_addr<false>(L, L2, img, v, k)] = x; }
+    __device__ void store(int img, int v, int k, float2 x) const {
+        data[f16_addr<false>(L, L2, img, v + row0, k)] = x;
+    }
     __device__ void finish(double*) const {}
 };
 
@@ -239,7 +242,27 @@ struct F16PairNormPfa : F16PairNorm {
     PfaCols pfa;
     static constexpr bool kStaged = true;
     __device__ int column(int k) const { return pfa.physical(k); }
-    __device__ void store_at(int img, int v, int p, float2 x) const { data[f16_addr<false>(L, L2, img, v, p)] = x; }
+    __device__ void store_at(int img, int v, int p, float2 x) const {
+        data[f16_addr<false>(L, L2, img, v + row0, p)] = x;
+    }
+};
+
+// Columns of the template-pair images: rows outside [row0, row1) are zero and
+// not read; the zero frequency, which holds nothing but the means, is set to
+// zero (see IoPairNorm).
+struct F16PairCols {
+    float2* data;
+    int L;
+    long long L2;
+    float scale;
+    int row0, row1;
+    __device__ float2 load(int img, int v, int k) const {
+        return k >= row0 && k < row1 ? data[f16_addr<true>(L, L2, img, v, k)] : make_float2(0.0f, 0.0f);
+    }
+    __device__ void store(int img, int v, int k, float2 x) const {
+        data[f16_addr<true>(L, L2, img, v, k)] = v + k == 0 ? make_float2(0.0f, 0.0f) : cscale(x, scale);
+    }
+    __device__ void finish(double*) const {}
 };
 
 // Row pass of the correlation: S = W_w conj(P_p), inverse FFT along x,

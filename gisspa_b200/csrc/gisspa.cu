@@ -503,8 +503,12 @@ static int pair_spectra_n(gs_ctx* ctx, float e, const float2* cs, int nang, floa
     const float2 c = rotation_cs(e);
     const int nimg = Np * nang;
     CK(cudaMemsetAsync(ctx->pstats.p, 0, sizeof(double) * 2 * N * nang, ctx->stream));
-    dim3 g(blocks_for(l2, 256, 32), Np, nang);
-    k_pair_rotate<<<g, 256, 0, ctx->stream>>>(P<float>(ctx->tmpl), N, l, c.x, c.y, cs, ctx->p.d_m, TS,
+    // rows that the mask's disc (radius 0.75 d_m + 12) reaches, in whole tiles of 16
+    const float rout = 0.75f * ctx->p.d_m + 12.0f;
+    const int row0 = std::max(0, (int)std::floor((float)(l / 2) - std::min(rout, (float)l)) - 1) / 16 * 16;
+    const int row1 = std::min(l, ((int)std::ceil((float)(l / 2) + std::min(rout, (float)l)) + 2 + 15) / 16 * 16);
+    dim3 g(blocks_for((long long)(row1 - row0) * l, 256, 32), Np, nang);
+    k_pair_rotate<<<g, 256, 0, ctx->stream>>>(P<float>(ctx->tmpl), N, l, c.x, c.y, cs, ctx->p.d_m, row0, row1, TS,
                                               P<double>(ctx->pstats));
     ++ctx->counters.kernel_launches;
     k_pair_coef<<<blocks_for(nimg, 128), 128, 0, ctx->stream>>>(P<double>(ctx->pstats), N, l,
@@ -512,15 +516,19 @@ static int pair_spectra_n(gs_ctx* ctx, float e, const float2* cs, int nang, floa
     ++ctx->counters.kernel_launches;
     CKL();
     if (const WinOps* w = win_of(ctx, l)) {
-        const F16PairNorm rows{TS, P<float4>(ctx->coef), l, l2};
-        if (pfa)
-            TRY(run_win(ctx, l, nimg, w->pair_rows_pfa, F16PairNormPfa{rows, PfaCols::make(l)}));
-        else
-            TRY(run_win(ctx, l, nimg, w->pair_rows, rows));
-        TRY(run_win(ctx, l, nimg, w->cols, F16Complex<true>{TS, l, l2, (float)(1.0 / (double)l2)}));
+        const F16PairNorm rows{TS, P<float4>(ctx->coef), l, l2, row0};
+        FftPlan* pl = nullptr;
+        TRY(get_plan(ctx, l, &pl));
+        if (nimg > 65535) return set_err(ctx, GS_ERR_UNSUPPORTED, "too many images in one FFT batch (%d)", nimg);
+        const int tiles = (row1 - row0) / 16;
+        TRY(win_status(ctx, pfa ? w->pair_rows_pfa(pl->tw, nimg, tiles, F16PairNormPfa{rows, PfaCols::make(l)}, ctx->stream)
+                                : w->pair_rows(pl->tw, nimg, tiles, rows, ctx->stream), "pair rows"));
+        TRY(run_win(ctx, l, nimg, w->pair_cols, F16PairCols{TS, l, l2, (float)(1.0 / (double)l2), row0, row1}));
     } else {
-        TRY(run_fft<false>(ctx, l, rows_of(l, l), nimg, IoPairNorm{TS, P<float4>(ctx->coef), l2}));
-        TRY(run_fft<false>(ctx, l, cols_of(l, l), nimg, IoComplex{TS, (float)(1.0 / (double)l2)}));
+        VecGeom rows = rows_of(l, l);
+        rows.nvec = row1 - row0;
+        TRY(run_fft<false>(ctx, l, rows, nimg, IoPairNorm{TS + (long long)row0 * l, P<float4>(ctx->coef)}));
+        TRY(run_fft<false>(ctx, l, cols_of(l, l), nimg, IoPairCols{TS, (float)(1.0 / (double)l2), row0, row1}));
     }
     return GS_OK;
 }

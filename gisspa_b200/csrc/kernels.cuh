@@ -381,8 +381,9 @@ static __global__ void k_scale_images(float2* __restrict__ d, long long per_img,
 // ---------------------------------------------------------------------------
 
 // Bilinear in-plane rotation + soft circular mask of both templates of pair
-// p, written as (t_2p, t_2p+1) in one complex image, with FP64 sums and sums of
-// squares of each template over the full l x l frame.
+// p, written as (t_2p, t_2p+1) in one complex image (rows [row0, row1), which hold
+// the mask's disc; the others are zero and not written), with FP64 sums and
+// sums of squares of each template over the full l x l frame.
 // Reference: rotate_subIMG + apply_mask + compute_sum_sqr
 // (GPU_func.cu:496-560, 229-247, 363-407; main.cu:669-685).
 // Several angles in one launch: with `cs` set, blockIdx.z selects angle z of
@@ -390,7 +391,8 @@ static __global__ void k_scale_images(float2* __restrict__ d, long long per_img,
 // sums at stats + 2 z ntmpl; without it, (cose, sine) and one angle.
 static __global__ void __launch_bounds__(256) k_pair_rotate(const float* __restrict__ tmpl, int ntmpl, int l, float cose,
                                                      float sine, const float2* __restrict__ cs, float d_m,
-                                                     float2* __restrict__ out, double* __restrict__ stats) {
+                                                     int row0, int row1, float2* __restrict__ out,
+                                                     double* __restrict__ stats) {
     __shared__ double red[4 * 32];
     const int p = blockIdx.y;
     const int J1 = 2 * p, J2 = 2 * p + 1;
@@ -409,8 +411,8 @@ static __global__ void __launch_bounds__(256) k_pair_rotate(const float* __restr
     const float dm = 1.5f * d_m;
     const float rin = dm / 2.0f, rout = dm / 2.0f + 12.0f;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    const int npix = l * l;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < npix; q += gridDim.x * blockDim.x) {
+    const int end = row1 * l;
+    for (int q = row0 * l + blockIdx.x * blockDim.x + threadIdx.x; q < end; q += gridDim.x * blockDim.x) {
         const int i = q % l, j = q / l;
         // mask first: outside radius rout the product with the mask is 0
         // whatever the rotated value, so its gathers are skipped
@@ -479,19 +481,33 @@ static __global__ void k_pair_coef(const double* __restrict__ stats, int ntmpl, 
     coef[p] = make_float4(c[0], c[1], c[2], c[3]);
 }
 
-// Loader of the pair spectra: z = t1n - i t2n, where tkn is template k
-// normalised to zero mean / unit variance, so that one complex FFT gives
-// P = T1 - i T2 and W conj(P) = W conj(T1) + i W conj(T2).
+// Rows of the pair spectra: z = t1n - i t2n, where tkn is template k normalised
+// to zero mean / unit variance, so that one complex FFT gives P = T1 - i T2 and
+// W conj(P) = W conj(T1) + i W conj(T2).  The means only reach the zero
+// frequency: instead of subtracting them (which would fill the frame outside
+// the mask) that frequency is set to zero in the column pass, and both passes
+// leave the rows outside the mask's disc alone.
 struct IoPairNorm {
-    float2* data;
+    float2* data;  // from the first row of the pass on
     const float4* coef;
-    long long img_elems;
     __device__ float2 load(int img, int, int, long long a) const {
         const float4 c = coef[img];
         const float2 z = data[a];
-        return make_float2((z.x - c.x) * c.y, -(z.y - c.z) * c.w);
+        return make_float2(z.x * c.y, -z.y * c.w);
     }
     __device__ void store(int, int, int, long long a, float2 v) const { data[a] = v; }
+    __device__ void finish(double*, int, int) const {}
+};
+struct IoPairCols {
+    float2* data;
+    float scale;
+    int row0, row1;
+    __device__ float2 load(int, int, int k, long long a) const {
+        return k >= row0 && k < row1 ? data[a] : make_float2(0.0f, 0.0f);
+    }
+    __device__ void store(int, int v, int k, long long a, float2 x) const {
+        data[a] = v + k == 0 ? make_float2(0.0f, 0.0f) : cscale(x, scale);
+    }
     __device__ void finish(double*, int, int) const {}
 };
 

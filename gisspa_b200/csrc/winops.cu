@@ -12,13 +12,18 @@ namespace gs {
 namespace {
 
 template <int N2, bool kInv, bool kCols, class IO>
-cudaError_t fft_launch(const float2* tw, int nimg, const IO& io, cudaStream_t st) {
+cudaError_t fft_launch_tiles(const float2* tw, int nimg, int tiles, const IO& io, cudaStream_t st) {
     using F = Fast16<N2>;
     auto kern = k_fft16<N2, kInv, kCols, IO>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::smem_bytes());
     if (e != cudaSuccess) return e;
-    kern<<<dim3(N2, (unsigned)nimg), F::kThreads, F::smem_bytes(), st>>>(tw, io);
+    kern<<<dim3((unsigned)tiles, (unsigned)nimg), F::kThreads, F::smem_bytes(), st>>>(tw, io);
     return cudaGetLastError();
+}
+
+template <int N2, bool kInv, bool kCols, class IO>
+cudaError_t fft_launch(const float2* tw, int nimg, const IO& io, cudaStream_t st) {
+    return fft_launch_tiles<N2, kInv, kCols>(tw, nimg, N2, io, st);
 }
 
 template <int N2, int V, CorrEpi kEpi = kCorrScore>
@@ -59,8 +64,9 @@ struct Ops {
                     o.corr_moments = corr_launch_v<N2, 16, kCorrMoments>;
                     o.corr_blocks = corr_launch_v<N2, 16, kCorrBlocks>;
                 }
-                if constexpr (N2 % 2 == 1) o.pair_rows_pfa = fft_launch<N2, false, false, F16PairNormPfa>;
-                o.pair_rows = fft_launch<N2, false, false, F16PairNorm>;
+                if constexpr (N2 % 2 == 1) o.pair_rows_pfa = fft_launch_tiles<N2, false, false, F16PairNormPfa>;
+                o.pair_rows = fft_launch_tiles<N2, false, false, F16PairNorm>;
+                o.pair_cols = fft_launch<N2, false, true, F16PairCols>;
                 o.rows = fft_launch<N2, false, false, F16Complex<false>>;
                 o.cols = fft_launch<N2, false, true, F16Complex<true>>;
                 o.inv_rows = fft_launch<N2, true, false, F16ScaleIn<false>>;

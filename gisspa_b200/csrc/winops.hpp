@@ -17,10 +17,12 @@ struct WinOps {
     // N2 (norm_type 1 takes windows that are multiples of 32)
     cudaError_t (*corr_moments)(const CorrArgs& a, int ctas, cudaStream_t st, bool* fits);
     cudaError_t (*corr_blocks)(const CorrArgs& a, int ctas, cudaStream_t st, bool* fits);
-    // forward transforms along rows: template pairs (natural or PfaCols column
-    // order) and complex images in place
-    cudaError_t (*pair_rows)(const float2* tw, int nimg, const F16PairNorm& io, cudaStream_t st);
-    cudaError_t (*pair_rows_pfa)(const float2* tw, int nimg, const F16PairNormPfa& io, cudaStream_t st);
+    // forward transforms of template pairs: `tiles` tiles of 16 rows (natural or
+    // PfaCols column order), and columns
+    cudaError_t (*pair_rows)(const float2* tw, int nimg, int tiles, const F16PairNorm& io, cudaStream_t st);
+    cudaError_t (*pair_rows_pfa)(const float2* tw, int nimg, int tiles, const F16PairNormPfa& io, cudaStream_t st);
+    cudaError_t (*pair_cols)(const float2* tw, int nimg, const F16PairCols& io, cudaStream_t st);
+    // forward transforms along rows of complex images, in place
     cudaError_t (*rows)(const float2* tw, int nimg, const F16Complex<false>& io, cudaStream_t st);
     // forward transform along columns, in place
     cudaError_t (*cols)(const float2* tw, int nimg, const F16Complex<true>& io, cudaStream_t st);
