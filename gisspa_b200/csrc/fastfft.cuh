@@ -248,19 +248,20 @@ struct F16PairNormPfa : F16PairNorm {
 };
 
 // Columns of the template-pair images: rows outside [row0, row1) are zero and
-// not read; the zero frequency, which holds nothing but the means, is set to
-// zero (see IoPairNorm).
+// not read; the zero frequency, which holds nothing but the means, is
+// multiplied by dc (0; see IoPairNorm).
 struct F16PairCols {
     float2* data;
     int L;
     long long L2;
     float scale;
     int row0, row1;
+    float dc = 0.0f;  // factor of the zero frequency
     __device__ float2 load(int img, int v, int k) const {
         return k >= row0 && k < row1 ? data[f16_addr<true>(L, L2, img, v, k)] : make_float2(0.0f, 0.0f);
     }
     __device__ void store(int img, int v, int k, float2 x) const {
-        data[f16_addr<true>(L, L2, img, v, k)] = v + k == 0 ? make_float2(0.0f, 0.0f) : cscale(x, scale);
+        data[f16_addr<true>(L, L2, img, v, k)] = cscale(x, v + k == 0 ? scale * dc : scale);
     }
     __device__ void finish(double*) const {}
 };

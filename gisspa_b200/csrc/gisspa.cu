@@ -90,7 +90,7 @@ struct gs_ctx {
     gs_ctf ctf0{};
     int l = 0, ntmpl = 0, tx = 0, ty = 0;
     DBuf tmpl;  // ntmpl x l x l float (real templates after preprocessing)
-    DBuf tbase; // ntmpl x l x l float (whitened templates before the CTF weight)
+    DBuf tbase; // ntmpl x l x (l/2 + 1) float2 (spectra of the whitened templates before the CTF weight)
     // per-search buffers
     DBuf in[2];                     // micrograph pixels, alternating within a batch
     cudaStream_t copy = nullptr;    // uploads of large micrographs
@@ -132,11 +132,10 @@ struct gs_ctx {
     DBuf tc2_w16, tc2_p16;    // their FP16 copies, scaled by powers of two
     DBuf rot_cs;              // (cos, sin) of every in-plane angle of the search
     // template preparation, kept for the next set: raw templates, shell RMS,
-    // double sums (edge, shells, amplitudes), weight map (the spectra use tspec
-    // and scratch)
+    // double sums (edge, shells, amplitudes), weight map (the spectra use tspec)
     DBuf tp_raw, tp_div, tp_sums, tp_wmap;
     // off-grid refinement (refine.cuh): per-pick chunk buffers
-    DBuf rf_pk, rf_acc, rf_B, rf_F1, rf_T, rf_TM, rf_F, rf_G, rf_TB, rf_mask;
+    DBuf rf_pk, rf_acc, rf_scale, rf_ph, rf_bins, rf_F1, rf_T, rf_TM, rf_F, rf_G, rf_TB, rf_mask;
     std::vector<cudaEvent_t> kev;  // pool of events for per-kernel timing
     gs_stats counters{0, 0, 0};
 };
@@ -484,6 +483,40 @@ unsigned blocks_for(long long n, int threads, unsigned cap = 1u << 30) {
 // ===========================================================================
 // C ABI
 // ===========================================================================
+// Image rows that the mask's disc (radius 0.75 d_m + 12, and one pixel of
+// interpolation) reaches, in whole tiles of 16.
+struct MaskRows {
+    int row0, row1;
+};
+static MaskRows mask_rows(float d_m, int l) {
+    const float r = std::min(0.75f * d_m + 12.0f, (float)l);
+    return MaskRows{std::max(0, (int)std::floor((float)(l / 2) - r) - 2) / 16 * 16,
+                    std::min(l, ((int)std::ceil((float)(l / 2) + r) + 3 + 15) / 16 * 16)};
+}
+
+// Forward transform, times `factor` (the zero frequency times `dc` besides), of
+// nimg images that are zero outside the rows mr, which alone are read; coef as
+// IoPairNorm takes it; pfa: the PfaCols column order.
+static int disc_transform(gs_ctx* ctx, float2* data, const float4* coef, int nimg, MaskRows mr, float factor, float dc,
+                          bool pfa) {
+    const int l = ctx->l;
+    const long long l2 = (long long)l * l;
+    if (const WinOps* w = win_of(ctx, l)) {
+        const F16PairNorm rows{data, coef, l, l2, mr.row0};
+        FftPlan* pl = nullptr;
+        TRY(get_plan(ctx, l, &pl));
+        if (nimg > 65535) return set_err(ctx, GS_ERR_UNSUPPORTED, "too many images in one FFT batch (%d)", nimg);
+        const int tiles = (mr.row1 - mr.row0) / 16;
+        TRY(win_status(ctx, pfa ? w->pair_rows_pfa(pl->tw, nimg, tiles, F16PairNormPfa{rows, PfaCols::make(l)}, ctx->stream)
+                                : w->pair_rows(pl->tw, nimg, tiles, rows, ctx->stream), "pair rows"));
+        return run_win(ctx, l, nimg, w->pair_cols, F16PairCols{data, l, l2, factor, mr.row0, mr.row1, dc});
+    }
+    VecGeom rows = rows_of(l, l);
+    rows.nvec = mr.row1 - mr.row0;
+    TRY(run_fft<false>(ctx, l, rows, nimg, IoPairNorm{data + (long long)mr.row0 * l, coef}));
+    return run_fft<false>(ctx, l, cols_of(l, l), nimg, IoPairCols{data, factor, mr.row0, mr.row1, dc});
+}
+
 // Template-pair spectra of one in-plane angle (rotate_template + the
 // normalisation and FFT of main.cu:1236-1249): TS[p] = FFT(t_2p - i t_2p+1) / l^2
 // with each rotated, masked template mean/variance normalised.
@@ -503,34 +536,16 @@ static int pair_spectra_n(gs_ctx* ctx, float e, const float2* cs, int nang, floa
     const float2 c = rotation_cs(e);
     const int nimg = Np * nang;
     CK(cudaMemsetAsync(ctx->pstats.p, 0, sizeof(double) * 2 * N * nang, ctx->stream));
-    // rows that the mask's disc (radius 0.75 d_m + 12) reaches, in whole tiles of 16
-    const float rout = 0.75f * ctx->p.d_m + 12.0f;
-    const int row0 = std::max(0, (int)std::floor((float)(l / 2) - std::min(rout, (float)l)) - 1) / 16 * 16;
-    const int row1 = std::min(l, ((int)std::ceil((float)(l / 2) + std::min(rout, (float)l)) + 2 + 15) / 16 * 16);
-    dim3 g(blocks_for((long long)(row1 - row0) * l, 256, 32), Np, nang);
-    k_pair_rotate<<<g, 256, 0, ctx->stream>>>(P<float>(ctx->tmpl), N, l, c.x, c.y, cs, ctx->p.d_m, row0, row1, TS,
+    const MaskRows mr = mask_rows(ctx->p.d_m, l);
+    dim3 g(blocks_for((long long)(mr.row1 - mr.row0) * l, 256, 32), Np, nang);
+    k_pair_rotate<<<g, 256, 0, ctx->stream>>>(P<float>(ctx->tmpl), N, l, c.x, c.y, cs, ctx->p.d_m, mr.row0, mr.row1, TS,
                                               P<double>(ctx->pstats));
     ++ctx->counters.kernel_launches;
     k_pair_coef<<<blocks_for(nimg, 128), 128, 0, ctx->stream>>>(P<double>(ctx->pstats), N, l,
                                                                 P<float4>(ctx->coef), nang);
     ++ctx->counters.kernel_launches;
     CKL();
-    if (const WinOps* w = win_of(ctx, l)) {
-        const F16PairNorm rows{TS, P<float4>(ctx->coef), l, l2, row0};
-        FftPlan* pl = nullptr;
-        TRY(get_plan(ctx, l, &pl));
-        if (nimg > 65535) return set_err(ctx, GS_ERR_UNSUPPORTED, "too many images in one FFT batch (%d)", nimg);
-        const int tiles = (row1 - row0) / 16;
-        TRY(win_status(ctx, pfa ? w->pair_rows_pfa(pl->tw, nimg, tiles, F16PairNormPfa{rows, PfaCols::make(l)}, ctx->stream)
-                                : w->pair_rows(pl->tw, nimg, tiles, rows, ctx->stream), "pair rows"));
-        TRY(run_win(ctx, l, nimg, w->pair_cols, F16PairCols{TS, l, l2, (float)(1.0 / (double)l2), row0, row1}));
-    } else {
-        VecGeom rows = rows_of(l, l);
-        rows.nvec = row1 - row0;
-        TRY(run_fft<false>(ctx, l, rows, nimg, IoPairNorm{TS + (long long)row0 * l, P<float4>(ctx->coef)}));
-        TRY(run_fft<false>(ctx, l, cols_of(l, l), nimg, IoPairCols{TS, (float)(1.0 / (double)l2), row0, row1}));
-    }
-    return GS_OK;
+    return disc_transform(ctx, TS, P<float4>(ctx->coef), nimg, mr, (float)(1.0 / (double)l2), 0.0f, pfa);
 }
 static int pair_spectra(gs_ctx* ctx, float e, float2* TS, bool pfa = false) {
     return pair_spectra_n(ctx, e, nullptr, 1, TS, pfa);
@@ -678,22 +693,6 @@ static int search_norm1_passes(gs_ctx* ctx, const float2* W, int nx, int ny, con
     return GS_OK;
 }
 
-// Soft mask factor of apply_mask (GPU_func.cu:229-247), the arithmetic of
-// k_pair_rotate.
-__global__ void k_ref_mask(float* __restrict__ mask, int l, float d_m) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= l * l) return;
-    const int h = l / 2;
-    const int i = q % l, j = q / l;
-    const float dm = 1.5f * d_m;
-    const float rin = dm / 2.0f, rout = dm / 2.0f + 12.0f;
-    const float r = hypotf((float)(i - h), (float)(j - h));
-    float m = 1.0f;
-    if (r > rout) m = 0.0f;
-    else if (r >= rin) m = (float)(0.5 * (double)cosf((float)(kPiRef * (double)(r - rin) / 12.0)) + 0.5);
-    mask[q] = m;
-}
-
 // Objective (and with grad, its gradient) of n picks, chunked.  tgrad: host
 // n x l x l floats or null.
 static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool grad, gs_refine_result* out,
@@ -712,22 +711,21 @@ static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool
             !std::isfinite(q.dfdiff) || !std::isfinite(q.dfang))
             return set_err(ctx, GS_ERR_ARG, "pick %d: parameter not finite", i);
     }
-    // per-pick bytes: 6 complex + 2 real maps
-    const long long per = l2 * (6 * (long long)sizeof(float2) + 2 * (long long)sizeof(float));
-    const int chunk = (int)std::max<long long>(1, std::min<long long>(n, (2ll << 30) / per));
+    // per pick three complex and three real maps, and the phase factors
+    const long long per = l2 * (3 * (long long)sizeof(float2) + 3 * (long long)sizeof(float)) + 2 * l * (long long)sizeof(double2);
+    const int chunk = (int)std::max<long long>(1, std::min<long long>(std::min(n, 65535), (2ll << 30) / per));
     TRY(ensure(ctx, ctx->rf_pk, sizeof(RefinePickDev) * chunk));
     TRY(ensure(ctx, ctx->rf_acc, sizeof(RefineAcc) * chunk));
-    TRY(ensure(ctx, ctx->rf_B, sizeof(float2) * l2 * chunk));
+    TRY(ensure(ctx, ctx->rf_scale, (sizeof(double) * 2 + sizeof(float4) * 2) * chunk));
+    TRY(ensure(ctx, ctx->rf_ph, sizeof(double2) * 2 * l * chunk));
     TRY(ensure(ctx, ctx->rf_F1, sizeof(float2) * l2 * chunk));
-    TRY(ensure(ctx, ctx->rf_T, sizeof(float2) * l2 * chunk));
+    TRY(ensure(ctx, ctx->rf_T, sizeof(float) * l2 * chunk));
     TRY(ensure(ctx, ctx->rf_TM, sizeof(float) * l2 * chunk));
     TRY(ensure(ctx, ctx->rf_F, sizeof(float2) * l2 * chunk));
     TRY(ensure(ctx, ctx->rf_G, sizeof(float2) * l2 * chunk));
     TRY(ensure(ctx, ctx->rf_TB, sizeof(float) * l2 * chunk));
     TRY(ensure(ctx, ctx->rf_mask, sizeof(float) * l2));
-    k_ref_mask<<<blocks_for(l2, 256), 256, 0, ctx->stream>>>(P<float>(ctx->rf_mask), l, p.d_m);
-    ++ctx->counters.kernel_launches;
-    CKL();
+    TRY(ensure(ctx, ctx->rf_bins, sizeof(RefineBin) * l2));
     RefineConsts rc;
     rc.l = l;
     rc.L2 = l2;
@@ -753,19 +751,45 @@ static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool
             }
         rc.cnt = (float)cnt;
     }
+    k_ref_maps<<<blocks_for(l2, 256), 256, 0, ctx->stream>>>(P<float>(ctx->rf_mask), P<RefineBin>(ctx->rf_bins), rc);
+    ++ctx->counters.kernel_launches;
+    CKL();
     const float sgn = ((l / 2) % 2 == 0) ? 1.0f : -1.0f;
     RefinePickDev* d_pk = P<RefinePickDev>(ctx->rf_pk);
     RefineAcc* d_acc = P<RefineAcc>(ctx->rf_acc);
-    float2* B = P<float2>(ctx->rf_B);
+    float4* coef = P<float4>(ctx->rf_scale);                          // 1 / sd, then 1
+    double* inva = reinterpret_cast<double*>(coef + 2 * chunk);
+    double* scale = inva + chunk;                                     // 1 / l^2
+    double2* phases = P<double2>(ctx->rf_ph);
     float2* F1 = P<float2>(ctx->rf_F1);
-    float2* T = P<float2>(ctx->rf_T);
+    float* T = P<float>(ctx->rf_T);
     float* TM = P<float>(ctx->rf_TM);
     float2* F = P<float2>(ctx->rf_F);
     float2* Gm = P<float2>(ctx->rf_G);
     float* TB = P<float>(ctx->rf_TB);
     const float* mask = P<float>(ctx->rf_mask);
+    const RefineBin* bins = P<RefineBin>(ctx->rf_bins);
+    const float2* base = P<float2>(ctx->tbase);
     const float2* W = P<float2>(ctx->win);
     const float inv_l2 = (float)(1.0 / (double)l2);
+    const MaskRows mr = mask_rows(p.d_m, l);
+    {
+        std::vector<double> one(chunk, 1.0 / (double)l2);
+        CK(cudaMemcpyAsync(scale, one.data(), sizeof(double) * chunk, cudaMemcpyHostToDevice, ctx->stream));
+    }
+    // transforms of nc maps: real part of the inverse (factor[img] on load, `data`
+    // overwritten), and the forward one of maps that are zero outside mr
+    auto inverse_real = [&](float2* data, const double* factor, float* out, int nc) -> int {
+        if (const WinOps* w = win_of(ctx, l)) {
+            TRY(run_win(ctx, l, nc, w->inv_rows, F16ScaleIn<false>{data, factor, l, l2}));
+            return run_win(ctx, l, nc, w->inv_cols, F16RealOut<true>{data, out, l, l2});
+        }
+        TRY(run_fft<true>(ctx, l, rows_of(l, l), nc, IoScaleIn{data, factor}));
+        return run_fft<true>(ctx, l, cols_of(l, l), nc, IoRealOut{data, out, 1.0f});
+    };
+    auto forward_disc = [&](float2* data, const float4* cf, float factor, float dc, int nc) -> int {
+        return disc_transform(ctx, data, cf, nc, mr, factor, dc, false);
+    };
     std::vector<RefinePickDev> hp(chunk);
     std::vector<RefineAcc> ha(chunk);
     for (int c0 = 0; c0 < n; c0 += chunk) {
@@ -782,41 +806,34 @@ static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool
         }
         CK(cudaMemcpyAsync(d_pk, hp.data(), sizeof(RefinePickDev) * nc, cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaMemsetAsync(d_acc, 0, sizeof(RefineAcc) * nc, ctx->stream));
-        const dim3 g(blocks_for(l2, 256, 128), nc);
+        const dim3 g(blocks_for(l2, 256, 128), nc), gd(blocks_for((long long)(mr.row1 - mr.row0) * l, 256, 128), nc);
         // forward
-        TRY(run_fft<false>(ctx, l, rows_of(l, l), nc, IoBaseIn{P<float>(ctx->tbase), d_pk, B, l2}));
-        TRY(run_fft<false>(ctx, l, cols_of(l, l), nc, IoComplex{B, inv_l2}));
-        k_ref_weight<<<g, 256, 0, ctx->stream>>>(B, F1, d_pk, rc, d_acc);
-        ++ctx->counters.kernel_launches;
-        TRY(run_fft<true>(ctx, l, rows_of(l, l), nc, IoInvA{F1, T, d_acc, rc.cnt, l2}));
-        TRY(run_fft<true>(ctx, l, cols_of(l, l), nc, IoComplex{T, 1.0f}));
-        k_ref_rotate<<<g, 256, 0, ctx->stream>>>(T, TM, d_pk, rc, mask, d_acc);
-        ++ctx->counters.kernel_launches;
-        TRY(run_fft<false>(ctx, l, rows_of(l, l), nc, IoNormIn{TM, d_acc, F, l2}));
-        TRY(run_fft<false>(ctx, l, cols_of(l, l), nc, IoComplex{F, inv_l2}));
-        k_ref_score<<<g, 256, 0, ctx->stream>>>(W, F, d_pk, rc, d_acc);
-        ++ctx->counters.kernel_launches;
+        k_ref_phases<<<dim3(blocks_for(2 * l, 128), nc), 128, 0, ctx->stream>>>(d_pk, l, phases);
+        k_ref_weight<<<g, 256, 0, ctx->stream>>>(base, bins, F1, Gm, d_pk, rc, d_acc);
+        k_ref_inva<<<blocks_for(nc, 128), 128, 0, ctx->stream>>>(d_acc, nc, (double)rc.cnt, inva);
+        TRY(inverse_real(Gm, inva, T, nc));
+        k_ref_rotate<<<gd, 256, 0, ctx->stream>>>(T, TM, F, d_pk, rc, mr.row0, mr.row1, mask, d_acc);
+        k_ref_coef<<<blocks_for(nc, 128), 128, 0, ctx->stream>>>(d_acc, nc, (double)l2, coef);
+        TRY(forward_disc(F, coef, inv_l2, 0.0f, nc));
+        k_ref_score<<<g, 256, 0, ctx->stream>>>(W, F, d_pk, phases, rc, d_acc);
+        ctx->counters.kernel_launches += 6;
         CKL();
         if (grad) {
-            TRY(run_fft<true>(ctx, l, rows_of(l, l), nc, IoFbarIn{W, F, d_pk, d_acc, Gm, l, l2, sgn}));
-            TRY(run_fft<true>(ctx, l, cols_of(l, l), nc, IoComplex{Gm, inv_l2}));
-            k_ref_gsum<<<g, 256, 0, ctx->stream>>>(Gm, TM, rc, d_acc);
-            ++ctx->counters.kernel_launches;
-            CK(cudaMemsetAsync(TB, 0, sizeof(float) * l2 * nc, ctx->stream));
-            k_ref_rot_adj<<<g, 256, 0, ctx->stream>>>(Gm, TM, T, d_pk, rc, mask, d_acc, TB);
-            ++ctx->counters.kernel_launches;
-            // Fbar2 = FFT(tbar), into Gm (gamma no longer needed)
-            TRY(run_fft<false>(ctx, l, rows_of(l, l), nc, IoRealIn2{TB, Gm}));
-            TRY(run_fft<false>(ctx, l, cols_of(l, l), nc, IoComplex{Gm, 1.0f}));
+            k_ref_fbar<<<g, 256, 0, ctx->stream>>>(W, F, d_pk, phases, d_acc, l, sgn, Gm);
+            TRY(inverse_real(Gm, scale, TB, nc));
+            k_ref_gsum<<<g, 256, 0, ctx->stream>>>(TB, TM, rc, mr.row0, mr.row1, d_acc);
+            CK(cudaMemset2DAsync(Gm + (size_t)mr.row0 * l, sizeof(float2) * l2, 0,
+                                 sizeof(float2) * (size_t)(mr.row1 - mr.row0) * l, nc, ctx->stream));
+            k_ref_rot_adj<<<gd, 256, 0, ctx->stream>>>(TB, TM, T, d_pk, rc, mr.row0, mr.row1, mask, d_acc, Gm);
+            // Fbar2 = FFT(tbar)
+            TRY(forward_disc(Gm, coef + nc, 1.0f, 1.0f, nc));
             k_ref_abar<<<g, 256, 0, ctx->stream>>>(Gm, F1, rc, d_acc);
-            ++ctx->counters.kernel_launches;
-            k_ref_theta<<<g, 256, 0, ctx->stream>>>(Gm, F1, B, d_pk, rc, d_acc);
-            ++ctx->counters.kernel_launches;
+            k_ref_theta<<<g, 256, 0, ctx->stream>>>(Gm, F1, base, bins, d_pk, rc, tgrad != nullptr, d_acc);
+            ctx->counters.kernel_launches += 5;
             CKL();
             if (tgrad) {
-                // bbar = Re IFFT(Bbar) / l^2, real maps into TB
-                TRY(run_fft<true>(ctx, l, rows_of(l, l), nc, IoComplex{Gm, 1.0f}));
-                TRY(run_fft<true>(ctx, l, cols_of(l, l), nc, IoRealOut{Gm, TB, inv_l2}));
+                // bbar = Re IFFT(Bbar) / l^2
+                TRY(inverse_real(Gm, scale, TB, nc));
                 CK(cudaMemcpyAsync(tgrad + (size_t)c0 * l2, TB, sizeof(float) * l2 * nc, cudaMemcpyDeviceToHost,
                                    ctx->stream));
             }
@@ -996,7 +1013,7 @@ int gs_ctx_destroy(gs_ctx* ctx) {
                     &ctx->off, &ctx->win, &ctx->wsum, &ctx->winv, &ctx->tspec, &ctx->scratch, &ctx->pstats,
                     &ctx->coef, &ctx->acc, &ctx->units, &ctx->picks, &ctx->count, &ctx->unit_wp,
                     &ctx->dep_counters, &ctx->pacc, &ctx->flags, &ctx->tbase, &ctx->rf_pk, &ctx->rf_acc,
-                    &ctx->rf_B, &ctx->rf_F1, &ctx->rf_T, &ctx->rf_TM, &ctx->rf_F, &ctx->rf_G, &ctx->rf_TB,
+                    &ctx->rf_scale, &ctx->rf_ph, &ctx->rf_bins, &ctx->rf_F1, &ctx->rf_T, &ctx->rf_TM, &ctx->rf_F, &ctx->rf_G, &ctx->rf_TB,
                     &ctx->rf_mask, &ctx->pix_keys, &ctx->pix_pairs, &ctx->pix_R, &ctx->tc2_wmax,
                     &ctx->tc2_pmax, &ctx->tc2_w16, &ctx->tc2_p16, &ctx->rot_cs, &ctx->tp_raw, &ctx->tp_div, &ctx->tp_sums, &ctx->tp_wmap};
     for (DBuf* b : bufs) free_buf(*b);
@@ -1057,11 +1074,11 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
     ctx->ty = ty;
     const size_t l2 = (size_t)l * l;
     TRY(ensure(ctx, ctx->tmpl, sizeof(float) * l2 * n));
-    TRY(ensure(ctx, ctx->tbase, sizeof(float) * l2 * n));
+    TRY(ensure(ctx, ctx->tbase, sizeof(float2) * (size_t)l * (l / 2 + 1) * n));
     // templates per pass: spectra of 256 MiB keep every kernel busy for tens of
     // microseconds
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>(std::min(n, 65535), (size_t)(256u << 20) / (l2 * 8)));
-    DBuf &raw = ctx->tp_raw, &F = ctx->tspec, &Fb = ctx->scratch, &div = ctx->tp_div, &wmap = ctx->tp_wmap;
+    DBuf &raw = ctx->tp_raw, &F = ctx->tspec, &div = ctx->tp_div, &wmap = ctx->tp_wmap;
     const int ns = l / 2;
     int st = GS_OK;
     do {
@@ -1073,7 +1090,6 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
         if ((st = ensure(ctx, div, sizeof(float) * (size_t)ns * chunk))) break;
         if ((st = ensure(ctx, ctx->tp_sums, sums_bytes))) break;
         if ((st = ensure(ctx, wmap, sizeof(float) * l2))) break;
-        if ((st = ensure(ctx, Fb, sizeof(float2) * l2 * chunk))) break;
         double* edge = P<double>(ctx->tp_sums);
         double* sumsq = edge + 4 * (size_t)chunk;
         double* inv = sumsq + 2 * (size_t)chunk;
@@ -1118,21 +1134,14 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
             k_tmpl_shells<<<dim3(blocks_for((long long)l2 / 2, 2048, 32), nc), 256, shs, ctx->stream>>>(
                 P<float2>(F), l, shells, shell_count);
             k_tmpl_shell_rms<<<blocks_for((long long)nc * ns, 256), 256, 0, ctx->stream>>>(shells, shell_count, ns, nc,
-                                                                                         P<float>(div), inv);
+                                                                                         P<float>(div));
             ctx->counters.kernel_launches += 2;
             // weighted spectra, and the whitened base (before the weight), kept for
             // the refinement
             dim3 g(blocks_for((long long)l2, 256, 64), nc);
-            k_tmpl_apply<<<g, 256, 0, ctx->stream>>>(P<float2>(F), l, P<float>(div), P<float>(wmap), sumsq, P<float2>(Fb));
+            k_tmpl_apply<<<g, 256, 0, ctx->stream>>>(P<float2>(F), l, P<float>(div), P<float>(wmap), sumsq,
+                                                     P<float2>(ctx->tbase) + (size_t)c0i * l * (l / 2 + 1));
             ++ctx->counters.kernel_launches;
-            float* base = P<float>(ctx->tbase) + (size_t)c0i * l2;
-            if (w) {
-                if ((st = run_win(ctx, l, nc, w->inv_rows, F16ScaleIn<false>{P<float2>(Fb), inv, l, (long long)l2}))) break;
-                if ((st = run_win(ctx, l, nc, w->inv_cols, F16RealOut<true>{P<float2>(Fb), base, l, (long long)l2}))) break;
-            } else {
-                if ((st = run_fft<true>(ctx, l, rows_of(l, l), nc, IoComplex{P<float2>(Fb), 1.0f}))) break;
-                if ((st = run_fft<true>(ctx, l, cols_of(l, l), nc, IoRealOut{P<float2>(Fb), base, 1.0f}))) break;
-            }
             k_inv_amp_norm<<<blocks_for(nc, 128), 128, 0, ctx->stream>>>(sumsq, nc, inv);
             ++ctx->counters.kernel_launches;
             if (cudaGetLastError() != cudaSuccess) { st = set_err(ctx, GS_ERR_CUDA, "template weighting"); break; }

@@ -109,12 +109,11 @@ static __global__ void __launch_bounds__(256) k_tmpl_shells(const float2* __rest
     }
 }
 
-// div[J ns + r]: the shell's RMS; one[J] = 1 (the base's scale).
+// div[J ns + r]: the shell's RMS.
 static __global__ void k_tmpl_shell_rms(const double* __restrict__ sum, const unsigned* __restrict__ count, int ns,
-                                        int n, float* __restrict__ div, double* __restrict__ one) {
+                                        int n, float* __restrict__ div) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n * ns) div[i] = (float)sqrt(sum[i] / (double)count[i % ns]);
-    if (i < n) one[i] = 1.0;
 }
 
 struct WeightConsts {
@@ -144,9 +143,9 @@ static __global__ void k_weight_map(float* __restrict__ wmap, int l, WeightConst
 }
 
 // Whiten by the shell RMS, apply the weight map, and accumulate per template
-// sum |F|^2 and the count over r < l/2, x <= l/2.  The whitened spectrum without
-// the weight goes to B: the base that the off-grid refinement re-weights with
-// other CTF parameters.
+// sum |F|^2 and the count over r < l/2, x <= l/2.  The half plane x <= l/2 of the
+// whitened spectrum without the weight goes to B (rows of l/2 + 1): the base that
+// the off-grid refinement re-weights with other CTF parameters.
 // Reference: whiten_Tmp + apply_weighting_function + compute_area_sum_ofSQR
 // (GPU_func.cu:130-152, 249-290, 318-362).  Grid (pixel chunks, templates).
 static __global__ void __launch_bounds__(256) k_tmpl_apply(float2* __restrict__ F, int l, const float* __restrict__ div,
@@ -164,7 +163,7 @@ static __global__ void __launch_bounds__(256) k_tmpl_apply(float2* __restrict__ 
         const int r = shell_index(x, y, l, l);
         float2 v = d[i];
         if (r >= 0 && r < ns) v = cscale(v, 1.0f / dv[r]);
-        B[(size_t)J * npix + i] = v;
+        if (x <= l / 2) B[((size_t)J * l + y) * (l / 2 + 1) + x] = v;
         v = cscale(v, wmap[i]);
         d[i] = v;
         if (r >= 0 && r < ns && x <= l / 2) {
@@ -502,11 +501,12 @@ struct IoPairCols {
     float2* data;
     float scale;
     int row0, row1;
+    float dc = 0.0f;  // factor of the zero frequency
     __device__ float2 load(int, int, int k, long long a) const {
         return k >= row0 && k < row1 ? data[a] : make_float2(0.0f, 0.0f);
     }
     __device__ void store(int, int v, int k, long long a, float2 x) const {
-        data[a] = v + k == 0 ? make_float2(0.0f, 0.0f) : cscale(x, scale);
+        data[a] = cscale(x, v + k == 0 ? scale * dc : scale);
     }
     __device__ void finish(double*, int, int) const {}
 };

@@ -5,7 +5,8 @@
 // position x0, in-plane angle e, sub-pixel shift d, CTF theta = (defocus,
 // dfdiff, dfang) of the template weight):
 //   B   = FFT(b_J) / l^2                 b_J: padded, edge-normalised,
-//                                        whitened template (main.cu:182-431)
+//                                        whitened template (main.cu:182-431);
+//                                        kept as its spectrum's half plane
 //   F1  = B w(k; theta)                  band-pass x |CTF| Wiener weight
 //                                        (GPU_func.cu:249-290)
 //   t   = Re IFFT(F1 / a), a = sqrt(sum_sel |F1|^2) / cnt  (main.cu:447-463)
@@ -21,6 +22,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "kernels.cuh"
 
 namespace gs {
 
@@ -50,27 +52,44 @@ struct RefineConsts {
     float cnt;  // number of (r < l/2, x <= l/2) bins
 };
 
-// Weight w(k; theta) and, optionally, its theta derivatives (float; the
-// value path is the same arithmetic as k_weight_map).
-__device__ __forceinline__ float refine_weight(int x, int y, const RefineConsts& rc, const RefinePickDev& pk,
-                                               bool* insel, float dw[3]) {
+// What the weight takes of a bin that does not depend on the pick: band-pass
+// factor (negative: bin not selected, the weight is its magnitude alone), s^2 and
+// azimuth of the CTF's folded frequency, noise curve over signal.  One table per
+// call, read by every pick.
+struct RefineBin {
+    float band, ss, ag, ncurve;
+};
+
+__device__ __forceinline__ RefineBin refine_bin(int x, int y, const RefineConsts& rc) {
     const int l = rc.l;
     float rf;
     const int r = shell_index(x, y, l, l, &rf);
     const float band = bandpass<false>(r, rc.hp, rc.lp);
-    *insel = (r < l / 2 && r >= 0);
-    dw[0] = dw[1] = dw[2] = 0.0f;
-    if (!*insel) return band;
+    if (!(r < l / 2 && r >= 0)) return RefineBin{-band - 1.0f, 0.0f, 0.0f, 1.0f};
     // CTF geometry of ctf_ast(x, (y + l/2) % l)
     int x1 = x, y1 = (y + l / 2) % l;
     y1 = x1 > l / 2 ? l - y1 : y1;
     x1 = min(x1, l - x1);
     const float fx = (float)x1, fy = (float)(y1 - l / 2);
     const float ss = (fx * fx / (float)(l * l) + fy * fy / (float)(l * l)) / (rc.apix * rc.apix);
-    const float ag = atan2f(fy, fx);
+    const float ssw = rf * rc.ds;
+    const float signal = expf(rc.bf * ssw * ssw + rc.bf2 * ssw + rc.bf3) / (rc.kk + 1.0f);
+    const float ncurve = expf(rc.a * ssw * ssw + rc.b * ssw + rc.b2) / signal;
+    return RefineBin{band, ss, atan2f(fy, fx), ncurve};
+}
+
+// Weight w(k; theta) and, with kGrad, its theta derivatives (float; the value
+// path is the same arithmetic as k_weight_map).
+template <bool kGrad>
+__device__ __forceinline__ float refine_weight(const RefineBin& bin, const RefineConsts& rc, const RefinePickDev& pk,
+                                               bool* insel, float dw[3]) {
+    *insel = bin.band >= 0.0f;
+    if constexpr (kGrad) dw[0] = dw[1] = dw[2] = 0.0f;
+    if (!*insel) return -bin.band - 1.0f;
+    const float ss = bin.ss;
     const float D = -pk.defocus;
     const float dfu = D + pk.dfdiff, dfv = D - pk.dfdiff;
-    const float ang2 = (float)(2.0 * ((double)pk.dfang * kPiRef / 180.0 - (double)ag));
+    const float ang2 = (float)(2.0 * ((double)pk.dfang * kPiRef / 180.0 - (double)bin.ag));
     const float cs2 = cosf(ang2);
     const float df_ast = 0.5f * (dfu + dfv + 2.0f * pk.dfdiff * cs2);
     const double lam = (double)rc.lambda;
@@ -82,52 +101,65 @@ __device__ __forceinline__ float refine_weight(int x, int y, const RefineConsts&
     sincosf(gamma, &sg, &cg);
     const float V = sa * sg + rc.ampconst * cg;
     const float v = fabsf(V);
-    const float ssw = rf * rc.ds;
-    const float signal = expf(rc.bf * ssw * ssw + rc.bf2 * ssw + rc.bf3) / (rc.kk + 1.0f);
-    const float ncurve = expf(rc.a * ssw * ssw + rc.b * ssw + rc.b2) / signal;
-    const float den = ncurve + rc.kk * v * v;
+    const float den = bin.ncurve + rc.kk * v * v;
     const float w = v * sqrtf(1.0f / den);
-    // d w / d gamma = band * ncurve den^-3/2 * sign(V) (sa cos g - a sin g)
-    const float dwdg = band * ncurve / (den * sqrtf(den)) * (V >= 0.0f ? 1.0f : -1.0f) *
-                       (sa * cg - rc.ampconst * sg);
-    const float dgdf = (float)(-2.0 * kPiRef * 5000.0 * lam * (double)ss);  // d gamma / d df_ast
-    dw[0] = dwdg * dgdf * -1.0f;                                            // d df_ast / d defocus = -1
-    dw[1] = dwdg * dgdf * cs2;                                              // d df_ast / d dfdiff
-    dw[2] = dwdg * dgdf * (-2.0f * pk.dfdiff * sinf(ang2)) * (float)(kPiRef / 180.0);
-    return band * w;
+    if constexpr (kGrad) {
+        // d w / d gamma = band * ncurve den^-3/2 * sign(V) (sa cos g - a sin g)
+        const float dwdg = bin.band * bin.ncurve / (den * sqrtf(den)) * (V >= 0.0f ? 1.0f : -1.0f) *
+                           (sa * cg - rc.ampconst * sg);
+        const float dgdf = (float)(-2.0 * kPiRef * 5000.0 * lam * (double)ss);  // d gamma / d df_ast
+        dw[0] = dwdg * dgdf * -1.0f;                                            // d df_ast / d defocus = -1
+        dw[1] = dwdg * dgdf * cs2;                                              // d df_ast / d dfdiff
+        dw[2] = dwdg * dgdf * (-2.0f * pk.dfdiff * sinf(ang2)) * (float)(kPiRef / 180.0);
+    }
+    return bin.band * w;
+}
+
+// Soft mask factor of apply_mask (GPU_func.cu:229-247), the arithmetic of
+// k_pair_rotate, and the bins' table.
+static __global__ void k_ref_maps(float* __restrict__ mask, RefineBin* __restrict__ bins, RefineConsts rc) {
+    const int l = rc.l, q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= l * l) return;
+    const int h = l / 2, i = q % l, j = q / l;
+    const float dm = 1.5f * rc.d_m;
+    const float rin = dm / 2.0f, rout = dm / 2.0f + 12.0f;
+    const float r = hypotf((float)(i - h), (float)(j - h));
+    float m = 1.0f;
+    if (r > rout) m = 0.0f;
+    else if (r >= rin) m = (float)(0.5 * (double)cosf((float)(kPiRef * (double)(r - rin) / 12.0)) + 0.5);
+    mask[q] = m;
+    bins[q] = refine_bin(i, j, rc);
+}
+
+// Bin (x, y) of a base spectrum from its half plane.
+__device__ __forceinline__ float2 ref_base(const float2* __restrict__ H, int x, int y, int l) {
+    const int hw = l / 2 + 1;
+    if (x <= l / 2) return __ldg(H + y * hw + x);
+    const float2 v = __ldg(H + (y ? l - y : 0) * hw + (l - x));
+    return make_float2(v.x, -v.y);
 }
 
 // ---- forward ----
 
-// Row pass input of B = FFT(b_J): real base template of the pick's template.
-struct IoBaseIn {
-    const float* base;     // N x L2
-    const RefinePickDev* pk;
-    float2* out;           // picks x L2 (complex)
-    long long L2;
-    __device__ float2 load(int img, int, int, long long a) const {
-        return make_float2(base[(long long)pk[img].tmpl * L2 + (a - (long long)img * L2)], 0.0f);
-    }
-    __device__ void store(int, int, int, long long a, float2 v) const { out[a] = v; }
-    __device__ void finish(double*, int, int) const {}
-};
-
-// F1 = B w(theta); sum_sel |F1|^2 per pick.  Grid (pixel chunks, picks).
-__global__ void __launch_bounds__(256) k_ref_weight(const float2* __restrict__ B, float2* __restrict__ F1,
-                                                    const RefinePickDev* __restrict__ pks, RefineConsts rc,
-                                                    RefineAcc* __restrict__ acc) {
+// F1 = B w(theta), a second copy of it (transformed in place), and sum_sel |F1|^2
+// per pick.  Grid (pixel chunks, picks).
+static __global__ void __launch_bounds__(256) k_ref_weight(const float2* __restrict__ base, const RefineBin* __restrict__ bins,
+                                                           float2* __restrict__ F1, float2* __restrict__ copy,
+                                                           const RefinePickDev* __restrict__ pks, RefineConsts rc,
+                                                           RefineAcc* __restrict__ acc) {
     __shared__ double red[32];
     const int p = blockIdx.y;
     const RefinePickDev pk = pks[p];
-    const int l = rc.l;
+    const int l = rc.l, npix = l * l;
+    const float2* H = base + (long long)pk.tmpl * l * (l / 2 + 1);
     double s = 0.0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rc.L2; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % l), y = (int)(i / l);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
+        const int y = i / l, x = i - y * l;
         bool insel;
-        float dw[3];
-        const float w = refine_weight(x, y, rc, pk, &insel, dw);
-        const float2 v = cscale(B[p * rc.L2 + i], w);
+        const float w = refine_weight<false>(bins[i], rc, pk, &insel, nullptr);
+        const float2 v = cscale(ref_base(H, x, y, l), w);
         F1[p * rc.L2 + i] = v;
+        copy[p * rc.L2 + i] = v;
         if (insel && x <= l / 2) s += (double)v.x * v.x + (double)v.y * v.y;
     }
     double v1[1] = {s};
@@ -135,20 +167,12 @@ __global__ void __launch_bounds__(256) k_ref_weight(const float2* __restrict__ B
     if (threadIdx.x == 0) atomicAdd(&acc[p].asum, v1[0]);
 }
 
-// t = Re IFFT(F1 / a) (row pass: in F1 scaled by 1/a into T; column pass real out).
-struct IoInvA {
-    const float2* F1;
-    float2* T;
-    const RefineAcc* acc;
-    float cnt;
-    long long L2;
-    __device__ float2 load(int img, int, int, long long a) const {
-        const float inva = (float)((double)cnt / sqrt(acc[img].asum));
-        return cscale(F1[a], inva);
-    }
-    __device__ void store(int, int, int, long long a, float2 v) const { T[a] = v; }
-    __device__ void finish(double*, int, int) const {}
-};
+// Per-pick factors of the transforms: 1 / a for t = Re IFFT(F1 / a); after the
+// rotation, (1 / sd of tm) as a pair coefficient.
+static __global__ void k_ref_inva(const RefineAcc* __restrict__ acc, int n, double cnt, double* __restrict__ inva) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < n) inva[p] = cnt / sqrt(acc[p].asum);
+}
 
 // Source coordinates of rotate_subIMG for output pixel (i, j) and angle e.
 __device__ __forceinline__ void rot_src(int i, int j, int l, float c, float s, float* x2, float* y2) {
@@ -187,27 +211,32 @@ __device__ __forceinline__ Bilin bilin(float x2, float y2, int l) {
     return b;
 }
 
-// tm = mask . rotate(t, e) into TM (real), sums of tm and tm^2.
-__global__ void __launch_bounds__(256) k_ref_rotate(const float2* __restrict__ T, float* __restrict__ TM,
-                                                    const RefinePickDev* __restrict__ pks, RefineConsts rc,
-                                                    const float* __restrict__ mask, RefineAcc* __restrict__ acc) {
+// tm = mask . rotate(t, e), real and as the input of its transform, in the rows
+// [row0, row1) that the mask's disc reaches; sums of tm and tm^2.
+static __global__ void __launch_bounds__(256) k_ref_rotate(const float* __restrict__ T, float* __restrict__ TM,
+                                                           float2* __restrict__ F, const RefinePickDev* __restrict__ pks,
+                                                           RefineConsts rc, int row0, int row1,
+                                                           const float* __restrict__ mask, RefineAcc* __restrict__ acc) {
     __shared__ double red[64];
     const int p = blockIdx.y;
     const int l = rc.l;
     const double ang = (double)pks[p].e * kPiRef / 180.0;
     const float c = (float)cos(ang), s = (float)sin(ang);
-    const float2* src = T + p * rc.L2;
+    const float* src = T + p * rc.L2;
     double a2[2] = {0.0, 0.0};
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rc.L2; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % l), y = (int)(i / l);
-        float x2, y2;
-        rot_src(x, y, l, c, s, &x2, &y2);
-        const Bilin b = bilin(x2, y2, l);
+    for (int i = row0 * l + blockIdx.x * blockDim.x + threadIdx.x; i < row1 * l; i += gridDim.x * blockDim.x) {
+        const int y = i / l, x = i - y * l;
+        const float m = mask[i];
         float v = 0.0f;
-        if (b.inb)
-            v = src[b.k[0]].x * b.w[0] + src[b.k[1]].x * b.w[1] + src[b.k[3]].x * b.w[3] + src[b.k[2]].x * b.w[2];
-        v *= mask[i];
+        if (m != 0.0f) {
+            float x2, y2;
+            rot_src(x, y, l, c, s, &x2, &y2);
+            const Bilin b = bilin(x2, y2, l);
+            if (b.inb) v = src[b.k[0]] * b.w[0] + src[b.k[1]] * b.w[1] + src[b.k[3]] * b.w[3] + src[b.k[2]] * b.w[2];
+            v *= m;
+        }
         TM[p * rc.L2 + i] = v;
+        F[p * rc.L2 + i] = make_float2(v, 0.0f);
         a2[0] += v;
         a2[1] += (double)v * v;
     }
@@ -224,60 +253,62 @@ __device__ __forceinline__ void ref_moments(const RefineAcc& a, double L2, doubl
     *sd = sqrt(var > 0.0 ? var : 1.0);
 }
 
-// Row pass input of F = FFT(tn): normalised tm.
-struct IoNormIn {
-    const float* TM;
-    const RefineAcc* acc;
-    float2* out;
-    long long L2;
-    __device__ float2 load(int img, int, int, long long a) const {
-        double mu, sd;
-        ref_moments(acc[img], (double)L2, &mu, &sd);
-        return make_float2((float)(((double)TM[a] - mu) / sd), 0.0f);
-    }
-    __device__ void store(int, int, int, long long a, float2 v) const { out[a] = v; }
-    __device__ void finish(double*, int, int) const {}
-};
+// coef[p]: tm's 1 / sd as IoPairNorm takes it (the mean only reaches the zero
+// frequency of FFT(tn), which is 0); coef[n + p]: no scaling.
+static __global__ void k_ref_coef(const RefineAcc* __restrict__ acc, int n, double L2, float4* __restrict__ coef) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    double mu, sd;
+    ref_moments(acc[p], L2, &mu, &sd);
+    coef[p] = make_float4(0.0f, (float)(1.0 / sd), 0.0f, 0.0f);
+    coef[n + p] = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
+}
 
-// Phase exp(2 pi i (kx (x0 + dx) + ky (y0 + dy)) / l) with signed k; the
-// integer part of the phase in integer arithmetic.
-__device__ __forceinline__ float2 ref_phase(int kx, int ky, int l, const RefinePickDev& pk, int* kxs, int* kys) {
-    const int sx = kx < (l + 1) / 2 ? kx : kx - l;
-    const int sy = ky < (l + 1) / 2 ? ky : ky - l;
-    *kxs = sx;
-    *kys = sy;
-    long long ip = ((long long)sx * pk.x0 + (long long)sy * pk.y0) % l;
+// Phase factors exp(2 pi i kx (x0 + dx) / l), kx = 0 .. l - 1 (signed), then the
+// same of ky, per pick; the integer part of the phase in integer arithmetic.
+static __global__ void k_ref_phases(const RefinePickDev* __restrict__ pks, int l, double2* __restrict__ ph) {
+    const int p = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 2 * l) return;
+    const int k = i < l ? i : i - l;
+    const int sk = k < (l + 1) / 2 ? k : k - l;
+    const RefinePickDev pk = pks[p];
+    long long ip = (long long)sk * (i < l ? pk.x0 : pk.y0) % l;
     if (ip < 0) ip += l;
-    const double frac = ((double)ip + (double)sx * pk.dx + (double)sy * pk.dy) / (double)l;
+    const double frac = ((double)ip + (double)sk * (i < l ? pk.dx : pk.dy)) / (double)l;
     double sn, cs;
     sincospi(2.0 * (frac - floor(frac)), &sn, &cs);
-    return make_float2((float)cs, (float)sn);
+    ph[(size_t)p * 2 * l + i] = make_double2(cs, sn);
+}
+__device__ __forceinline__ float2 ref_phase(const double2* __restrict__ ph, int kx, int ky, int l) {
+    const double2 a = ph[kx], b = ph[l + ky];
+    return make_float2((float)(a.x * b.x - a.y * b.y), (float)(a.x * b.y + a.y * b.x));
 }
 
 // c, sigma^2 and d c / d (dx, dy): reductions over the spectrum.
-__global__ void __launch_bounds__(256) k_ref_score(const float2* __restrict__ W, const float2* __restrict__ F,
-                                                   const RefinePickDev* __restrict__ pks, RefineConsts rc,
-                                                   RefineAcc* __restrict__ acc) {
+static __global__ void __launch_bounds__(256) k_ref_score(const float2* __restrict__ W, const float2* __restrict__ F,
+                                                          const RefinePickDev* __restrict__ pks,
+                                                          const double2* __restrict__ phases, RefineConsts rc,
+                                                          RefineAcc* __restrict__ acc) {
     __shared__ double red[4 * 32];
     const int p = blockIdx.y;
-    const RefinePickDev pk = pks[p];
-    const int l = rc.l;
-    const float2* Wp = W + (long long)pk.window * rc.L2;
+    const int l = rc.l, npix = l * l;
+    const float2* Wp = W + (long long)pks[p].window * rc.L2;
     const float2* Fp = F + p * rc.L2;
+    const double2* ph = phases + (size_t)p * 2 * l;
+    const double step = 2.0 * kPiRef / l;
     double a4[4] = {0.0, 0.0, 0.0, 0.0};
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rc.L2; i += (long long)gridDim.x * blockDim.x) {
-        const int kx = (int)(i % l), ky = (int)(i / l);
-        int sx, sy;
-        const float2 E = ref_phase(kx, ky, l, pk, &sx, &sy);
-        const float2 G = cmulc(Wp[i], Fp[i]);          // W conj(F)
-        const float2 GE = cmul(G, E);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
+        const int ky = i / l, kx = i - ky * l;
+        const int sx = kx < (l + 1) / 2 ? kx : kx - l, sy = ky < (l + 1) / 2 ? ky : ky - l;
+        const float2 E = ref_phase(ph, kx, ky, l), w = Wp[i], f = Fp[i];
+        const float2 GE = cmul(cmulc(w, f), E);        // W conj(F) E
         a4[0] += GE.x;
-        const float w2 = Wp[i].x * Wp[i].x + Wp[i].y * Wp[i].y;
-        const float f2 = Fp[i].x * Fp[i].x + Fp[i].y * Fp[i].y;
+        const float w2 = w.x * w.x + w.y * w.y;
+        const float f2 = f.x * f.x + f.y * f.y;
         a4[1] += (double)w2 * f2;
         // d/d dx of Re(GE) = Re(GE * 2 pi i kx / l) = -Im(GE) 2 pi kx / l
-        a4[2] += -(double)GE.y * (2.0 * kPiRef * sx / l);
-        a4[3] += -(double)GE.y * (2.0 * kPiRef * sy / l);
+        a4[2] += -(double)GE.y * (step * sx);
+        a4[3] += -(double)GE.y * (step * sy);
     }
     block_sum<4>(a4, red);
     if (threadIdx.x == 0) {
@@ -290,63 +321,58 @@ __global__ void __launch_bounds__(256) k_ref_score(const float2* __restrict__ W,
 
 // ---- backward ----
 
-// Fbar = (sgn / sig) W E - (sgn c / sig^3) |W|^2 F, then (column pass of) the
-// inverse transform: gamma = Re IFFT(Fbar) / l^2.
-struct IoFbarIn {
-    const float2* W;
-    const float2* F;
-    const RefinePickDev* pk;
-    const RefineAcc* acc;
-    float2* out;
-    int l;
-    long long L2;
-    float sgn;
-    __device__ float2 load(int img, int, int, long long a) const {
-        const long long i = a - (long long)img * L2;
-        const int kx = (int)(i % l), ky = (int)(i / l);
-        int sx, sy;
-        const RefinePickDev q = pk[img];
-        const float2 E = ref_phase(kx, ky, l, q, &sx, &sy);
-        const float2 w = W[(long long)q.window * L2 + i];
-        const float2 f = F[a];
-        const double sig = sqrt(acc[img].sig2);
-        const float c1 = (float)(sgn / sig);
-        const float c2 = (float)(sgn * acc[img].c / (sig * sig * sig));
+// Fbar = (sgn / sig) W E - (sgn c / sig^3) |W|^2 F, whose inverse transform is
+// gamma l^2.
+static __global__ void __launch_bounds__(256) k_ref_fbar(const float2* __restrict__ W, const float2* __restrict__ F,
+                                                         const RefinePickDev* __restrict__ pks,
+                                                         const double2* __restrict__ phases,
+                                                         const RefineAcc* __restrict__ acc, int l, float sgn,
+                                                         float2* __restrict__ out) {
+    const int p = blockIdx.y, npix = l * l;
+    const float2* Wp = W + (long long)pks[p].window * npix;
+    const double2* ph = phases + (size_t)p * 2 * l;
+    const double sig = sqrt(acc[p].sig2);
+    const float c1 = (float)(sgn / sig);
+    const float c2 = (float)(sgn * acc[p].c / (sig * sig * sig));
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
+        const int ky = i / l, kx = i - ky * l;
+        const float2 w = Wp[i], f = F[(long long)p * npix + i];
         const float w2 = w.x * w.x + w.y * w.y;
-        const float2 we = cmul(w, E);
-        return make_float2(c1 * we.x - c2 * w2 * f.x, c1 * we.y - c2 * w2 * f.y);
+        const float2 we = cmul(w, ref_phase(ph, kx, ky, l));
+        out[(long long)p * npix + i] = make_float2(c1 * we.x - c2 * w2 * f.x, c1 * we.y - c2 * w2 * f.y);
     }
-    __device__ void store(int, int, int, long long a, float2 v) const { out[a] = v; }
-    __device__ void finish(double*, int, int) const {}
-};
+}
 
-// sums of gamma and gamma tn (gamma = real part of G, already / l^2).
-__global__ void __launch_bounds__(256) k_ref_gsum(const float2* __restrict__ Gm, const float* __restrict__ TM,
-                                                  RefineConsts rc, RefineAcc* __restrict__ acc) {
+// sums of gamma and gamma tn (tn = (tm - mu) / sd; tm is 0 outside [row0, row1)).
+static __global__ void __launch_bounds__(256) k_ref_gsum(const float* __restrict__ G, const float* __restrict__ TM,
+                                                         RefineConsts rc, int row0, int row1,
+                                                         RefineAcc* __restrict__ acc) {
     __shared__ double red[64];
-    const int p = blockIdx.y;
+    const int p = blockIdx.y, npix = rc.l * rc.l;
     double mu, sd;
     ref_moments(acc[p], (double)rc.L2, &mu, &sd);
     double a2[2] = {0.0, 0.0};
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rc.L2; i += (long long)gridDim.x * blockDim.x) {
-        const double g = Gm[p * rc.L2 + i].x;
-        const double tn = ((double)TM[p * rc.L2 + i] - mu) / sd;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
+        const double g = G[p * rc.L2 + i];
+        const bool in = i >= row0 * rc.l && i < row1 * rc.l;
         a2[0] += g;
-        a2[1] += g * tn;
+        a2[1] += g * ((in ? (double)TM[p * rc.L2 + i] : 0.0) - mu);
     }
     block_sum<2>(a2, red);
     if (threadIdx.x == 0) {
         atomicAdd(&acc[p].g1, a2[0]);
-        atomicAdd(&acc[p].g2, a2[1]);
+        atomicAdd(&acc[p].g2, a2[1] / sd);
     }
 }
 
 // Normalisation, mask and rotation adjoints: d s / d e (reduction) and
-// tbar (scatter-add into TB, real parts, zeroed beforehand).
-__global__ void __launch_bounds__(256) k_ref_rot_adj(const float2* __restrict__ Gm, const float* __restrict__ TM,
-                                                     const float2* __restrict__ T, const RefinePickDev* __restrict__ pks,
-                                                     RefineConsts rc, const float* __restrict__ mask,
-                                                     RefineAcc* __restrict__ acc, float* __restrict__ TB) {
+// tbar (scatter-add into the real parts of TB, zeroed beforehand in the rows
+// [row0, row1), which hold all of it).
+static __global__ void __launch_bounds__(256) k_ref_rot_adj(const float* __restrict__ G, const float* __restrict__ TM,
+                                                            const float* __restrict__ T,
+                                                            const RefinePickDev* __restrict__ pks, RefineConsts rc,
+                                                            int row0, int row1, const float* __restrict__ mask,
+                                                            RefineAcc* __restrict__ acc, float2* __restrict__ TB) {
     __shared__ double red[32];
     const int p = blockIdx.y;
     const int l = rc.l;
@@ -356,21 +382,24 @@ __global__ void __launch_bounds__(256) k_ref_rot_adj(const float2* __restrict__ 
     const double mg = acc[p].g1 / L2, mgt = acc[p].g2 / L2;
     const double ang = (double)pks[p].e * kPiRef / 180.0;
     const float c = (float)cos(ang), s = (float)sin(ang);
-    const float2* src = T + p * rc.L2;
-    float* tb = TB + p * rc.L2;
+    const float* src = T + p * rc.L2;
+    float2* tb = TB + p * rc.L2;
+    const double inv_sd = 1.0 / sd;
     const float dr = (float)(kPiRef / 180.0);
     double de = 0.0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rc.L2; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % l), y = (int)(i / l);
-        const double g = Gm[p * rc.L2 + i].x;
-        const double tn = ((double)TM[p * rc.L2 + i] - mu) / sd;
-        const float gm = (float)((g - mg - tn * mgt) / sd) * mask[i];  // d s / d rotated pixel
+    for (int i = row0 * l + blockIdx.x * blockDim.x + threadIdx.x; i < row1 * l; i += gridDim.x * blockDim.x) {
+        const float m = mask[i];
+        if (m == 0.0f) continue;
+        const int y = i / l, x = i - y * l;
+        const double g = G[p * rc.L2 + i];
+        const double tn = ((double)TM[p * rc.L2 + i] - mu) * inv_sd;
+        const float gm = (float)((g - mg - tn * mgt) * inv_sd) * m;  // d s / d rotated pixel
         if (gm == 0.0f) continue;
         float x2, y2;
         rot_src(x, y, l, c, s, &x2, &y2);
         const Bilin b = bilin(x2, y2, l);
         if (!b.inb) continue;
-        const float v0 = src[b.k[0]].x, v1 = src[b.k[1]].x, v2 = src[b.k[2]].x, v3 = src[b.k[3]].x;
+        const float v0 = src[b.k[0]], v1 = src[b.k[1]], v2 = src[b.k[2]], v3 = src[b.k[3]];
         // value = (1-t)(1-u) v0 + t(1-u) v1 + t u v2 + (1-t) u v3
         const float dvdt = (1.0f - b.du) * (v1 - v0) + b.du * (v2 - v3);
         const float dvdu = (1.0f - b.dt) * (v3 - v0) + b.dt * (v2 - v1);
@@ -378,24 +407,15 @@ __global__ void __launch_bounds__(256) k_ref_rot_adj(const float2* __restrict__ 
         const float dx2 = dr * (-s * xf + c * yf), dy2 = dr * (-c * xf - s * yf);
         de += (double)gm * (dvdt * dx2 + dvdu * dy2);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) atomicAdd(&tb[b.k[q]], gm * b.w[q]);
+        for (int q = 0; q < 4; ++q) atomicAdd(&tb[b.k[q]].x, gm * b.w[q]);
     }
     double v1[1] = {de};
     block_sum<1>(v1, red);
     if (threadIdx.x == 0) atomicAdd(&acc[p].de, v1[0]);
 }
 
-// Row pass input of Fbar2 = FFT(tbar) (real).
-struct IoRealIn2 {
-    const float* src;
-    float2* out;
-    __device__ float2 load(int, int, int, long long a) const { return make_float2(src[a], 0.0f); }
-    __device__ void store(int, int, int, long long a, float2 v) const { out[a] = v; }
-    __device__ void finish(double*, int, int) const {}
-};
-
 // abar = -Re sum Fbar2 conj(F1) / a^2 (only the sum here).
-__global__ void __launch_bounds__(256) k_ref_abar(const float2* __restrict__ Fb2, const float2* __restrict__ F1,
+static __global__ void __launch_bounds__(256) k_ref_abar(const float2* __restrict__ Fb2, const float2* __restrict__ F1,
                                                   RefineConsts rc, RefineAcc* __restrict__ acc) {
     __shared__ double red[32];
     const int p = blockIdx.y;
@@ -410,35 +430,41 @@ __global__ void __launch_bounds__(256) k_ref_abar(const float2* __restrict__ Fb2
 }
 
 // Fbar1 = Fbar2 / a + abar_total F1 sel / (cnt^2 a); theta gradient
-// reductions; Bbar = Fbar1 w written over Fb2 (for the template gradient).
-__global__ void __launch_bounds__(256) k_ref_theta(float2* __restrict__ Fb2, const float2* __restrict__ F1,
-                                                   const float2* __restrict__ B, const RefinePickDev* __restrict__ pks,
-                                                   RefineConsts rc, RefineAcc* __restrict__ acc) {
+// reductions; with `store`, Bbar = Fbar1 w written over Fb2 (for the template
+// gradient).
+static __global__ void __launch_bounds__(256) k_ref_theta(float2* __restrict__ Fb2, const float2* __restrict__ F1,
+                                                          const float2* __restrict__ base,
+                                                          const RefineBin* __restrict__ bins,
+                                                          const RefinePickDev* __restrict__ pks, RefineConsts rc,
+                                                          bool store, RefineAcc* __restrict__ acc) {
     __shared__ double red[3 * 32];
     const int p = blockIdx.y;
     const RefinePickDev pk = pks[p];
-    const int l = rc.l;
+    const int l = rc.l, npix = l * l;
+    const float2* H = base + (long long)pk.tmpl * l * (l / 2 + 1);
     const double a = sqrt(acc[p].asum) / (double)rc.cnt;
     const double abar = -acc[p].abar / (a * a);
     const double k2 = abar / ((double)rc.cnt * (double)rc.cnt * a);
+    const float inva = (float)(1.0 / a);
     double t3[3] = {0.0, 0.0, 0.0};
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rc.L2; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % l), y = (int)(i / l);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
+        const int y = i / l, x = i - y * l;
         bool insel;
         float dw[3];
-        const float w = refine_weight(x, y, rc, pk, &insel, dw);
-        const float2 f1 = F1[p * rc.L2 + i];
-        float2 fb = cscale(Fb2[p * rc.L2 + i], (float)(1.0 / a));
+        const float w = refine_weight<true>(bins[i], rc, pk, &insel, dw);
+        if (!insel && !store) continue;
+        float2 fb = cscale(Fb2[p * rc.L2 + i], inva);
         if (insel && x <= l / 2) {
+            const float2 f1 = F1[p * rc.L2 + i];
             fb.x += (float)(k2 * f1.x);
             fb.y += (float)(k2 * f1.y);
         }
-        const float2 bb = B[p * rc.L2 + i];
+        const float2 bb = ref_base(H, x, y, l);
         const double re = (double)fb.x * bb.x + (double)fb.y * bb.y;  // Re(Fbar1 conj(B))
         t3[0] += re * dw[0];
         t3[1] += re * dw[1];
         t3[2] += re * dw[2];
-        Fb2[p * rc.L2 + i] = cscale(fb, w);
+        if (store) Fb2[p * rc.L2 + i] = cscale(fb, w);
     }
     block_sum<3>(t3, red);
     if (threadIdx.x == 0) {
