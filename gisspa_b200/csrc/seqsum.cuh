@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kSeqThreads) k_seq_apply(const float* __restri
                                                            const SeqBlock* __restrict__ blocks, int nblocks,
                                                            float* __restrict__ sums) {
     extern __shared__ __align__(16) float seq_buf[];
-    __shared__ SeqRun runs[32];
+    __shared__ SeqRun runs[2][32];
     __shared__ float sh_s;
     __shared__ int sh_b;
     q += blockIdx.x * stride;
@@ -295,49 +295,69 @@ __global__ void __launch_bounds__(kSeqThreads) k_seq_apply(const float* __restri
         __syncthreads();
         b = sh_b;
         if (b >= nblocks) break;
-        // block b by its parts
+        // block b by its warps' parts, whose runs are kept for two binades (a sum
+        // near a power of two goes back and forth); in any other one warp 0
+        // composes the part it needs itself
         seq_stage(seq_buf, q, (long long)b * kSeqBlock, n);
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        const unsigned binade = seq_binade(sh_s);
-        auto part = [&](int w, unsigned bin) {  // the run of warp w's 512 terms, by the calling warp
-            float t[kSeqTerms];
+        float t[kSeqTerms];
 #pragma unroll
-            for (int j = 0; j < kSeqTerms; j += 4) {
-                const float4 v = *reinterpret_cast<const float4*>(seq_buf + (w * 32 + lane) * kSeqPitch + j);
-                t[j] = v.x; t[j + 1] = v.y; t[j + 2] = v.z; t[j + 3] = v.w;
+        for (int j = 0; j < kSeqTerms; j += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(seq_buf + threadIdx.x * kSeqPitch + j);
+            t[j] = v.x; t[j + 1] = v.y; t[j + 2] = v.z; t[j + 3] = v.w;
+        }
+        unsigned have[2] = {0u, 0u};  // binades of runs[0], runs[1]
+        int w = 0;                    // parts before w are in the sum
+        while (w < 32) {
+            const unsigned binade = seq_binade(sh_s);
+            if (binade) {
+                const int slot = have[0] ? 1 : 0;
+                const SeqRun r = seq_warp(seq_run(t, seq_scale(binade)));
+                if (lane == 0) runs[slot][warp] = r;
+                have[slot] = binade;
             }
-            return seq_warp(seq_run(t, seq_scale(bin)));
-        };
-        SeqRun r = seq_identity();
-        if (binade) r = part(warp, binade);
-        if (lane == 0) runs[warp] = r;
-        __syncthreads();
-        if (warp == 0) {
-            float s = sh_s;
-            for (int w = 0; w < 32; ++w) {
-                const unsigned now = seq_binade(s);
-                // (only lane 0 of a warp holds its composition)
-                bool ok = false;
-                if (now && now == binade) {
-                    ok = seq_apply(s, now, runs[w]);
-                } else if (now) {
-                    const SeqRun p = part(w, now);
-                    if (lane == 0) ok = seq_apply(s, now, p);
-                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                    s = __shfl_sync(0xffffffffu, s, 0);
-                }
-                if (ok) continue;
-                const float4* v = reinterpret_cast<const float4*>(seq_buf + w * 32 * kSeqPitch);
-#pragma unroll 4
-                for (int c = 0; c < 32; ++c)
+            __syncthreads();
+            if (warp == 0) {
+                float s = sh_s;
+                for (; w < 32; ++w) {
+                    const unsigned now = seq_binade(s);
+                    bool ok = false;
+                    if (now == have[0]) {
+                        ok = seq_apply(s, now, runs[0][w]);
+                    } else if (now == have[1]) {
+                        ok = seq_apply(s, now, runs[1][w]);
+                    } else if (now && !have[1]) {
+                        break;
+                    } else if (now) {
+                        float u[kSeqTerms];
 #pragma unroll
-                    for (int j = 0; j < kSeqTerms / 4; ++j) {
-                        const float4 a = v[c * (kSeqPitch / 4) + j];
-                        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a.x), a.y), a.z), a.w);
+                        for (int j = 0; j < kSeqTerms; j += 4) {
+                            const float4 v = *reinterpret_cast<const float4*>(seq_buf + (w * 32 + lane) * kSeqPitch + j);
+                            u[j] = v.x; u[j + 1] = v.y; u[j + 2] = v.z; u[j + 3] = v.w;
+                        }
+                        const SeqRun r = seq_warp(seq_run(u, seq_scale(now)));  // in lane 0
+                        if (lane == 0) ok = seq_apply(s, now, r);
+                        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                        s = __shfl_sync(0xffffffffu, s, 0);
                     }
+                    if (ok) continue;
+                    const float4* v = reinterpret_cast<const float4*>(seq_buf + w * 32 * kSeqPitch);
+#pragma unroll 4
+                    for (int c = 0; c < 32; ++c)
+#pragma unroll
+                        for (int j = 0; j < kSeqTerms / 4; ++j) {
+                            const float4 a = v[c * (kSeqPitch / 4) + j];
+                            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a.x), a.y), a.z), a.w);
+                        }
+                }
+                if (lane == 0) {
+                    sh_s = s;
+                    sh_b = w;
+                }
             }
-            if (lane == 0) sh_s = s;
+            __syncthreads();
+            w = sh_b;
         }
         ++b;
         __syncthreads();
