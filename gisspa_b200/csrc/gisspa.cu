@@ -96,6 +96,7 @@ struct gs_ctx {
     cudaStream_t copy = nullptr;    // uploads of large micrographs
     cudaEvent_t in_ready[2] = {nullptr, nullptr}, in_free[2] = {nullptr, nullptr};
     void* pinned = nullptr;         // staging of uploads from pageable memory (upload_host)
+    size_t uploaded = 0;            // bytes that went through upload_host
     std::vector<cudaEvent_t> pinned_ev;
     DBuf q, cimg, img, stats, ra, rb, off, win, wsum, winv;
     DBuf tspec, scratch, pstats, coef, acc, units, picks, count;
@@ -1192,15 +1193,17 @@ struct MicPlan {
 // through the driver's own staging with one core, at about 10 GB/s: 9.0 ms for a
 // 5760 x 4092 micrograph.  Four threads fill eight pinned buffers of 1 MiB
 // instead: 2.8 ms (two threads 4.1, eight 3.4; buffers of 512 KiB 3.9).
-// Whatever part of that cannot be had (pinned memory, threads) only makes it
-// slower.
-constexpr size_t kUploadChunk = 1u << 20, kUploadStaged = 4u << 20;
+// The buffers take 5 to 20 ms to pin, so the first 64 MiB of a context go the
+// driver's way.  Whatever part of it cannot be had (pinned memory, threads) only
+// makes it slower.
+constexpr size_t kUploadChunk = 1u << 20, kUploadStaged = 4u << 20, kUploadFirst = 64u << 20;
 constexpr int kUploadThreads = 4;
 static int upload_host(gs_ctx* ctx, void* dst, const void* src, size_t bytes) {
     cudaPointerAttributes at{};
     const bool pageable = cudaPointerGetAttributes(&at, src) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    bool staged = pageable;
+    bool staged = pageable && ctx->uploaded >= kUploadFirst;
+    ctx->uploaded += bytes;
     if (staged && !ctx->pinned &&
         cudaHostAlloc(&ctx->pinned, 2 * kUploadThreads * kUploadChunk, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
