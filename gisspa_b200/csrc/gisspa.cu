@@ -1635,13 +1635,14 @@ static int search_norm1(gs_ctx* ctx, const float2* W, int nx, int ny, const std:
     const long long per_angle = (long long)nw * N * nblk;  // block maxima
     const long long nu = (long long)Np * nw;
     const WinOps* ops = win_of(ctx, l);
-    if (ctx->two_pass || !ops || !ops->corr_moments || !units_fit(l, nu)) {
+    auto passes = [&]() -> int {
         TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np));
         TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * Np));
         TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N));
         TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np));
         return search_norm1_passes(ctx, W, nx, ny, offx, offy, angles, ms_spec, ms_corr, out);
-    }
+    };
+    if (ctx->two_pass || !ops || !ops->corr_moments || !units_fit(l, nu)) return passes();
     // angles per launch as in the norm_type 0 search, with the block maxima and
     // their picks within 2 GiB
     int A = launch_angles(ctx, (int)nu, na, false);
@@ -1650,16 +1651,25 @@ static int search_norm1(gs_ctx* ctx, const float2* W, int nx, int ny, const std:
     CorrTuning tune;
     TRY(default_tuning(ctx, false, &tune));
     tune.tile = 16;
-    TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np * A));
-    TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N * A));
-    TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np * A));
-    TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * tune.slots));
-    TRY(ensure(ctx, ctx->dep_counters, sizeof(int) * (2 * (size_t)nu * A + 4)));
-    TRY(ensure(ctx, ctx->flags, sizeof(int) * 4));
-    TRY(ensure(ctx, ctx->pacc, sizeof(float2) * l2 * nw));  // per-pixel moments
-    TRY(ensure(ctx, ctx->units, sizeof(unsigned long long) * per_angle * A));
-    TRY(ensure(ctx, ctx->picks, sizeof(BlockPickDev) * per_angle * A));
-    TRY(ensure(ctx, ctx->count, sizeof(unsigned long long)));
+    auto buffers = [&]() -> int {
+        TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np * A));
+        TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N * A));
+        TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np * A));
+        TRY(ensure(ctx, ctx->unit_wp, sizeof(int2) * (size_t)nu * A));
+        TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * tune.slots));
+        TRY(ensure(ctx, ctx->dep_counters, sizeof(int) * (2 * (size_t)nu * A + 4)));
+        TRY(ensure(ctx, ctx->flags, sizeof(int) * 4));
+        TRY(ensure(ctx, ctx->pacc, sizeof(float2) * l2 * nw));  // per-pixel moments
+        TRY(ensure(ctx, ctx->units, sizeof(unsigned long long) * per_angle * A));
+        TRY(ensure(ctx, ctx->picks, sizeof(BlockPickDev) * per_angle * A));
+        return ensure(ctx, ctx->count, sizeof(unsigned long long));
+    };
+    // fewer angles per launch where memory is short, then the passes of one window
+    for (int st; (st = buffers()) != GS_OK; A = (A + 1) / 2) {
+        if (st != GS_ERR_OOM) return st;
+        for (DBuf* b : {&ctx->tspec, &ctx->scratch, &ctx->dep_counters, &ctx->pacc, &ctx->units, &ctx->picks}) free_buf(*b);
+        if (A == 1) return passes();
+    }
     TRY(upload_rotations(ctx, angles));
     TRY(upload_unit_order(ctx, nw, Np, tune.window_block, (int)(nu * A), A));
     CK(cudaMemsetAsync(ctx->flags.p, 0, sizeof(int) * 4, ctx->stream));
@@ -1728,7 +1738,14 @@ static int prefetch_pair_spectra(gs_ctx* ctx, int NW, const std::vector<float>& 
     if (!units_fit(l, nu)) return GS_OK;  // the correlation reports it
     const bool pfa = (p.precision == GS_PREC_FP32 || tc2) && PfaCols::make(l).N2 != 0;
     const int A = launch_angles(ctx, nu, na, tc2);
-    TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np * A));
+    // the preparation's and the correlation's own buffers come first where memory is short
+    const size_t spec_bytes = sizeof(float2) * l2 * Np * A;
+    size_t mem_free = 0, mem_total = 0;
+    if (ctx->tspec.cap < spec_bytes) {
+        CK(cudaMemGetInfo(&mem_free, &mem_total));
+        if (mem_free / 2 < spec_bytes) return GS_OK;
+    }
+    TRY(ensure(ctx, ctx->tspec, spec_bytes));
     TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N * A));
     TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np * A));
     TRY(upload_rotations(ctx, angles));
@@ -1799,19 +1816,38 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         CK(cudaStreamWaitEvent(ctx->stream, ctx->side_ev[1], 0));
         prefetched = 0;
     }
-    TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np * A));
-    TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N * A));
-    TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np * A));
+    CorrTuning tune;
+    TRY(default_tuning(ctx, tc2, &tune));
+    // a launch takes fewer angles where the device has no memory for A of them
+    // (the frees wait for whatever still uses the buffers)
+    auto buffers = [&]() -> int {
+        TRY(ensure(ctx, ctx->units, sizeof(UnitOut) * std::max<long long>(1, total_units)));
+        TRY(ensure(ctx, ctx->acc, sizeof(UnitAcc) * N));
+        TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np * A));
+        TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N * A));
+        TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np * A));
+        if (persistent || chunked) {
+            TRY(ensure(ctx, ctx->unit_wp, sizeof(int2) * std::max<size_t>(1, (size_t)nu * A)));
+            TRY(ensure(ctx, ctx->pacc, sizeof(UnitAcc) * 2 * (size_t)nu * A));
+        }
+        if (persistent) {
+            TRY(ensure(ctx, ctx->dep_counters, sizeof(int) * (2 * (size_t)nu * A + 4)));
+            return ensure(ctx, ctx->scratch, sizeof(float2) * l2 * (ctx->autotune ? std::max(32, tune.slots) : tune.slots));
+        }
+        return ensure(ctx, ctx->scratch, sizeof(float2) * l2 * (chunked ? std::min<long long>(chunk, (long long)nu * A) : Np));
+    };
+    for (int st; (st = buffers()) != GS_OK; A = (A + 1) / 2) {
+        if (st != GS_ERR_OOM || A == 1) return st;
+        if (prefetched) CK(cudaStreamWaitEvent(ctx->stream, ctx->side_ev[1], 0));
+        prefetched = 0;
+        for (DBuf* b : {&ctx->tspec, &ctx->pacc, &ctx->dep_counters, &ctx->scratch}) free_buf(*b);
+    }
     // (a prefetch uploaded them already, and its kernels may still read them)
     if (!prefetched) TRY(upload_rotations(ctx, angles));
-    TRY(ensure(ctx, ctx->acc, sizeof(UnitAcc) * N));
-    TRY(ensure(ctx, ctx->units, sizeof(UnitOut) * std::max<long long>(1, total_units)));
     float2* TS = P<float2>(ctx->tspec);
     UnitOut* units = P<UnitOut>(ctx->units);
     FftPlan* plan = nullptr;
     TRY(get_plan(ctx, l, &plan));  // before any capture: plan creation copies synchronously
-    CorrTuning tune;
-    TRY(default_tuning(ctx, tc2, &tune));
     // window spectra in PfaCols order for the duration of the correlation,
     // natural order again afterwards (on every return path)
     struct PfaWindows {
@@ -1847,12 +1883,9 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         CKL();
     }
     if (persistent) {
-        TRY(ensure(ctx, ctx->dep_counters, sizeof(int) * (2 * (size_t)nu * A + 4)));
-        TRY(ensure(ctx, ctx->pacc, sizeof(UnitAcc) * 2 * (size_t)nu * A));
         TRY(ensure(ctx, ctx->flags, sizeof(int) * 4));
         CK(cudaMemsetAsync(ctx->flags.p, 0, sizeof(int) * 4, ctx->stream));
         if (ctx->autotune) {
-            TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * std::max(32, tune.slots)));
             TRY(pair_spectra(ctx, angles[0], TS, pfa));
             if (tc2) {
                 CK(cudaMemsetAsync(ctx->tc2_pmax.p, 0, sizeof(float) * Np, ctx->stream));
@@ -1869,10 +1902,6 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * tune.slots));
     } else if (chunked) {
         TRY(upload_unit_order(ctx, NW, Np, tune.window_block, nu * A, A));
-        TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * std::min<long long>(chunk, (long long)nu * A)));
-        TRY(ensure(ctx, ctx->pacc, sizeof(UnitAcc) * 2 * (size_t)nu * A));
-    } else {
-        TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * Np));
     }
     ctx->last_tuning[0] = tune.slots;
     ctx->last_tuning[1] = tune.lag;
