@@ -264,7 +264,7 @@ int run_fft(gs_ctx* ctx, int n, VecGeom g, int nimg, IO io, int max_tile = 16) {
     if (pl->plan.A && !ctx->generic_fft && nimg <= 65535) {
         PlanDesc d = pl->plan;
         int tile = plan_tile(&d, g.nvec, g.elem_stride != 1);
-        if (tile) {
+        if (tile && plan_strides_fit(d, g, tile)) {
             tile = std::min(tile, max_tile);
             plan_layout(&d, tile);
             const size_t smem = plan_smem_bytes(d, tile);

@@ -582,7 +582,9 @@ struct IoPass2 {
         int Y = k + h; if (Y >= l) Y -= l;
         const int pos = Y * l + X;
         const float v1 = sgn * val.x, v2 = sgn * val.y;
-        const bool border = (float)X < q_lo || (float)X > q_hi || (float)Y < q_lo || (float)Y > q_hi;
+        // q_lo and q_hi as whole numbers: X < q_lo as floats is X < ceil(q_lo)
+        const int lo = q_lo > 0.0f ? (int)ceilf(q_lo) : 0, hi = q_hi < (float)l ? (int)floorf(q_hi) : l;
+        const bool border = X < lo || X > hi || Y < lo || Y > hi;
         if (!border) {
             const unsigned long long a = argmax_key(v1, pos), b = argmax_key(v2, pos);
             k1 = a > k1 ? a : k1;

@@ -178,7 +178,7 @@ cudaError_t launch_plan(PlanDesc d, VecGeom g, int nimg, IO io, cudaStream_t st,
     for (int tile = 16; d.A && tile >= 1; tile /= 2) {
         plan_layout(&d, tile);
         const size_t smem = plan_smem_bytes(d, tile);
-        if (smem > (tile > 4 ? 72u << 10 : 220u << 10)) continue;
+        if (smem > (tile > 4 ? 72u << 10 : 220u << 10) || !plan_strides_fit(d, g, tile)) continue;
         auto kern = fft_plan_kernel<kInv, IO>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

@@ -13,6 +13,10 @@
 // Bound by latency and issue: rows of 5760 values take two CTAs of 256
 // threads to an SM.  The stage code is one function per direction, called by every IO
 // variant of the kernel, so that its radices are compiled once.
+// Without batching, a thread waits for one load at a time (long scoreboard 8 of
+// 14 stalled cycles per issue at length 300, 27 % issue): with four in flight and
+// 32-bit offsets the 4320 units of 300 x 300 take 5.4 ms instead of 7.5, the
+// preparation of a 4096 x 4096 micrograph 5.0 instead of 6.4 (eight in flight: the same).
 #pragma once
 
 #include "regfft.cuh"
@@ -105,6 +109,11 @@ inline void plan_layout(PlanDesc* d, int tile) {
 inline size_t plan_smem_bytes(const PlanDesc& d, int tile) {
     return ((size_t)tile * d.VP * (d.dense ? 2 : 1) + (d.dense ? d.C : 0)) * sizeof(float2) +
            (size_t)kFftRedDoubles * sizeof(double);
+}
+
+// A tile's offsets fit an int.
+inline bool plan_strides_fit(const PlanDesc& d, const VecGeom& g, int tile) {
+    return (long long)tile * g.vec_stride + (long long)d.n * g.elem_stride < (1ll << 31);
 }
 
 // One stage: per vector `d_count.d` butterflies of radix R; butterfly j starts at
@@ -272,13 +281,28 @@ __global__ void __launch_bounds__(256, 3) fft_plan_kernel(const __grid_constant_
     const int nv = min(tile, g.nvec - v0);
     const int n = D.n, tot = nv * n;
     const bool contiguous = g.elem_stride == 1;
+    // 32-bit offsets within the tile (plan_strides_fit)
+    const long long base = vec_addr(g, img, v0, 0);
+    const int vs = (int)g.vec_stride, es = (int)g.elem_stride;
     const SmallDiv dv = nv == tile ? D.dtile : SmallDiv{(unsigned)nv, nv == 1 ? 0u : (0xffffffffu / (unsigned)nv + 1u)};
-    for (int i = threadIdx.x; i < tot; i += blockDim.x) {
-        int t, k;
-        if (contiguous) { t = quot(i, D.dn); k = i - t * n; }
-        else { k = quot(i, dv); t = i - k * nv; }
-        const int n1 = quot(k, D.dBC), m = k - n1 * (int)D.dBC.d, n2 = quot(m, D.dC), n3 = m - n2 * D.C;
-        buf[t * D.VP + n1 * D.P1 + n2 * D.P2 + n3] = io.load(img, v0 + t, k, vec_addr(g, img, v0 + t, k));
+    // four loads in flight per thread (a clamped index repeats the last load)
+    constexpr int kU = 4;
+    for (int i0 = threadIdx.x; i0 < tot; i0 += kU * blockDim.x) {
+        float2 x[kU];
+        int at[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int i = min(i0 + u * (int)blockDim.x, tot - 1);
+            int t, k;
+            if (contiguous) { t = quot(i, D.dn); k = i - t * n; }
+            else { k = quot(i, dv); t = i - k * nv; }
+            const int n1 = quot(k, D.dBC), m = k - n1 * (int)D.dBC.d, n2 = quot(m, D.dC), n3 = m - n2 * D.C;
+            at[u] = t * D.VP + n1 * D.P1 + n2 * D.P2 + n3;
+            x[u] = io.load(img, v0 + t, k, base + (t * vs + k * es));
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+            if (i0 + u * (int)blockDim.x < tot) buf[at[u]] = x[u];
     }
     __syncthreads();
     const float2* res = plan_block_fft<kInv>(buf, alt, tab, nv, D);
@@ -287,7 +311,7 @@ __global__ void __launch_bounds__(256, 3) fft_plan_kernel(const __grid_constant_
         if (contiguous) { t = quot(i, D.dn); k = i - t * n; }
         else { k = quot(i, dv); t = i - k * nv; }
         const int q = quot(k, D.dA), k1 = k - q * D.A, k3 = quot(q, D.dB), k2 = q - k3 * D.B;
-        io.store(img, v0 + t, k, vec_addr(g, img, v0 + t, k), res[t * D.VP + k1 * D.P1 + k2 * D.P2 + k3]);
+        io.store(img, v0 + t, k, base + (t * vs + k * es), res[t * D.VP + k1 * D.P1 + k2 * D.P2 + k3]);
     }
     double* red = reinterpret_cast<double*>(smem_plan + (size_t)tile * D.VP * (D.dense ? 2 : 1) + (D.dense ? D.C : 0));
     io.finish(red, v0, nv);
