@@ -1775,9 +1775,11 @@ static int prefetch_pair_spectra(gs_ctx* ctx, int NW, const std::vector<float>& 
     return GS_OK;
 }
 
-// Row-pass maps of one chunked launch (correlate_all): enough units for many
-// CTAs per SM (window 300: 186 units, 3534 CTAs) while the maps stay in L2.
-constexpr long long kChunkBytes = 128ll << 20;
+// Row-pass maps of one chunked launch (correlate_all).  The transforms are bound
+// by issue, not by where the maps lie, and every launch ends in a wave that is
+// nearly empty: 4320 units of window 300 take 5.96, 5.77, 5.42, 5.05 and 4.86 ms
+// with 32, 64, 128, 256 and 512 MiB of them.
+constexpr long long kChunkBytes = 512ll << 20;
 
 // Correlation of every window with every template over all angles (the
 // angle loop of main.cu:1232-1257): per angle the template-pair spectra, then
@@ -1807,7 +1809,7 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
     // windows without a persistent kernel: row and column launches over chunks
     // of units, unless one of the cross-check options asks for the per-window ones
     const bool chunked = !persistent && !ctx->two_pass && !ctx->generic_fft;
-    const int chunk = (int)std::max<long long>(1, std::min<long long>(65535, kChunkBytes / (l2 * (long long)sizeof(float2))));
+    int chunk = (int)std::max<long long>(1, std::min<long long>(65535, kChunkBytes / (l2 * (long long)sizeof(float2))));
     int A = persistent || chunked ? launch_angles(ctx, nu, na, tc2) : 1;
     // pair spectra of the first launch already enqueued on the side stream
     // (prefetch_pair_spectra): used when the group matches, else awaited
@@ -1818,7 +1820,8 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
     }
     CorrTuning tune;
     TRY(default_tuning(ctx, tc2, &tune));
-    // a launch takes fewer angles where the device has no memory for A of them
+    // a launch takes fewer angles, and smaller chunks, where the device has no
+    // memory for them
     // (the frees wait for whatever still uses the buffers)
     auto buffers = [&]() -> int {
         TRY(ensure(ctx, ctx->units, sizeof(UnitOut) * std::max<long long>(1, total_units)));
@@ -1836,8 +1839,8 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         }
         return ensure(ctx, ctx->scratch, sizeof(float2) * l2 * (chunked ? std::min<long long>(chunk, (long long)nu * A) : Np));
     };
-    for (int st; (st = buffers()) != GS_OK; A = (A + 1) / 2) {
-        if (st != GS_ERR_OOM || A == 1) return st;
+    for (int st; (st = buffers()) != GS_OK; A = (A + 1) / 2, chunk = (chunk + 1) / 2) {
+        if (st != GS_ERR_OOM || (A == 1 && !(chunked && chunk > 1))) return st;
         if (prefetched) CK(cudaStreamWaitEvent(ctx->stream, ctx->side_ev[1], 0));
         prefetched = 0;
         for (DBuf* b : {&ctx->tspec, &ctx->pacc, &ctx->dep_counters, &ctx->scratch}) free_buf(*b);

@@ -17,8 +17,8 @@ def _built():
     build.build_library()
 
 
-# 100: many angles in one chunk; 316 = 4 79 (dense prime); 804: two units to spare per chunk; 1084: units of several chunks
-@pytest.mark.parametrize("l,templates", [(100, 3), (252, 4), (316, 3), (804, 5), (1084, 2)])
+# 100: many angles in one chunk; 316 = 4 79 (dense prime); 804 and 1084 with few units; 1084 with eight templates: two chunks
+@pytest.mark.parametrize("l,templates", [(100, 3), (252, 4), (316, 3), (804, 5), (1084, 2), (1084, 8)])
 def test_chunked_windows(l, templates):
     t = 2 * (l // 10)
     d_m = float(int(0.8 * t))
