@@ -483,6 +483,15 @@ __device__ __forceinline__ UnitOut unit_score(const UnitAcc& ac, double s1, int 
 }
 __device__ __forceinline__ UnitOut unit_score(const UnitAcc& ac, int l) { return unit_score(ac, ac.s1, l); }
 
+// Item indices of one persistent launch over n units (2 x l/8 tiles per unit)
+// must fit an int.
+inline bool corr_units_fit(int l, long long n) { return n < (1ll << 31) && (n + 64) * 2 * (l / 8) < (1ll << 31); }
+
+// Whether a claim is one of the launch's `total` items.  Every CTA claims two items
+// past the last one, more in all than the room that corr_units_fit leaves
+// below 2^31 at windows under 160: such a claim is negative, and no item either.
+__host__ __device__ __forceinline__ bool corr_claimed(int item, int total) { return (unsigned)item < (unsigned)total; }
+
 // What a claimed item is.
 struct CorrItem {
     int u, j;  // unit, tile
@@ -490,7 +499,7 @@ struct CorrItem {
 };
 
 template <int T>
-__device__ __forceinline__ CorrItem corr_item(const CorrArgs& a, int item) {
+__host__ __device__ __forceinline__ CorrItem corr_item(const CorrArgs& a, int item) {
     const int head = a.lag * T;
     if (item < head) return CorrItem{item / T, item % T, true};
     const int i = item - head, s = i / (2 * T), j = i - s * (2 * T);
@@ -569,7 +578,7 @@ __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCta
     __syncthreads();
     int item = ish[0];
     int claimed = 0;  // the publisher's claim for slot (iter + 1) & 3, made after the previous barrier
-    for (int iter = 0; item < total; ++iter) {
+    for (int iter = 0; corr_claimed(item, total); ++iter) {
         // the unit's (window, pair) is read-only in this launch: its load is
         // issued before the dependency wait and overlaps it
         const CorrItem it = corr_item<F::T>(a, item);

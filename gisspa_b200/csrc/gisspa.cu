@@ -1583,10 +1583,6 @@ static int autotune(gs_ctx* ctx, const float2* W, const float2* TS, int NW, Corr
     return GS_OK;
 }
 
-// Item indices of one persistent launch over n units (2 x l/8 tiles per
-// unit) must fit an int.
-static bool units_fit(int l, long long n) { return n < (1ll << 31) && (n + 64) * 2 * (l / 8) < (1ll << 31); }
-
 // In-plane angles per persistent launch before any tuning: the option's
 // count, else enough angles for about kUnitsPerLaunch units (a launch's
 // ramp-up and drain, and the per-launch overhead, then weigh little against
@@ -1607,7 +1603,7 @@ static int launch_angles(const gs_ctx* ctx, int nu, int na, bool tc2) {
         A = (int)std::min<double>(A, std::max(1.0, std::floor(kAngleBudget / angle_bytes)));
     }
     A = std::max(1, std::min(A, na));
-    while (A > 1 && !units_fit(l, (long long)A * nu)) --A;
+    while (A > 1 && !corr_units_fit(l, (long long)A * nu)) --A;
     return A;
 }
 
@@ -1642,7 +1638,7 @@ static int search_norm1(gs_ctx* ctx, const float2* W, int nx, int ny, const std:
         TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np));
         return search_norm1_passes(ctx, W, nx, ny, offx, offy, angles, ms_spec, ms_corr, out);
     };
-    if (ctx->two_pass || !ops || !ops->corr_moments || !units_fit(l, nu)) return passes();
+    if (ctx->two_pass || !ops || !ops->corr_moments || !corr_units_fit(l, nu)) return passes();
     // angles per launch as in the norm_type 0 search, with the block maxima and
     // their picks within 2 GiB
     int A = launch_angles(ctx, (int)nu, na, false);
@@ -1735,7 +1731,7 @@ static int prefetch_pair_spectra(gs_ctx* ctx, int NW, const std::vector<float>& 
     if (!persistent || ctx->autotune || p.norm_type == 1 || na == 0 || (tc2 && l != 720)) return GS_OK;
     if (p.precision != GS_PREC_FP32 && !fast_ok(ctx, l)) return GS_OK;  // the correlation refuses it
     const int nu = Np * NW;
-    if (!units_fit(l, nu)) return GS_OK;  // the correlation reports it
+    if (!corr_units_fit(l, nu)) return GS_OK;  // the correlation reports it
     const bool pfa = (p.precision == GS_PREC_FP32 || tc2) && PfaCols::make(l).N2 != 0;
     const int A = launch_angles(ctx, nu, na, tc2);
     // the preparation's and the correlation's own buffers come first where memory is short
@@ -1804,7 +1800,7 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         return set_err(ctx, GS_ERR_UNSUPPORTED,
                        "tensor-core precision needs window 512, 720 or 768 and the persistent path (window %d)", l);
     const int nu = Np * NW;
-    if (!units_fit(l, nu))
+    if (!corr_units_fit(l, nu))
         return set_err(ctx, GS_ERR_UNSUPPORTED, "too many (window, template pair) units in one search (%d)", nu);
     // windows without a persistent kernel: row and column launches over chunks
     // of units, unless one of the cross-check options asks for the per-window ones
