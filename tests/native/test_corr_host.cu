@@ -1,7 +1,10 @@
 // Host parts of gisspa_b200/csrc/corr.cuh.
 //   claims: the items of the largest launch that is allowed, and the claims behind
 //   its last item, at every window
+//   border: the masked indices at every window and particle diameter, to infinity
+#include <cmath>
 #include <cstdio>
+#include <initializer_list>
 #include <string>
 
 #include "corr.cuh"
@@ -43,10 +46,31 @@ static int check_windows() {
     }
 }
 
+static int check_border() {
+    int bad = 0;
+    for (int l = 96; l <= 768; l += 16)
+        for (float d_m : {1e-45f, 0.1f, 4.0f, 47.9f, 48.0f, (float)l, 1.9f * l, 2.0f * l, 2.1f * l, 3.0f * l, 4.0f * l,
+                          5.0f * l, 1e6f, 8.5e9f, 9e9f, 1e20f, 3e38f, INFINITY}) {
+            CorrArgs a{};
+            corr_border(&a, d_m, l);
+            const float q_lo = d_m / 4.0f, q_hi = (float)l - q_lo;
+            for (int x = 0; x < l && !bad; ++x) {
+                const int X = (x + l / 2) % l;
+                const bool want = (float)X < q_lo || (float)X > q_hi;
+                if (((unsigned)(x - a.yb0) <= (unsigned)(a.yb1 - a.yb0)) != want) {
+                    printf("window %d, diameter %g: index %d %smasked\n", l, d_m, x, want ? "not " : "");
+                    bad = 1;
+                }
+            }
+        }
+    return bad;
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     int bad = 1;
     if (what == "claims") bad = check_windows<6>();
+    if (what == "border") bad = check_border();
     printf(bad ? "FAIL\n" : "OK\n");
     return bad;
 }
