@@ -79,14 +79,14 @@ struct CorrArgs {
 
 // Border interval of unshifted indices: X = (x + l/2) mod l is masked when X <
 // d_m/4 or X > l - d_m/4 (GPU_func.cu:681).  Bounds outside the window are brought
-// to its edge before they become integers: any positive d_m, infinity too,
-// masks what it says.
+// to its edge before they become integers, so that any positive d_m masks what
+// it says, one that rounds away and infinity too.
 inline void corr_border(CorrArgs* a, float d_m, int l) {
     const float q_lo = d_m / 4.0f, q_hi = (float)l - q_lo;
     const int h = l / 2;
-    a->yb0 = (int)floorf(fmaxf(q_hi, -1.0f)) - h + 1;
+    a->yb0 = (int)floorf(fminf(fmaxf(q_hi, -1.0f), (float)(l - 1))) - h + 1;
     a->yb1 = (int)ceilf(fminf(q_lo, (float)l)) + h - 1;
-    if (a->yb1 < a->yb0) { a->yb0 = 1; a->yb1 = 0; }
+    if (a->yb1 < a->yb0) a->yb0 = a->yb1 = -1;  // no index
 }
 
 // Lag of the column tiles in units for `ctas` resident CTAs and units of `tiles`

@@ -49,7 +49,7 @@ static int check_windows() {
 static int check_border() {
     int bad = 0;
     for (int l = 96; l <= 768; l += 16)
-        for (float d_m : {1e-45f, 0.1f, 4.0f, 47.9f, 48.0f, (float)l, 1.9f * l, 2.0f * l, 2.1f * l, 3.0f * l, 4.0f * l,
+        for (float d_m : {1e-45f, 1e-20f, 1e-5f, 1e-4f, 0.1f, 4.0f, 47.9f, 48.0f, (float)l, 1.9f * l, 2.0f * l, 2.1f * l, 3.0f * l, 4.0f * l,
                           5.0f * l, 1e6f, 8.5e9f, 9e9f, 1e20f, 3e38f, INFINITY}) {
             CorrArgs a{};
             corr_border(&a, d_m, l);
