@@ -33,7 +33,9 @@
 // later, so the earliest unpublished item can always proceed.  Every wait is
 // bounded; a wait that gives up raises the error flag (reported as
 // GS_ERR_TIMEOUT) and the item still completes and is published, so no other
-// CTA is left waiting on it.
+// CTA is left waiting on it.  Units scored once the flag is up get NaN: those whose
+// maps the wait was for, and the launch's later ones (gs_correlate_window_noalloc
+// does not wait for its launches and has no other way to tell).
 //
 // Memory ordering: producers store the maps bypassing L1 (st.global with an
 // L2 cache hint) and add their accumulator atomics; the CTA barrier that ends
@@ -113,7 +115,10 @@ __device__ __forceinline__ void wait_counter(const int* p, int target, int* erro
         __nanosleep(256);
         ok = ld_acquire_gpu(p) >= target;
     }
-    if (!ok) atomicExch(error, 1);
+    if (!ok) {
+        atomicExch(error, 1);
+        __threadfence();  // the flag before anything the item overwrites too early
+    }
 }
 
 // The calling warp waits until *p >= target: lane 0 spins (bounded, about a
@@ -536,6 +541,8 @@ __device__ __forceinline__ void corr_publish(const CorrArgs& a, const CorrItem& 
     int prev;
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(prev) : "l"(&a.done_cols[u]) : "memory");
     if (prev != F::T - 1) return;
+    const bool gave_up = ld_acquire_gpu(a.error) != 0;
+    const float nan = __int_as_float(0x7fc00000);
     const int2 wp = a.unit_wp[u];
     const UnitAcc* ac = a.acc + 2 * (long long)u;
     // sum of the map c1 + i c2 = L^2 S(0, 0), S = W conj(P)
@@ -552,7 +559,7 @@ __device__ __forceinline__ void corr_publish(const CorrArgs& a, const CorrItem& 
         UnitAcc v;
         v.key = __ldcg(&ac[q].key);
         v.s2 = __ldcg(&ac[q].s2);
-        a.out[o] = unit_score(v, sums[q], F::L);
+        a.out[o] = gave_up ? UnitOut{nan, 0, nan, nan} : unit_score(v, sums[q], F::L);
     }
 }
 
