@@ -99,6 +99,12 @@ __host__ __device__ __forceinline__ int key_index(unsigned long long k) {
     return k ? (int)(~(unsigned)(k & 0xffffffffull)) : 0;
 }
 
+// Order-preserving map of any float to uint32 (negative values too).
+__device__ __forceinline__ unsigned float_order(float v) {
+    const unsigned u = __float_as_uint(v);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
 template <class T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

@@ -308,9 +308,10 @@ __device__ __forceinline__ void corr_moments(const CorrArgs& a, int u, int x, in
 }
 
 // norm_type 1, sweep 2: z-scores against the window's per-pixel (mean, 1 /
-// deviation) and the maximum of every 1024-element block of the flat map
-// (update_CCG + get_peak_pos, GPU_func.cu:648-662, 711-745).  The tile's z go
-// through the tile buffer (l rows of 16, both templates), so that a thread
+// deviation), 0 where that is marked negative (no positive deviation), and the
+// maximum of every 1024-element block of the flat map (update_CCG +
+// get_peak_pos, GPU_func.cu:648-662, 711-745).  The tile's z go through the tile
+// buffer as float_order keys (l rows of 16, both templates), so that a thread
 // takes a whole 16-column run of one row, which lies inside one block (l is a
 // multiple of 32); runs of one block in neighbouring lanes are combined before
 // the one atomic.  One atomic per map value instead cost 173 us per
@@ -318,7 +319,7 @@ __device__ __forceinline__ void corr_moments(const CorrArgs& a, int u, int x, in
 // index to keep both sides free of bank conflicts.
 template <int N2, int V>
 __device__ __forceinline__ void corr_blocks(const CorrArgs& a, int u, int v, int x, int k1, const float2 (&b)[N2],
-                                            float* z) {
+                                            unsigned* z) {
     using F = CorrCfg<N2, V>;
     static_assert(V == 16 && !F::kPfa, "16-column runs in natural order");
     constexpr int L = F::L, h = L / 2;
@@ -333,29 +334,27 @@ __device__ __forceinline__ void corr_blocks(const CorrArgs& a, int u, int v, int
         const int y = k1 + 16 * k2, Y = y + h < L ? y + h : y - h;
         const float2 m = __ldg(mom + (long long)Y * L);
         const float2 c = cscale(b[rf::rpos<N2>(k2)], s);
-        float* o = z + Y * 16 + (((v >> 2) ^ ((Y >> 1) & 3)) << 2) + (v & 3);
-        o[0] = (c.x - m.x) * m.y;
-        o[L * 16] = (c.y - m.x) * m.y;
+        unsigned* o = z + Y * 16 + (((v >> 2) ^ ((Y >> 1) & 3)) << 2) + (v & 3);
+        o[0] = float_order(m.y >= 0.0f ? (c.x - m.x) * m.y : 0.0f);
+        o[L * 16] = float_order(m.y >= 0.0f ? (c.y - m.x) * m.y : 0.0f);
     });
     __syncthreads();
     const int X0 = X & ~15;  // V = 16: the tile's columns start at a multiple of 16
     for (int r = threadIdx.x; r < 2 * L; r += F::kThreads) {  // L is a multiple of 32: no partial warps
         const int q = r >= L, Y = q ? r - L : r, J = 2 * p + q;
-        const float4* row = reinterpret_cast<const float4*>(z + (q * L + Y) * 16);
-        float best = __int_as_float(0xff800000);  // -inf
+        const uint4* row = reinterpret_cast<const uint4*>(z + (q * L + Y) * 16);
+        unsigned best = 0u;
         int at = 0;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const float4 w = row[c ^ ((Y >> 1) & 3)];
+            const uint4 w = row[c ^ ((Y >> 1) & 3)];
             if (w.x > best) { best = w.x; at = 4 * c; }
             if (w.y > best) { best = w.y; at = 4 * c + 1; }
             if (w.z > best) { best = w.z; at = 4 * c + 2; }
             if (w.w > best) { best = w.w; at = 4 * c + 3; }
         }
         const int pos = Y * L + X0 + at, blk = (Y * L + X0) >> 10;
-        const unsigned bits = __float_as_uint(best);
-        unsigned long long key =
-            ((unsigned long long)((bits & 0x80000000u) ? ~bits : bits | 0x80000000u) << 32) | (unsigned)~pos;
+        unsigned long long key = ((unsigned long long)best << 32) | (unsigned)~pos;
         // rows of one block sit in neighbouring lanes (a warp holds rows of one template)
 #pragma unroll
         for (int o = 1; o < 32; o *= 2) {
@@ -416,7 +415,7 @@ __device__ __forceinline__ void corr_col_tile(const CorrArgs& a, int u, int t, f
         for (int n2 = 0; n2 < N2; ++n2) b[n2] = src[n2];
         rf::rfft<N2, 1, true>(b);
         if constexpr (kEpi == kCorrMoments) corr_moments<N2, V>(a, u, x, k1, b);
-        else corr_blocks<N2, V>(a, u, v, x, k1, b, reinterpret_cast<float*>(tile));
+        else corr_blocks<N2, V>(a, u, v, x, k1, b, reinterpret_cast<unsigned*>(tile));
         return;
     }
     constexpr float sgn = ((L / 2) % 2 == 0) ? 1.0f : -1.0f;

@@ -20,11 +20,7 @@
 
 namespace gs {
 
-// Order-preserving map of any finite float to uint32 (negative values too).
-__device__ __forceinline__ unsigned int float_order(float v) {
-    const unsigned int u = __float_as_uint(v);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
+// The float of an order-preserving float_order key.
 __host__ __device__ __forceinline__ float float_unorder(unsigned int m) {
     const unsigned int u = (m & 0x80000000u) ? (m & 0x7fffffffu) : ~m;
 #ifdef __CUDA_ARCH__
@@ -115,15 +111,16 @@ __global__ void k_norm1_moments(float* s1, float* s2, long long n, float total) 
     s2[i] = var;
 }
 
-// The same for the persistent kernel's interleaved sums: (mean, 1 / standard
-// deviation), 0 where the deviation is not positive (z = 0 there).
+// The same for the persistent kernel's interleaved sums: (mean, 1 / deviation), 0
+// for an infinite deviation, -1 where the deviation is not
+// positive (z = 0 there).
 __global__ void k_norm1_moments2(float2* mom, long long n, float total) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float2 s = mom[i];
     const float avg = s.x / total;
     const float sd = sqrtf(s.y / total - avg * avg);
-    mom[i] = make_float2(avg, sd > 0.0f ? 1.0f / sd : 0.0f);
+    mom[i] = make_float2(avg, sd > 0.0f ? 1.0f / sd : -1.0f);
 }
 
 struct BlockPickDev {
