@@ -310,12 +310,15 @@ __device__ __forceinline__ void corr_moments(const CorrArgs& a, int u, int x, in
 // norm_type 1, sweep 2: z-scores against the window's per-pixel (mean, 1 /
 // deviation), 0 where that is marked negative (no positive deviation), and the
 // maximum of every 1024-element block of the flat map (update_CCG +
-// get_peak_pos, GPU_func.cu:648-662, 711-745).  The tile's z go through the tile
-// buffer as float_order keys (l rows of 16, both templates), so that a thread
-// takes a whole 16-column run of one row, which lies inside one block (l is a
-// multiple of 32); runs of one block in neighbouring lanes are combined before
-// the one atomic.  One atomic per map value instead cost 173 us per
-// 12 pairs at window 512.  The 16-byte pieces of a row are rotated by its
+// get_peak_pos, GPU_func.cu:648-662, 711-745).  The product rounds as the
+// reference's division does: 1 / deviation is rounded once, from double, where the
+// deviation was (dividing instead took norm_type 1 at window 512 from 6.2 to
+// 8.0 ms); the rounding of 1 / l^2 is in the maps of both sweeps and cancels.
+// The tile's z go through the tile buffer as float_order keys (l rows of 16, both
+// templates), so that a thread takes a whole 16-column run of one row, which lies
+// inside one block (l is a multiple of 32); runs of one block in neighbouring lanes
+// are combined before the one atomic.  One atomic per map value instead cost 173
+// us per 12 pairs at window 512.  The 16-byte pieces of a row are rotated by its
 // index to keep both sides free of bank conflicts.
 template <int N2, int V>
 __device__ __forceinline__ void corr_blocks(const CorrArgs& a, int u, int v, int x, int k1, const float2 (&b)[N2],

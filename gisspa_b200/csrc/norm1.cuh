@@ -111,16 +111,16 @@ __global__ void k_norm1_moments(float* s1, float* s2, long long n, float total) 
     s2[i] = var;
 }
 
-// The same for the persistent kernel's interleaved sums: (mean, 1 / deviation), 0
-// for an infinite deviation, -1 where the deviation is not
+// The same for the persistent kernel's interleaved sums: (mean, 1 / deviation), the
+// latter rounded once, 0 for an infinite deviation, -1 where the deviation is not
 // positive (z = 0 there).
 __global__ void k_norm1_moments2(float2* mom, long long n, float total) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float2 s = mom[i];
     const float avg = s.x / total;
-    const float sd = sqrtf(s.y / total - avg * avg);
-    mom[i] = make_float2(avg, sd > 0.0f ? 1.0f / sd : -1.0f);
+    const float var = s.y / total - avg * avg;
+    mom[i] = make_float2(avg, var > 0.0f ? (float)(1.0 / sqrt((double)var)) : -1.0f);
 }
 
 struct BlockPickDev {

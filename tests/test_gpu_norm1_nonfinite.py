@@ -1,11 +1,16 @@
 """norm_type 1 on maps that are not finite, zero or overflow their squares:
 the persistent kernel's block maxima and picks are those of the per-window
 passes (z = 0 where the deviation is not positive)."""
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
 import gisspa_b200 as G
 from gisspa_b200 import synth
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +58,14 @@ def test_norm1_not_finite(l, what):
     assert len(want) > 100
     for c in ("angle_index", "window_x", "window_y", "template_index", "center_x", "center_y", "score"):
         assert np.array_equal(want[c], have[c]), c
+
+
+def test_reciprocal_deviation(tmp_path):
+    """tests/native/test_norm1_moments.cu"""
+    exe = str(tmp_path / "test_norm1_moments")
+    subprocess.run(["nvcc", "-std=c++17", "-O2", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
+                    "-I" + os.path.join(ROOT, "gisspa_b200", "csrc"), "-o", exe,
+                    os.path.join(ROOT, "tests", "native", "test_norm1_moments.cu")], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert "OK" in r.stdout
