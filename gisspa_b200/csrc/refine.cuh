@@ -53,9 +53,9 @@ struct RefineConsts {
 };
 
 // What the weight takes of a bin that does not depend on the pick: band-pass
-// factor (negative: bin not selected, the weight is its magnitude alone), s^2 and
-// azimuth of the CTF's folded frequency, noise curve over signal.  One table per
-// call, read by every pick.
+// factor, s^2 and azimuth of the CTF's folded frequency, noise curve over signal
+// (negative: bin not selected, the weight is the band-pass factor alone).  One
+// table per call, read by every pick.
 struct RefineBin {
     float band, ss, ag, ncurve;
 };
@@ -65,7 +65,7 @@ __device__ __forceinline__ RefineBin refine_bin(int x, int y, const RefineConsts
     float rf;
     const int r = shell_index(x, y, l, l, &rf);
     const float band = bandpass<false>(r, rc.hp, rc.lp);
-    if (!(r < l / 2 && r >= 0)) return RefineBin{-band - 1.0f, 0.0f, 0.0f, 1.0f};
+    if (!(r < l / 2 && r >= 0)) return RefineBin{band, 0.0f, 0.0f, -1.0f};
     // CTF geometry of ctf_ast(x, (y + l/2) % l)
     int x1 = x, y1 = (y + l / 2) % l;
     y1 = x1 > l / 2 ? l - y1 : y1;
@@ -83,9 +83,9 @@ __device__ __forceinline__ RefineBin refine_bin(int x, int y, const RefineConsts
 template <bool kGrad>
 __device__ __forceinline__ float refine_weight(const RefineBin& bin, const RefineConsts& rc, const RefinePickDev& pk,
                                                bool* insel, float dw[3]) {
-    *insel = bin.band >= 0.0f;
+    *insel = !(bin.ncurve < 0.0f);
     if constexpr (kGrad) dw[0] = dw[1] = dw[2] = 0.0f;
-    if (!*insel) return -bin.band - 1.0f;
+    if (!*insel) return bin.band;
     const float ss = bin.ss;
     const float D = -pk.defocus;
     const float dfu = D + pk.dfdiff, dfv = D - pk.dfdiff;
