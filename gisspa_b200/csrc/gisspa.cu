@@ -717,7 +717,7 @@ static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool
     const int chunk = (int)std::max<long long>(1, std::min<long long>(std::min(n, 65535), (2ll << 30) / per));
     TRY(ensure(ctx, ctx->rf_pk, sizeof(RefinePickDev) * chunk));
     TRY(ensure(ctx, ctx->rf_acc, sizeof(RefineAcc) * chunk));
-    TRY(ensure(ctx, ctx->rf_scale, (sizeof(double) * 2 + sizeof(float4) * 2) * chunk));
+    TRY(ensure(ctx, ctx->rf_scale, (sizeof(double) * 2 + sizeof(float4)) * chunk));
     TRY(ensure(ctx, ctx->rf_ph, sizeof(double2) * 2 * l * chunk));
     TRY(ensure(ctx, ctx->rf_F1, sizeof(float2) * l2 * chunk));
     TRY(ensure(ctx, ctx->rf_T, sizeof(float) * l2 * chunk));
@@ -758,8 +758,8 @@ static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool
     const float sgn = ((l / 2) % 2 == 0) ? 1.0f : -1.0f;
     RefinePickDev* d_pk = P<RefinePickDev>(ctx->rf_pk);
     RefineAcc* d_acc = P<RefineAcc>(ctx->rf_acc);
-    float4* coef = P<float4>(ctx->rf_scale);                          // 1 / sd, then 1
-    double* inva = reinterpret_cast<double*>(coef + 2 * chunk);
+    float4* as_is = P<float4>(ctx->rf_scale);
+    double* inva = reinterpret_cast<double*>(as_is + chunk);
     double* scale = inva + chunk;                                     // 1 / l^2
     double2* phases = P<double2>(ctx->rf_ph);
     float2* F1 = P<float2>(ctx->rf_F1);
@@ -788,8 +788,8 @@ static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool
         TRY(run_fft<true>(ctx, l, rows_of(l, l), nc, IoScaleIn{data, factor}));
         return run_fft<true>(ctx, l, cols_of(l, l), nc, IoRealOut{data, out, 1.0f});
     };
-    auto forward_disc = [&](float2* data, const float4* cf, float factor, float dc, int nc) -> int {
-        return disc_transform(ctx, data, cf, nc, mr, factor, dc, false);
+    auto forward_disc = [&](float2* data, float factor, float dc, int nc) -> int {
+        return disc_transform(ctx, data, as_is, nc, mr, factor, dc, false);
     };
     std::vector<RefinePickDev> hp(chunk);
     std::vector<RefineAcc> ha(chunk);
@@ -811,11 +811,11 @@ static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool
         // forward
         k_ref_phases<<<dim3(blocks_for(2 * l, 128), nc), 128, 0, ctx->stream>>>(d_pk, l, phases);
         k_ref_weight<<<g, 256, 0, ctx->stream>>>(base, bins, F1, Gm, d_pk, rc, d_acc);
-        k_ref_inva<<<blocks_for(nc, 128), 128, 0, ctx->stream>>>(d_acc, nc, (double)rc.cnt, inva);
+        k_ref_factors<<<blocks_for(nc, 128), 128, 0, ctx->stream>>>(d_acc, nc, (double)rc.cnt, inva, as_is);
         TRY(inverse_real(Gm, inva, T, nc));
-        k_ref_rotate<<<gd, 256, 0, ctx->stream>>>(T, TM, F, d_pk, rc, mr.row0, mr.row1, mask, d_acc);
-        k_ref_coef<<<blocks_for(nc, 128), 128, 0, ctx->stream>>>(d_acc, nc, (double)l2, coef);
-        TRY(forward_disc(F, coef, inv_l2, 0.0f, nc));
+        k_ref_rotate<<<gd, 256, 0, ctx->stream>>>(T, TM, d_pk, rc, mr.row0, mr.row1, mask, d_acc);
+        k_ref_norm<<<gd, 256, 0, ctx->stream>>>(TM, rc, mr.row0, mr.row1, d_acc, F);
+        TRY(forward_disc(F, inv_l2, 0.0f, nc));
         k_ref_score<<<g, 256, 0, ctx->stream>>>(W, F, d_pk, phases, rc, d_acc);
         ctx->counters.kernel_launches += 6;
         CKL();
@@ -827,7 +827,7 @@ static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool
                                  sizeof(float2) * (size_t)(mr.row1 - mr.row0) * l, nc, ctx->stream));
             k_ref_rot_adj<<<gd, 256, 0, ctx->stream>>>(TB, TM, T, d_pk, rc, mr.row0, mr.row1, mask, d_acc, Gm);
             // Fbar2 = FFT(tbar)
-            TRY(forward_disc(Gm, coef + nc, 1.0f, 1.0f, nc));
+            TRY(forward_disc(Gm, 1.0f, 1.0f, nc));
             k_ref_abar<<<g, 256, 0, ctx->stream>>>(Gm, F1, rc, d_acc);
             k_ref_theta<<<g, 256, 0, ctx->stream>>>(Gm, F1, base, bins, d_pk, rc, tgrad != nullptr, d_acc);
             ctx->counters.kernel_launches += 5;

@@ -16,9 +16,9 @@
 //   c   = Re sum_k W(k) conj(F(k)) exp(2 pi i k.(x0 + d) / l), k signed
 //   sig = sqrt(sum_k |W|^2 |F|^2)        map standard deviation (Parseval)
 //   s   = sgn c / sig
-// The adjoint runs the same chain backwards; it recomputes nothing it can
-// keep from the forward of the same call (the per-pick buffers B, F1, tn and
-// F stay in device memory for the backward) and stores no map.
+// The adjoint runs the same chain backwards; the forward's per-pick buffers (F1, t,
+// tm and F) stay in device memory for it, tn is taken from tm again, and B is
+// read from the context's half planes.
 #pragma once
 
 #include "common.cuh"
@@ -167,11 +167,14 @@ static __global__ void __launch_bounds__(256) k_ref_weight(const float2* __restr
     if (threadIdx.x == 0) atomicAdd(&acc[p].asum, v1[0]);
 }
 
-// Per-pick factors of the transforms: 1 / a for t = Re IFFT(F1 / a); after the
-// rotation, (1 / sd of tm) as a pair coefficient.
-static __global__ void k_ref_inva(const RefineAcc* __restrict__ acc, int n, double cnt, double* __restrict__ inva) {
+// Per-pick factors of the transforms: 1 / a for t = Re IFFT(F1 / a), and the pair
+// coefficient (IoPairNorm) of a map that is to be taken as it is.
+static __global__ void k_ref_factors(const RefineAcc* __restrict__ acc, int n, double cnt, double* __restrict__ inva,
+                                     float4* __restrict__ as_is) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n) inva[p] = cnt / sqrt(acc[p].asum);
+    if (p >= n) return;
+    inva[p] = cnt / sqrt(acc[p].asum);
+    as_is[p] = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
 }
 
 // Source coordinates of rotate_subIMG for output pixel (i, j) and angle e.
@@ -211,11 +214,11 @@ __device__ __forceinline__ Bilin bilin(float x2, float y2, int l) {
     return b;
 }
 
-// tm = mask . rotate(t, e), real and as the input of its transform, in the rows
-// [row0, row1) that the mask's disc reaches; sums of tm and tm^2.
+// tm = mask . rotate(t, e) in the rows [row0, row1) that the mask's disc reaches;
+// sums of tm and tm^2.
 static __global__ void __launch_bounds__(256) k_ref_rotate(const float* __restrict__ T, float* __restrict__ TM,
-                                                           float2* __restrict__ F, const RefinePickDev* __restrict__ pks,
-                                                           RefineConsts rc, int row0, int row1,
+                                                           const RefinePickDev* __restrict__ pks, RefineConsts rc,
+                                                           int row0, int row1,
                                                            const float* __restrict__ mask, RefineAcc* __restrict__ acc) {
     __shared__ double red[64];
     const int p = blockIdx.y;
@@ -236,7 +239,6 @@ static __global__ void __launch_bounds__(256) k_ref_rotate(const float* __restri
             v *= m;
         }
         TM[p * rc.L2 + i] = v;
-        F[p * rc.L2 + i] = make_float2(v, 0.0f);
         a2[0] += v;
         a2[1] += (double)v * v;
     }
@@ -253,15 +255,16 @@ __device__ __forceinline__ void ref_moments(const RefineAcc& a, double L2, doubl
     *sd = sqrt(var > 0.0 ? var : 1.0);
 }
 
-// coef[p]: tm's 1 / sd as IoPairNorm takes it (the mean only reaches the zero
-// frequency of FFT(tn), which is 0); coef[n + p]: no scaling.
-static __global__ void k_ref_coef(const RefineAcc* __restrict__ acc, int n, double L2, float4* __restrict__ coef) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
+// The input of FFT(tn): tm / sd in the rows [row0, row1), rounded once from double
+// (the mean only reaches the zero frequency, which is 0).
+static __global__ void __launch_bounds__(256) k_ref_norm(const float* __restrict__ TM, RefineConsts rc, int row0, int row1,
+                                                         const RefineAcc* __restrict__ acc, float2* __restrict__ F) {
+    const int p = blockIdx.y;
     double mu, sd;
-    ref_moments(acc[p], L2, &mu, &sd);
-    coef[p] = make_float4(0.0f, (float)(1.0 / sd), 0.0f, 0.0f);
-    coef[n + p] = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
+    ref_moments(acc[p], (double)rc.L2, &mu, &sd);
+    const double inv_sd = 1.0 / sd;
+    for (int i = row0 * rc.l + blockIdx.x * blockDim.x + threadIdx.x; i < row1 * rc.l; i += gridDim.x * blockDim.x)
+        F[p * rc.L2 + i] = make_float2((float)((double)TM[p * rc.L2 + i] * inv_sd), 0.0f);
 }
 
 // Phase factors exp(2 pi i kx (x0 + dx) / l), kx = 0 .. l - 1 (signed), then the

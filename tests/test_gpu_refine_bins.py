@@ -1,4 +1,5 @@
-"""Bins of the refinement's weight (tests/native/test_refine_bins.cu)."""
+"""Element kernels of the refinement: the bins of its weight and the normalised
+template (tests/native/test_refine_*.cu)."""
 import os
 import subprocess
 
@@ -9,11 +10,12 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 pytestmark = pytest.mark.gpu
 
 
-def test_refinement_bins(tmp_path):
-    exe = str(tmp_path / "test_refine_bins")
+@pytest.mark.parametrize("name", ["test_refine_bins", "test_refine_norm"])
+def test_refinement_kernels(tmp_path, name):
+    exe = str(tmp_path / name)
     subprocess.run(["nvcc", "-std=c++17", "-O2", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
                     "-I" + os.path.join(ROOT, "gisspa_b200", "csrc"), "-o", exe,
-                    os.path.join(ROOT, "tests", "native", "test_refine_bins.cu")], check=True)
+                    os.path.join(ROOT, "tests", "native", name + ".cu")], check=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
     assert "OK" in r.stdout
