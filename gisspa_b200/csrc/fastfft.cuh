@@ -11,8 +11,11 @@
 // per transform, and the shared layout (block pitch BP odd, vector pitch
 // 16 BP + 1) makes both the step-1 writes and the step-2 reads of a
 // half-warp hit distinct banks.  All twiddles inside the register DFTs are
-// compile-time constants (regfft.cuh); the W_l^{n2 k1} twiddles are built
-// from one table entry per thread by at most three complex products.
+// compile-time constants (regfft.cuh).  The W_l^{n2 k1} are entries of the
+// twiddle table, put in shared memory by [k1][n2] once per CTA: products of entries,
+// up to three deep, made twice the transform's rounding error of it (window 320
+// 2.0e-7 against 0.94e-7 rms, 512 2.2e-7 against 1.0e-7; the mixed-radix kernel
+// 0.98e-7 and 1.0e-7) for under 1 % of a search's time.
 #pragma once
 
 #include <type_traits>
@@ -31,25 +34,9 @@ struct Fast16 {
     static constexpr int VP = 16 * BP + 1;             // vector pitch
     static constexpr int kThreads = 256;
     static constexpr size_t smem_bytes() {
-        return (size_t)V * VP * sizeof(float2) + kFftRedDoubles * sizeof(double);
+        return (size_t)(V * VP + L) * sizeof(float2) + kFftRedDoubles * sizeof(double);
     }
 };
-
-// W_l^{n2 k1} for k1 = 0..15 from w1 = W_l^{n2}: w2 = w1^2, w4 = w2^2,
-// w8 = w4^2 and w_k = products of those (at most three products deep).
-__device__ __forceinline__ void twiddle16(float2 w1, float2 (&w)[16]) {
-    w[0] = make_float2(1.0f, 0.0f);
-    w[1] = w1;
-    w[2] = cmul(w1, w1);
-    w[3] = cmul(w[2], w1);
-    w[4] = cmul(w[2], w[2]);
-    w[5] = cmul(w[4], w1);
-    w[6] = cmul(w[4], w[2]);
-    w[7] = cmul(w[4], w[3]);
-    w[8] = cmul(w[4], w[4]);
-#pragma unroll
-    for (int k = 9; k < 16; ++k) w[k] = cmul(w[8], w[k - 8]);
-}
 
 // IO functors with `static constexpr bool kStaged = true` store a row
 // transform's outputs in their own column order (column(k) for output k)
@@ -66,6 +53,12 @@ __global__ void __launch_bounds__(256, 2) k_fft16(const float2* __restrict__ tw,
     IO io = io_param;
     const int img = blockIdx.y;
     const int v0 = blockIdx.x * F::V;
+    float2* twt = sm16 + F::V * F::VP;  // W_l^{n2 k1} at k1 N2 + n2
+    for (int i = threadIdx.x; i < F::L; i += F::kThreads) {
+        const int k1 = i / N2, n2 = i - k1 * N2;
+        twt[i] = twiddle(tw, n2 * k1, kInv);
+    }
+    __syncthreads();
     // ---- step 1: 16-point DFTs down the stride-N2 columns of each vector
     for (int task = threadIdx.x; task < F::V * N2; task += F::kThreads) {
         int v, n2;
@@ -75,13 +68,11 @@ __global__ void __launch_bounds__(256, 2) k_fft16(const float2* __restrict__ tw,
 #pragma unroll
         for (int n1 = 0; n1 < 16; ++n1) a[n1] = io.load(img, v0 + v, N2 * n1 + n2);
         rf::rfft<16, 1, kInv>(a);
-        float2 w[16];
-        twiddle16(twiddle(tw, n2, kInv), w);
         float2* dst = sm16 + v * F::VP + n2;
         rf::static_for<16>([&](auto kc) {
             constexpr int k1 = decltype(kc)::value;
             constexpr int r = rf::rpos<16>(k1);
-            dst[k1 * F::BP] = k1 ? cmul(a[r], w[k1]) : a[r];
+            dst[k1 * F::BP] = k1 ? cmul(a[r], twt[k1 * N2 + n2]) : a[r];
         });
     }
     __syncthreads();
@@ -117,7 +108,7 @@ __global__ void __launch_bounds__(256, 2) k_fft16(const float2* __restrict__ tw,
             io.store_at(img, v0 + vv, p, sm16[vv * F::VP + p]);
         }
     }
-    io.finish(reinterpret_cast<double*>(sm16 + F::V * F::VP));
+    io.finish(reinterpret_cast<double*>(sm16 + F::V * F::VP + F::L));
 }
 
 // ---- IO functors: (img, v, k) -> element k of vector v of image img ----
