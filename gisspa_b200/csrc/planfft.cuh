@@ -118,8 +118,7 @@ inline bool plan_strides_fit(const PlanDesc& d, const VecGeom& g, int tile) {
 
 // One stage: per vector `d_count.d` butterflies of radix R; butterfly j starts at
 // (j / split) pa + j % split and steps by `stride`.  kTw: output q is multiplied
-// by W_n^{q e}, e = tw_mul * (tw_low ? j % split : j) (twiddles from at most
-// two table entries each: W^{q & 3} and W^{q & ~3}).
+// by W_n^{q e}, e = tw_mul * (tw_low ? j % split : j), a table entry each.
 struct PlanStage {
     SmallDiv count, split;
     int pa, pb, stride, tw_mul;
@@ -139,23 +138,10 @@ __device__ __forceinline__ void plan_stage(float2* buf, int nv, int VP, const Pl
         if constexpr (R > 1) rf::rfft<R, 1, kInv>(a);
         if constexpr (kTw) {
             const int e = s.tw_mul * (s.tw_low ? lo : j);
-            float2 w[4];  // W^0..W^3
-#pragma unroll
-            for (int q = 1; q < 4 && q < R; ++q) w[q] = twiddle(tw, q * e, kInv);
-            rf::static_for<(R + 3) / 4>([&](auto hc) {
-                constexpr int h = 4 * decltype(hc)::value;
-                float2 wh = make_float2(1.0f, 0.0f);
-                if constexpr (h > 0) wh = twiddle(tw, h * e, kInv);
-                rf::static_for<4>([&](auto lc) {
-                    constexpr int q = h + decltype(lc)::value;
-                    if constexpr (q < R) {
-                        constexpr int r = rf::rpos<R>(q);
-                        if constexpr (q == 0) p[0] = a[r];
-                        else if constexpr (q == h) p[q * s.stride] = cmul(a[r], wh);
-                        else if constexpr (h == 0) p[q * s.stride] = cmul(a[r], w[q]);
-                        else p[q * s.stride] = cmul(a[r], cmul(wh, w[q - h]));
-                    }
-                });
+            rf::static_for<R>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                constexpr int r = rf::rpos<R>(q);
+                p[q * s.stride] = q ? cmul(a[r], twiddle(tw, q * e, kInv)) : a[r];
             });
         } else {
             rf::static_for<R>([&](auto qc) {

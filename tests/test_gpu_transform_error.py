@@ -9,7 +9,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("name", ["test_fft16_error"])
+@pytest.mark.parametrize("name", ["test_fft16_error", "test_plan_twiddles"])
 def test_transform_error(tmp_path, name):
     exe = str(tmp_path / name)
     subprocess.run(["nvcc", "-std=c++17", "-O2", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
