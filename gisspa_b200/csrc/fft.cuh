@@ -232,6 +232,11 @@ __global__ void __launch_bounds__(256) fft_batched_kernel(FftDesc P, VecGeom g, 
 // Shared memory of fft_batched_kernel: two ping-pong buffers of tile x (n+1)
 // complex values, then kFftRedDoubles doubles of reduction scratch for finish().
 constexpr int kFftRedDoubles = 128;
+// Limit of dynamic shared memory of the kernels whose launches take different
+// amounts, all that a CTA can have.  It belongs to the kernel, not to a
+// launch: with the launch's own amount a second host thread could lower it
+// between another one's setting it and launching.
+constexpr size_t kMaxSmem = 227 * 1024;
 __host__ __device__ inline size_t fft_smem_bytes(int n, int tile) {
     return 2 * (size_t)tile * (n + 1) * sizeof(float2) + kFftRedDoubles * sizeof(double);
 }

@@ -241,7 +241,6 @@ int get_plan(gs_ctx* ctx, int n, FftPlan** out) {
 
 constexpr int kFftThreads = 256;
 constexpr size_t kFftSmemBudget = 96 * 1024;
-constexpr size_t kMaxSmem = 227 * 1024;
 
 // Vectors per CTA of the in-place kernel: three CTAs to an SM where that takes
 // 16 vectors, down to four (a 32-byte sector of neighbouring columns) with
@@ -269,7 +268,7 @@ int run_fft(gs_ctx* ctx, int n, VecGeom g, int nimg, IO io, int max_tile = 16) {
             plan_layout(&d, tile);
             const size_t smem = plan_smem_bytes(d, tile);
             auto kern = fft_plan_kernel<kInv, IO>;
-            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
             kern<<<dim3((unsigned)((g.nvec + tile - 1) / tile), (unsigned)nimg), kFftThreads, smem, ctx->stream>>>(
                 d, g, tile, io);
             ++ctx->counters.kernel_launches;
@@ -286,7 +285,7 @@ int run_fft(gs_ctx* ctx, int n, VecGeom g, int nimg, IO io, int max_tile = 16) {
     if (smem > kMaxSmem) return set_err(ctx, GS_ERR_UNSUPPORTED, "FFT length %d exceeds shared memory", n);
     if (nimg > 65535) return set_err(ctx, GS_ERR_UNSUPPORTED, "too many images in one FFT batch (%d)", nimg);
     auto kern = fft_batched_kernel<kInv, IO>;
-    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
     dim3 grid((unsigned)((g.nvec + tile - 1) / tile), (unsigned)nimg);
     kern<<<grid, kFftThreads, smem, ctx->stream>>>(pl->d, g, (int)tile, io);
     ++ctx->counters.kernel_launches;
@@ -1131,7 +1130,7 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
             }
             const size_t shs = (size_t)ns * (sizeof(double) + sizeof(unsigned));
             if (shs > kMaxSmem) { st = set_err(ctx, GS_ERR_UNSUPPORTED, "window too large"); break; }
-            cudaFuncSetAttribute(k_tmpl_shells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shs);
+            cudaFuncSetAttribute(k_tmpl_shells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
             k_tmpl_shells<<<dim3(blocks_for((long long)l2 / 2, 2048, 32), nc), 256, shs, ctx->stream>>>(
                 P<float2>(F), l, shells, shell_count);
             k_tmpl_shell_rms<<<blocks_for((long long)nc * ns, 256), 256, 0, ctx->stream>>>(shells, shell_count, ns, nc,
@@ -1312,7 +1311,7 @@ static int prep_micrograph(gs_ctx* ctx, const MicPlan& mp, int index, float2* W)
         CK(cudaMemsetAsync(ctx->rb.p, 0, sizeof(unsigned) * ns, ctx->stream));
         const size_t shs = (size_t)ns * (sizeof(double) + sizeof(unsigned));
         if (shs > kMaxSmem) return set_err(ctx, GS_ERR_UNSUPPORTED, "micrograph too large for the shell histogram");
-        CK(cudaFuncSetAttribute(k_mic_flip_shells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shs));
+        CK(cudaFuncSetAttribute(k_mic_flip_shells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
         const unsigned nb = (unsigned)std::min(ny, 296);
         k_mic_flip_shells<<<nb, 256, shs, ctx->stream>>>(C, nx, ny, cm, P<double>(ctx->ra), P<unsigned>(ctx->rb));
         ++ctx->counters.kernel_launches;

@@ -180,7 +180,7 @@ cudaError_t launch_plan(PlanDesc d, VecGeom g, int nimg, IO io, cudaStream_t st,
         const size_t smem = plan_smem_bytes(d, tile);
         if (smem > (tile > 4 ? 72u << 10 : 220u << 10) || !plan_strides_fit(d, g, tile)) continue;
         auto kern = fft_plan_kernel<kInv, IO>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
         if (e != cudaSuccess) return e;
         kern<<<dim3((unsigned)((g.nvec + tile - 1) / tile), nimg), 256, smem, st>>>(d, g, tile, io);
         *done = true;
@@ -196,9 +196,9 @@ cudaError_t launch_generic(const FftDesc& d, VecGeom g, int nimg, IO io, cudaStr
     tile = std::min<size_t>(tile, 16);
     tile = std::min<size_t>(tile, (size_t)g.nvec);
     const size_t smem = fft_smem_bytes(d.n, (int)tile);
-    if (smem > (227u << 10)) return cudaErrorInvalidValue;
+    if (smem > kMaxSmem) return cudaErrorInvalidValue;
     auto kern = fft_batched_kernel<kInv, IO>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
     if (e != cudaSuccess) return e;
     kern<<<dim3((unsigned)((g.nvec + tile - 1) / tile), nimg), 256, smem, st>>>(d, g, (int)tile, io);
     return cudaGetLastError();
@@ -220,7 +220,7 @@ extern "C" int gs_correlate_window_noalloc(const float* d_window_spectrum, const
     if (desc.nst > kFftMaxStages) return GS_ERR_UNSUPPORTED;
     const int n2 = l / 16;
     const bool fast = l == 512 || l == 720 || l == 768;
-    if (!fast && 2 * (size_t)(l + 1) * sizeof(float2) + kFftRedDoubles * sizeof(double) > (227u << 10))
+    if (!fast && 2 * (size_t)(l + 1) * sizeof(float2) + kFftRedDoubles * sizeof(double) > kMaxSmem)
         return GS_ERR_UNSUPPORTED;
     unsigned char* base = nullptr;
     int st = scratch_for_current_device(&base);
