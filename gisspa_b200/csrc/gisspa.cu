@@ -192,6 +192,29 @@ void free_buf(DBuf& b) {
     b.cap = 0;
 }
 
+// Gives back what a call allocates anew and no later one reads: pair spectra, maps
+// and accumulators of a search's launches, work buffers of the template
+// preparation, of the refinement and of the per-pixel maximum.
+void free_work(gs_ctx* ctx) {
+    for (cudaStream_t s : {ctx->stream, ctx->side, ctx->copy}) cudaStreamSynchronize(s);
+    for (DBuf* b : {&ctx->tspec, &ctx->scratch, &ctx->pacc, &ctx->dep_counters, &ctx->unit_wp, &ctx->picks,
+                    &ctx->tc2_w16, &ctx->tc2_p16, &ctx->tp_raw, &ctx->tp_div, &ctx->tp_sums, &ctx->tp_wmap, &ctx->rf_F1,
+                    &ctx->rf_T, &ctx->rf_TM, &ctx->rf_F, &ctx->rf_G, &ctx->rf_TB, &ctx->rf_ph, &ctx->pix_keys,
+                    &ctx->pix_R})
+        free_buf(*b);
+}
+
+// Runs a call's work, and once more on a context without its work buffers where the
+// first time found no memory: the spectra of many angles that one search takes
+// ahead, or leaves, may be all that the next one's micrograph needs.
+template <class F>
+int with_room(gs_ctx* ctx, F work) {
+    const int st = work(false);
+    if (st != GS_ERR_OOM) return st;
+    free_work(ctx);
+    return work(true);
+}
+
 // Radix order: 8s while they divide, then 4, 2, 3, 5, then any other prime.
 int factorize(int n, int* radix) {
     int ns = 0;
@@ -1051,19 +1074,9 @@ static int validate_params(gs_ctx* ctx, const gs_params* p) {
     return GS_OK;
 }
 
-int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_templates, int n, int tx, int ty,
-                     const gs_ctf* first_ctf) {
-    if (!ctx || !p || !host_templates || !first_ctf || n <= 0 || tx <= 0 || ty <= 0)
-        return set_err(ctx, GS_ERR_ARG, "null pointer or empty template stack");
-    TRY(validate_params(ctx, p));
-    if (n > 2 * 65535) return set_err(ctx, GS_ERR_UNSUPPORTED, "at most %d templates", 2 * 65535);
-    CK(cudaSetDevice(ctx->device));
-    const int l = adjust_padding(p->window_size, tx, ty);
-    if (l % 2) return set_err(ctx, GS_ERR_UNSUPPORTED, "window size %d must be even", l);
-    // norm_type 1 reduces 1024-element blocks of the flat l x l map
-    // (GPU_func.cu:711-745 with the launch at main.cu:798)
-    if (p->norm_type == 1 && ((long long)l * l) % 1024)
-        return set_err(ctx, GS_ERR_UNSUPPORTED, "norm_type 1 needs window*window to be a multiple of 1024 (window %d)", l);
+// Template preparation of a checked call (window l).
+static int prepare_templates(gs_ctx* ctx, const gs_params* p, const float* host_templates, int n, int tx, int ty,
+                             const gs_ctf* first_ctf, int l) {
     ctx->have_tmpl = false;
     ctx->have_units = false;
     ctx->p = *p;
@@ -1162,6 +1175,22 @@ int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_template
     cudaStreamSynchronize(ctx->stream);
     if (st == GS_OK) ctx->have_tmpl = true;
     return st;
+}
+
+int gs_set_templates(gs_ctx* ctx, const gs_params* p, const float* host_templates, int n, int tx, int ty,
+                     const gs_ctf* first_ctf) {
+    if (!ctx || !p || !host_templates || !first_ctf || n <= 0 || tx <= 0 || ty <= 0)
+        return set_err(ctx, GS_ERR_ARG, "null pointer or empty template stack");
+    TRY(validate_params(ctx, p));
+    if (n > 2 * 65535) return set_err(ctx, GS_ERR_UNSUPPORTED, "at most %d templates", 2 * 65535);
+    CK(cudaSetDevice(ctx->device));
+    const int l = adjust_padding(p->window_size, tx, ty);
+    if (l % 2) return set_err(ctx, GS_ERR_UNSUPPORTED, "window size %d must be even", l);
+    // norm_type 1 reduces 1024-element blocks of the flat l x l map
+    // (GPU_func.cu:711-745 with the launch at main.cu:798)
+    if (p->norm_type == 1 && ((long long)l * l) % 1024)
+        return set_err(ctx, GS_ERR_UNSUPPORTED, "norm_type 1 needs window*window to be a multiple of 1024 (window %d)", l);
+    return with_room(ctx, [&](bool) { return prepare_templates(ctx, p, host_templates, n, tx, ty, first_ctf, l); });
 }
 
 int gs_get_geometry(gs_ctx* ctx, int nx, int ny, gs_geometry* out) {
@@ -2170,7 +2199,7 @@ static int compact_picks(gs_ctx* ctx, const MicPlan& mp, int NW, const std::vect
 // windows of all micrographs share one window-spectrum array and every angle's
 // template-pair spectra; each micrograph's picks come out in the reference's
 // order, micrographs in the given order.
-static int search_many(gs_ctx* ctx, std::vector<MicPlan>& mics, std::vector<std::vector<gs_pick>>* res) {
+static int search_once(gs_ctx* ctx, std::vector<MicPlan>& mics, bool prefetch, std::vector<std::vector<gs_pick>>* res) {
     const gs_params& p = ctx->p;
     const int l = ctx->l;
     const long long l2 = (long long)l * l;
@@ -2202,7 +2231,7 @@ static int search_many(gs_ctx* ctx, std::vector<MicPlan>& mics, std::vector<std:
     // micrograph preparation; whatever path the search takes, the main
     // stream's later work is ordered after them
     int prefetched = 0;
-    TRY(prefetch_pair_spectra(ctx, NW, angles, &prefetched));
+    if (prefetch) TRY(prefetch_pair_spectra(ctx, NW, angles, &prefetched));
     struct SideJoin {
         gs_ctx* ctx;
         const int* on;
@@ -2240,6 +2269,10 @@ static int search_many(gs_ctx* ctx, std::vector<MicPlan>& mics, std::vector<std:
     ctx->counters.searches += 1;
     ctx->counters.units += (unsigned long long)total_units;
     return GS_OK;
+}
+
+static int search_many(gs_ctx* ctx, std::vector<MicPlan>& mics, std::vector<std::vector<gs_pick>>* res) {
+    return with_room(ctx, [&](bool again) { return search_once(ctx, mics, !again, res); });
 }
 
 // Per-pixel maximum of cc / sigma over (angle, template) for micrograph `mic`
@@ -2465,7 +2498,7 @@ int gs_get_pixel_max(gs_ctx* ctx, int micrograph, float thres, float* value, int
     if (micrograph < 0 || micrograph >= (int)ctx->last_mics.size())
         return set_err(ctx, GS_ERR_ARG, "micrograph %d not in the last search", micrograph);
     CK(cudaSetDevice(ctx->device));
-    return pixel_max_impl(ctx, micrograph, thres, value, template_index, angle_index);
+    return with_room(ctx, [&](bool) { return pixel_max_impl(ctx, micrograph, thres, value, template_index, angle_index); });
 }
 
 void gs_picks_free(gs_pick* p) { free(p); }
@@ -2527,7 +2560,9 @@ int gs_score_grad(gs_ctx* ctx, const gs_refine_pick* picks, int n, int with_grad
     if (n == 0) return GS_OK;
     if (!ctx->have_tmpl) return set_err(ctx, GS_ERR_STATE, "gs_set_templates must come first");
     CK(cudaSetDevice(ctx->device));
-    return score_grad_impl(ctx, picks, n, with_gradient != 0, out, with_gradient ? template_gradients : nullptr);
+    return with_room(ctx, [&](bool) {
+        return score_grad_impl(ctx, picks, n, with_gradient != 0, out, with_gradient ? template_gradients : nullptr);
+    });
 }
 
 int gs_refine(gs_ctx* ctx, gs_refine_pick* picks, int n, int steps, gs_refine_result* out) {
@@ -2536,7 +2571,7 @@ int gs_refine(gs_ctx* ctx, gs_refine_pick* picks, int n, int steps, gs_refine_re
     if (n == 0) return GS_OK;
     if (!ctx->have_tmpl) return set_err(ctx, GS_ERR_STATE, "gs_set_templates must come first");
     CK(cudaSetDevice(ctx->device));
-    return refine_impl(ctx, picks, n, steps, out);
+    return with_room(ctx, [&](bool) { return refine_impl(ctx, picks, n, steps, out); });
 }
 
 int gs_get_tuning(gs_ctx* ctx, int* out, int n) {
