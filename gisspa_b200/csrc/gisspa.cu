@@ -1844,8 +1844,8 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
     }
     CorrTuning tune;
     TRY(default_tuning(ctx, tc2, &tune));
-    // a launch takes fewer angles, and smaller chunks, where the device has no
-    // memory for them
+    // a launch takes fewer angles, smaller chunks and a shorter ring where the device
+    // has no memory for them
     // (the frees wait for whatever still uses the buffers)
     auto buffers = [&]() -> int {
         TRY(ensure(ctx, ctx->units, sizeof(UnitOut) * std::max<long long>(1, total_units)));
@@ -1863,8 +1863,18 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         }
         return ensure(ctx, ctx->scratch, sizeof(float2) * l2 * (chunked ? std::min<long long>(chunk, (long long)nu * A) : Np));
     };
-    for (int st; (st = buffers()) != GS_OK; A = (A + 1) / 2, chunk = (chunk + 1) / 2) {
-        if (st != GS_ERR_OOM || (A == 1 && !(chunked && chunk > 1))) return st;
+    for (int st; (st = buffers()) != GS_OK;) {
+        if (st != GS_ERR_OOM) return st;
+        if (A > 1 || (chunked && chunk > 1)) {
+            A = (A + 1) / 2;
+            chunk = (chunk + 1) / 2;
+        } else if (persistent && p.precision == GS_PREC_FP32 && !ctx->corr_ring_set && tune.slots > 4) {
+            // fewer maps in flight, as the allocation-free call does it
+            tune.slots = std::max(4, (tune.slots + 1) / 2);
+            tune.lag = std::max(1, std::min(tune.lag, 5 * tune.slots / 11));
+        } else {
+            return st;
+        }
         if (prefetched) CK(cudaStreamWaitEvent(ctx->stream, ctx->side_ev[1], 0));
         prefetched = 0;
         for (DBuf* b : {&ctx->tspec, &ctx->pacc, &ctx->dep_counters, &ctx->scratch}) free_buf(*b);

@@ -49,3 +49,28 @@ def test_room_for_the_micrograph(before, free_mb):
     assert len(units[0]) == 72 * 24 * 80 * (2 if before else 1)
     # sums of squares are added in any order
     np.testing.assert_allclose(units[1]["score"], units[0]["score"], rtol=1e-5)
+
+
+# one template and one window: a search needs some 6 and 20 MB, the default rings have 51 and 72 MB of maps
+@pytest.mark.parametrize("l,free_mb", [(320, 30), (640, 50)])
+def test_room_for_the_ring(l, free_mb):
+    import torch
+    kw = dict(apix=1.0, phi_step=30.0, kk=3.0, energy=300.0, cs=2.7, highres=8.0, lowres=100.0, d_m=20.0, thres=0.0,
+              phase_flip=1, overlap=0)
+    ds = synth.make_dataset(6, nx=l, ny=l, n_templates=1, tsize=24, n_particles=2, snr=0.3, n_blobs=40, ball_radius=7.0,
+                            phistep=30.0, diameter=20.0, window=l, overlap=0, defocus=(1.0, 2.0), astig_A=300.0)
+    m = ds.micrographs[0]
+    ctf = (m.defocus, m.dfdiff, m.dfang)
+    units = []
+    for short in (False, True):
+        held = None
+        with G.Context(0) as ctx:
+            ctx.set_templates(G.default_params(window_size=l, **kw), ds.templates, ctf)
+            if short:
+                torch.cuda.empty_cache()
+                held = torch.empty(torch.cuda.mem_get_info(0)[0] - (free_mb << 20), dtype=torch.uint8, device="cuda:0")
+            ctx.search(m.image, ctf)
+            units.append(ctx.units())
+        del held
+        torch.cuda.empty_cache()
+    np.testing.assert_allclose(units[1]["score"], units[0]["score"], rtol=1e-5)
