@@ -196,7 +196,8 @@ extern "C" int gs_merge_duplicates(int device, const gs_merge_item* items, size_
     const size_t b_it = sizeof(gs_merge_item) * n, b_ll = sizeof(long long) * n, b_cnt = (sizeof(unsigned) * n + 7) / 8 * 8;
     const size_t b_dev = sizeof(MergeDev) * n, b_in = b_it + b_dev;
     const size_t head = b_in + 2 * b_ll + 8 + b_cnt;
-    unsigned long long cap = 32ull * n + 1024, total = 0;
+    constexpr unsigned long long kFewPairs = 1024;
+    unsigned long long cap = 32ull * n + kFewPairs, total = 0;
     std::vector<unsigned> cnt(n), pairs;
     std::vector<unsigned long long> off(n);
     int st;
@@ -206,6 +207,12 @@ extern "C" int gs_merge_duplicates(int device, const gs_merge_item* items, size_
         DevMem mem;
         if (cudaMalloc(&mem.p, head + sizeof(unsigned) * cap) != cudaSuccess) {
             cudaGetLastError();
+            mem.p = nullptr;
+            // not counted yet: without room for pairs first, then for as many as there are
+            if (!total && cap > kFewPairs) {
+                cap = kFewPairs;
+                continue;
+            }
             return GS_ERR_OOM;
         }
         char* base = (char*)mem.p;

@@ -74,3 +74,22 @@ def test_room_for_the_ring(l, free_mb):
         del held
         torch.cuda.empty_cache()
     np.testing.assert_allclose(units[1]["score"], units[0]["score"], rtol=1e-5)
+
+
+def test_room_for_merging():
+    import torch
+    n = 1000000  # 148 MB without room for pairs, 284 MB with the room that is taken first
+    r = np.random.default_rng(4)
+    items = np.zeros(n, G.MERGE_ITEM_DTYPE)
+    items["group"] = np.arange(n) // 4
+    for c in ("x", "y", "alt", "az", "phi"):
+        items[c] = r.uniform(0, 20, n)
+    items["score"] = r.uniform(7, 12, n)
+    want = G.merge_duplicates(items, 10.0, 12.0)
+    assert 0.1 * n < want.sum() < 0.95 * n
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info(0)[0] - (200 << 20), dtype=torch.uint8, device="cuda:0")
+    got = G.merge_duplicates(items, 10.0, 12.0)
+    del held
+    torch.cuda.empty_cache()
+    assert np.array_equal(got, want)
