@@ -51,6 +51,9 @@
 // tile only the end-of-item barrier, as each warp owns two whole rows.
 #pragma once
 
+#include <algorithm>
+#include <vector>
+
 #include "fastfft.cuh"
 
 namespace gs {
@@ -94,6 +97,27 @@ inline void corr_border(CorrArgs* a, float d_m, int l) {
 // Lag of the column tiles in units for `ctas` resident CTAs and units of `tiles`
 // tiles a pass: 2.5 times as many items as CTAs.
 inline int corr_lag(int ctas, int tiles) { return (5 * ctas + 4 * tiles - 1) / (4 * tiles); }
+
+// Slots and lags that the autotuner tries around a window's own ring: fixed ones
+// where the ring is (`fixed`: windows 512, 720 and 768), else in proportion, since
+// rings that go by the resident CTAs have up to some hundred slots.
+struct CorrRingTrials {
+    std::vector<int> slots, lags;
+};
+inline CorrRingTrials corr_ring_trials(int slots, int lag, bool fixed) {
+    CorrRingTrials t;
+    if (fixed) {
+        t.slots = {8, 12, 16, 24, 32};
+        t.lags = {2, 4, 6, 10};
+        return t;
+    }
+    for (int f : {5, 7, 14, 20}) {
+        t.slots.push_back(std::max(2, slots * f / 10));
+        t.lags.push_back(std::max(1, lag * f / 10));
+    }
+    return t;
+}
+inline int corr_ring_most(int slots, bool fixed) { return fixed ? std::max(32, slots) : 2 * slots; }
 
 // What the column tiles do with the maps: score them; add them into the
 // per-pixel moments; z-score them and keep every 1024-element block's maximum.

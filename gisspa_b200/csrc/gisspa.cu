@@ -1555,10 +1555,10 @@ static int autotune(gs_ctx* ctx, const float2* W, const float2* TS, int NW, Corr
     }
     const int nu_full = Np * NW;
     const int nu = std::min(nu_full, 8192);
-    std::vector<int> slots_c = {8, 12, 16, 24, 32}, lag_c = {2, 4, 6, 10}, wb_c = {1, 2, 4, 8}, ctas_c = {0, 1};
-    std::vector<int> tile_c = {16, 8};
     CorrTuning cur = *best;  // the defaults for this window and precision
     cur.ctas = 0;
+    const CorrRingTrials ring = corr_ring_trials(cur.slots, cur.lag, fast_ok(ctx, ctx->l));
+    const std::vector<int>&slots_c = ring.slots, &lag_c = ring.lags, wb_c = {1, 2, 4, 8}, ctas_c = {0, 1}, tile_c = {16, 8};
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
@@ -1859,7 +1859,7 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         }
         if (persistent) {
             TRY(ensure(ctx, ctx->dep_counters, sizeof(int) * (2 * (size_t)nu * A + 4)));
-            return ensure(ctx, ctx->scratch, sizeof(float2) * l2 * (ctx->autotune ? std::max(32, tune.slots) : tune.slots));
+            return ensure(ctx, ctx->scratch, sizeof(float2) * l2 * (ctx->autotune ? corr_ring_most(tune.slots, fast_ok(ctx, l)) : tune.slots));
         }
         return ensure(ctx, ctx->scratch, sizeof(float2) * l2 * (chunked ? std::min<long long>(chunk, (long long)nu * A) : Np));
     };

@@ -1,6 +1,7 @@
 // Host parts of gisspa_b200/csrc/corr.cuh.
 //   claims: the items of the largest launch that is allowed, and the claims behind
 //   its last item, at every window
+//   rings: what the autotuner tries lies around the ring that a window's rule gives
 //   border: the masked indices at every window and particle diameter, to infinity
 #include <cmath>
 #include <cstdio>
@@ -46,6 +47,28 @@ static int check_windows() {
     }
 }
 
+static int check_rings() {
+    int bad = 0;
+    for (int l = 96; l <= 752; l += 16) {
+        const int tile = l <= 576 ? 8 : 16, tiles = l / tile;
+        for (int threads : {512, 768, 1024}) {
+            const int lag = corr_lag(148 * threads / (16 * tile), tiles), slots = (11 * lag + 4) / 5;
+            const CorrRingTrials t = corr_ring_trials(slots, lag, false);
+            int below = 0, above = 0, fit = 0;
+            for (int s : t.slots) {
+                below += s < slots && s > lag;
+                above += s > slots;
+                if (s < 2 || s > corr_ring_most(slots, false)) bad = 1;
+            }
+            for (int g : t.lags) fit += g >= 1 && g < slots && g != lag;
+            if (bad || !below || !above || fit < 3) { printf("window %d: slots %d, lag %d\n", l, slots, lag); return 1; }
+        }
+    }
+    const CorrRingTrials t = corr_ring_trials(16, 6, true);
+    for (int s : t.slots) bad |= s > corr_ring_most(16, true);
+    return bad;
+}
+
 static int check_border() {
     int bad = 0;
     for (int l = 96; l <= 768; l += 16)
@@ -70,6 +93,7 @@ int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     int bad = 1;
     if (what == "claims") bad = check_windows<6>();
+    if (what == "rings") bad = check_rings();
     if (what == "border") bad = check_border();
     printf(bad ? "FAIL\n" : "OK\n");
     return bad;

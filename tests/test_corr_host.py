@@ -20,7 +20,7 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("what", ["claims", "border"])
+@pytest.mark.parametrize("what", ["claims", "border", "rings"])
 def test_corr_host(exe, what):
     r = subprocess.run([exe, what], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
