@@ -2345,6 +2345,7 @@ static int pixel_max_impl(gs_ctx* ctx, int mic, float thres, float* value, int* 
             epi.L = l;
             epi.ntmpl = N;
             epi.nx = mg.nx;
+            epi.ny = mg.ny;
             epi.offx = mg.offx[wl % bx];
             epi.offy = mg.offy[wl / bx];
             epi.idx0 = (unsigned int)a * (unsigned int)N;

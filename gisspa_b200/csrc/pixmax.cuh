@@ -56,13 +56,20 @@ struct IoPass1Sel {
     __device__ void finish(double*, int, int) const {}
 };
 
+// Micrograph pixel of map position (X, Y) of the window at (offx, offy), or -1: a
+// window that is larger than the micrograph reaches beyond it.
+__host__ __device__ __forceinline__ long long pixel_of_map(int X, int Y, int offx, int offy, int nx, int ny) {
+    const int x = offx + X, y = offy + Y;
+    return x < nx && y < ny ? (long long)y * nx + x : -1;
+}
+
 // Column-pass epilogue: value (x, y) of the map of scratch slot `img` (pair
 // pairs[img], real part template 2p, imaginary part 2p + 1).
 struct PixelMaxEpi {
     unsigned long long* keys;  // micrograph, ny x nx
     const UnitOut* out;        // this (angle, window): ntmpl results of the search
     const int* pairs;
-    int L, ntmpl, nx, offx, offy;
+    int L, ntmpl, nx, ny, offx, offy;
     unsigned int idx0;         // angle index * ntmpl
     float q_lo, q_hi, thres, sgn;
     __device__ __forceinline__ void put(int img, int x, int y, float2 val) const {
@@ -71,6 +78,8 @@ struct PixelMaxEpi {
         int Y = y + h; if (Y >= L) Y -= L;
         // the border the score's maximum leaves out (GPU_func.cu:681)
         if ((float)X < q_lo || (float)X > q_hi || (float)Y < q_lo || (float)Y > q_hi) return;
+        const long long at = pixel_of_map(X, Y, offx, offy, nx, ny);
+        if (at < 0) return;
         const int pair = __ldg(pairs + img);
         for (int q = 0; q < 2; ++q) {
             const int J = 2 * pair + q;
@@ -81,7 +90,7 @@ struct PixelMaxEpi {
             if (!(z >= thres)) continue;
             const unsigned long long key =
                 ((unsigned long long)float_order(z) << 32) | (unsigned int)(~(idx0 + (unsigned int)J));
-            atomicMax(keys + (long long)(offy + Y) * nx + offx + X, key);
+            atomicMax(keys + at, key);
         }
     }
 };

@@ -659,6 +659,8 @@ def search(micrograph: np.ndarray, templates_raw: np.ndarray, p: Params,
                         if not (np.isfinite(st.score[J]) and st.sd[J] > 0):
                             continue
                         z = np.where(inner, cc[J] / st.sd[J], -np.inf)
+                        # a window larger than the micrograph reaches beyond it
+                        z = z[:ny - offy[j], :nx - offx[i]]
                         sub_v = pix_v[offy[j]:offy[j] + l, offx[i]:offx[i] + l]
                         win = (z >= pixel_thres) & (z > sub_v)
                         sub_v[win] = z[win]
