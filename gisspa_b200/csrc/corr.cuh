@@ -1,5 +1,5 @@
 // Persistent correlation kernel: the row pass and the column pass of every
-// (window, template pair) unit of one in-plane angle in a single launch.
+// (window, template pair) unit of one or more in-plane angles in a single launch.
 //
 // Work items, claimed in increasing order from one atomic counter (lag <= Nu):
 //   the row tiles of units 0 .. lag - 1, then for every later unit s
@@ -161,8 +161,8 @@ constexpr int inv_mod(int b, int m) {
 }
 
 // Tile geometry: V vectors per tile (16 or 8), 16 V threads per CTA (step 2
-// has one (vector, k1) task per thread), 512 / (16 V) CTAs per SM.  A pass of
-// one unit is T = L / V tiles.
+// has one (vector, k1) task per thread), kThreadsPerSm / (16 V) CTAs per SM (more
+// where registers allow).  A pass of one unit is T = L / V tiles.
 template <int N2, int V_>
 struct CorrCfg {
     static constexpr int L = 16 * N2;

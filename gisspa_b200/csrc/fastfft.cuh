@@ -212,14 +212,13 @@ struct F16RealOut {
 // on load (see IoPairNorm), in place, from image row row0 on (a multiple of 16).
 struct F16PairNorm {
     float2* data;
-    const float4* coef;
+    const float2* coef;
     int L;
     long long L2;
     int row0;
     __device__ float2 load(int img, int v, int k) const {
-        const float4 c = coef[img];
-        const float2 z = data[f16_addr<false>(L, L2, img, v + row0, k)];
-        return make_float2(z.x * c.y, -z.y * c.w);
+        const float2 c = coef[img], z = data[f16_addr<false>(L, L2, img, v + row0, k)];
+        return make_float2(z.x * c.x, -z.y * c.y);
     }
     __device__ void store(int img, int v, int k, float2 x) const {
         data[f16_addr<false>(L, L2, img, v + row0, k)] = x;

@@ -73,10 +73,6 @@ struct CorrTuningSaved {
     int slots, lag, window_block, ctas, tile;
 };
 
-namespace {
-
-}  // namespace
-
 struct gs_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -520,7 +516,7 @@ static MaskRows mask_rows(float d_m, int l) {
 // Forward transform, times `factor` (the zero frequency times `dc` besides), of
 // nimg images that are zero outside the rows mr, which alone are read; coef as
 // IoPairNorm takes it; pfa: the PfaCols column order.
-static int disc_transform(gs_ctx* ctx, float2* data, const float4* coef, int nimg, MaskRows mr, float factor, float dc,
+static int disc_transform(gs_ctx* ctx, float2* data, const float2* coef, int nimg, MaskRows mr, float factor, float dc,
                           bool pfa) {
     const int l = ctx->l;
     const long long l2 = (long long)l * l;
@@ -540,19 +536,17 @@ static int disc_transform(gs_ctx* ctx, float2* data, const float4* coef, int nim
     return run_fft<false>(ctx, l, cols_of(l, l), nimg, IoPairCols{data, factor, mr.row0, mr.row1, dc});
 }
 
-// Template-pair spectra of one in-plane angle (rotate_template + the
-// normalisation and FFT of main.cu:1236-1249): TS[p] = FFT(t_2p - i t_2p+1) / l^2
-// with each rotated, masked template mean/variance normalised.
-// pfa: store the spectra in the PfaCols column order of the prime-factor
-// correlation kernel (window 720) instead of natural order.
 // (cos, sin) of in-plane angle e (degrees) as the rotation takes them.
 static float2 rotation_cs(float e) {
     const double ang = (double)e * kPiRef / 180.0;
     return make_float2((float)cos(ang), (float)sin(ang));
 }
-// The spectra of `nang` consecutive angles in one pass (angle z's at
-// TS + z Np l^2; pstats and coef hold nang angles): cs = their (cos, sin) on
-// the device, or nullptr for the single angle e.
+// Template-pair spectra (rotate_template + the normalisation and FFT of
+// main.cu:1236-1249): TS[p] = FFT(t_2p - i t_2p+1) / l^2 with each rotated, masked
+// template mean/variance normalised; of `nang` consecutive angles in one pass (angle
+// z's at TS + z Np l^2; pstats and coef hold nang angles): cs = their (cos, sin)
+// on the device, or nullptr for the single angle e.  pfa: in the PfaCols column
+// order of the prime-factor correlation kernel (odd N2) instead of natural order.
 static int pair_spectra_n(gs_ctx* ctx, float e, const float2* cs, int nang, float2* TS, bool pfa) {
     const int l = ctx->l, N = ctx->ntmpl, Np = (N + 1) / 2;
     const long long l2 = (long long)l * l;
@@ -565,10 +559,10 @@ static int pair_spectra_n(gs_ctx* ctx, float e, const float2* cs, int nang, floa
                                               P<double>(ctx->pstats));
     ++ctx->counters.kernel_launches;
     k_pair_coef<<<blocks_for(nimg, 128), 128, 0, ctx->stream>>>(P<double>(ctx->pstats), N, l,
-                                                                P<float4>(ctx->coef), nang);
+                                                                P<float2>(ctx->coef), nang);
     ++ctx->counters.kernel_launches;
     CKL();
-    return disc_transform(ctx, TS, P<float4>(ctx->coef), nimg, mr, (float)(1.0 / (double)l2), 0.0f, pfa);
+    return disc_transform(ctx, TS, P<float2>(ctx->coef), nimg, mr, (float)(1.0 / (double)l2), 0.0f, pfa);
 }
 static int pair_spectra(gs_ctx* ctx, float e, float2* TS, bool pfa = false) {
     return pair_spectra_n(ctx, e, nullptr, 1, TS, pfa);
@@ -590,13 +584,8 @@ static int corr_cols(gs_ctx* ctx, const float2* R, const Epi& epi) {
     return run_fft<true>(ctx, l, cols_of(l, l), Np, IoNorm1<Epi>{R, epi});
 }
 
-// norm_type 1 (pickPartcles_CCG_NORM path, main.cu:1170-1229): sweep 1 sums
-// cc / l^2 and its square per window pixel over all templates and angles
-// (compute_CCG_sum, main.cu:724-749) and turns them into mean and standard
-// deviation (compute_CCG_mean); sweep 2 recomputes every map, z-scores it
-// and reports the maximum of every 1024-element block (main.cu:770-820).
-// Picks come out in the reference's order: angle, window row, window
-// column, template, block.
+// norm_type 1's picks in the reference's order: angle, window row, window column,
+// template, block.
 static void norm1_picks(std::vector<BlockPickDev>& hp, const std::vector<float>& angles, int N, int nw, int bx, int nblk,
                         std::vector<gs_pick>* out) {
     std::sort(hp.begin(), hp.end(), [](const BlockPickDev& a, const BlockPickDev& b) { return a.key < b.key; });
@@ -641,7 +630,12 @@ static int norm1_compact(gs_ctx* ctx, long long nkeys, int nblk, int bx, int by,
     return GS_OK;
 }
 
-// Without the persistent kernel (other windows, GS_OPT_TWO_PASS,
+// norm_type 1 (pickPartcles_CCG_NORM path, main.cu:1170-1229): sweep 1 sums
+// cc / l^2 and its square per window pixel over all templates and angles
+// (compute_CCG_sum, main.cu:724-749) and turns them into mean and standard
+// deviation (compute_CCG_mean); sweep 2 recomputes every map, z-scores it
+// and reports the maximum of every 1024-element block (main.cu:770-820).
+// Here without the persistent kernel (other windows, GS_OPT_TWO_PASS,
 // GS_OPT_GENERIC_FFT): row and column launches per (angle, window).
 static int search_norm1_passes(gs_ctx* ctx, const float2* W, int nx, int ny, const std::vector<int>& offx,
                                const std::vector<int>& offy, const std::vector<float>& angles, float* ms_spec,
@@ -739,7 +733,7 @@ static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool
     const int chunk = (int)std::max<long long>(1, std::min<long long>(std::min(n, 65535), (2ll << 30) / per));
     TRY(ensure(ctx, ctx->rf_pk, sizeof(RefinePickDev) * chunk));
     TRY(ensure(ctx, ctx->rf_acc, sizeof(RefineAcc) * chunk));
-    TRY(ensure(ctx, ctx->rf_scale, (sizeof(double) * 2 + sizeof(float4)) * chunk));
+    TRY(ensure(ctx, ctx->rf_scale, (sizeof(double) * 2 + sizeof(float2)) * chunk));
     TRY(ensure(ctx, ctx->rf_ph, sizeof(double2) * 2 * l * chunk));
     TRY(ensure(ctx, ctx->rf_F1, sizeof(float2) * l2 * chunk));
     TRY(ensure(ctx, ctx->rf_T, sizeof(float) * l2 * chunk));
@@ -780,7 +774,7 @@ static int score_grad_impl(gs_ctx* ctx, const gs_refine_pick* picks, int n, bool
     const float sgn = ((l / 2) % 2 == 0) ? 1.0f : -1.0f;
     RefinePickDev* d_pk = P<RefinePickDev>(ctx->rf_pk);
     RefineAcc* d_acc = P<RefineAcc>(ctx->rf_acc);
-    float4* as_is = P<float4>(ctx->rf_scale);
+    float2* as_is = P<float2>(ctx->rf_scale);
     double* inva = reinterpret_cast<double*>(as_is + chunk);
     double* scale = inva + chunk;                                     // 1 / l^2
     double2* phases = P<double2>(ctx->rf_ph);
@@ -1663,7 +1657,7 @@ static int search_norm1(gs_ctx* ctx, const float2* W, int nx, int ny, const std:
         TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np));
         TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * Np));
         TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N));
-        TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np));
+        TRY(ensure(ctx, ctx->coef, sizeof(float2) * Np));
         return search_norm1_passes(ctx, W, nx, ny, offx, offy, angles, ms_spec, ms_corr, out);
     };
     if (ctx->two_pass || !ops || !ops->corr_moments || !corr_units_fit(l, nu)) return passes();
@@ -1678,7 +1672,7 @@ static int search_norm1(gs_ctx* ctx, const float2* W, int nx, int ny, const std:
     auto buffers = [&]() -> int {
         TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np * A));
         TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N * A));
-        TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np * A));
+        TRY(ensure(ctx, ctx->coef, sizeof(float2) * Np * A));
         TRY(ensure(ctx, ctx->unit_wp, sizeof(int2) * (size_t)nu * A));
         TRY(ensure(ctx, ctx->scratch, sizeof(float2) * l2 * tune.slots));
         TRY(ensure(ctx, ctx->dep_counters, sizeof(int) * (2 * (size_t)nu * A + 4)));
@@ -1745,7 +1739,8 @@ static int search_norm1(gs_ctx* ctx, const float2* W, int nx, int ny, const std:
 
 // The first persistent launch's pair spectra, enqueued on the side stream
 // so that they overlap the micrograph preparation that follows on the main
-// stream (its exact-order statistics keep one SM busy for milliseconds).
+// stream (an upload, and kernels that leave SMs idle: the running sums' last one has
+// two CTAs).
 // *count = angles prefetched, 0 when the correlation tunes first (the tuner
 // times its own pair spectra), has no persistent launch, or norm_type 1.
 // side_ev[1] marks their completion.
@@ -1771,7 +1766,7 @@ static int prefetch_pair_spectra(gs_ctx* ctx, int NW, const std::vector<float>& 
     }
     TRY(ensure(ctx, ctx->tspec, spec_bytes));
     TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N * A));
-    TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np * A));
+    TRY(ensure(ctx, ctx->coef, sizeof(float2) * Np * A));
     TRY(upload_rotations(ctx, angles));
     FftPlan* plan = nullptr;
     TRY(get_plan(ctx, l, &plan));  // created (synchronously) before the side work
@@ -1852,7 +1847,7 @@ static int correlate_all(gs_ctx* ctx, float2* W, int NW, const std::vector<float
         TRY(ensure(ctx, ctx->acc, sizeof(UnitAcc) * N));
         TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np * A));
         TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N * A));
-        TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np * A));
+        TRY(ensure(ctx, ctx->coef, sizeof(float2) * Np * A));
         if (persistent || chunked) {
             TRY(ensure(ctx, ctx->unit_wp, sizeof(int2) * std::max<size_t>(1, (size_t)nu * A)));
             TRY(ensure(ctx, ctx->pacc, sizeof(UnitAcc) * 2 * (size_t)nu * A));
@@ -2311,7 +2306,7 @@ static int pixel_max_impl(gs_ctx* ctx, int mic, float thres, float* value, int* 
     TRY(ensure(ctx, ctx->pix_R, sizeof(float2) * l2 * chunk));
     TRY(ensure(ctx, ctx->tspec, sizeof(float2) * l2 * Np));
     TRY(ensure(ctx, ctx->pstats, sizeof(double) * 2 * N));
-    TRY(ensure(ctx, ctx->coef, sizeof(float4) * Np));
+    TRY(ensure(ctx, ctx->coef, sizeof(float2) * Np));
     CK(cudaMemsetAsync(ctx->pix_keys.p, 0, sizeof(unsigned long long) * npix, ctx->stream));
     unsigned long long* keys = P<unsigned long long>(ctx->pix_keys);
     int* d_pairs = P<int>(ctx->pix_pairs);

@@ -454,12 +454,11 @@ static __global__ void __launch_bounds__(256) k_pair_rotate(const float* __restr
     }
 }
 
-// Per-template (mean, 1/sd) over the full frame; mean subtraction skipped if
-// the mean is 0 and scaling skipped if the variance is 0, as in
-// substract_by_mean / divided_by_var (GPU_func.cu:424-443, main.cu:696-707).
-// `nang` angles one after the other: pair p of angle z at coef[z Np + p],
-// from stats + 2 z ntmpl.
-static __global__ void k_pair_coef(const double* __restrict__ stats, int ntmpl, int l, float4* __restrict__ coef,
+// 1/sd over the full frame of a pair's two templates; scaling skipped if the
+// variance is 0, as in divided_by_var (GPU_func.cu:424-443, main.cu:696-707).  (The
+// mean is taken off with the zero frequency, see IoPairNorm.)  `nang` angles one
+// after the other: pair p of angle z at coef[z Np + p], from stats + 2 z ntmpl.
+static __global__ void k_pair_coef(const double* __restrict__ stats, int ntmpl, int l, float2* __restrict__ coef,
                             int nang) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int np = (ntmpl + 1) / 2;
@@ -468,16 +467,15 @@ static __global__ void k_pair_coef(const double* __restrict__ stats, int ntmpl, 
     stats += (size_t)z * 2 * ntmpl;
     coef += (size_t)z * np;
     const double n = (double)l * l;
-    float c[4] = {0.0f, 1.0f, 0.0f, 0.0f};
+    float c[2] = {1.0f, 0.0f};
     for (int k = 0; k < 2; ++k) {
         const int J = 2 * p + k;
         if (J >= ntmpl) break;
         const double mean = stats[2 * J] / n;
         const double var = stats[2 * J + 1] / n - mean * mean;
-        c[2 * k] = (float)mean;
-        c[2 * k + 1] = var != 0.0 ? (float)(1.0 / sqrt(var)) : 1.0f;
+        c[k] = var != 0.0 ? (float)(1.0 / sqrt(var)) : 1.0f;
     }
-    coef[p] = make_float4(c[0], c[1], c[2], c[3]);
+    coef[p] = make_float2(c[0], c[1]);
 }
 
 // Rows of the pair spectra: z = t1n - i t2n, where tkn is template k normalised
@@ -488,11 +486,10 @@ static __global__ void k_pair_coef(const double* __restrict__ stats, int ntmpl, 
 // leave the rows outside the mask's disc alone.
 struct IoPairNorm {
     float2* data;  // from the first row of the pass on
-    const float4* coef;
+    const float2* coef;
     __device__ float2 load(int img, int, int, long long a) const {
-        const float4 c = coef[img];
-        const float2 z = data[a];
-        return make_float2(z.x * c.y, -z.y * c.w);
+        const float2 c = coef[img], z = data[a];
+        return make_float2(z.x * c.x, -z.y * c.y);
     }
     __device__ void store(int, int, int, long long a, float2 v) const { data[a] = v; }
     __device__ void finish(double*, int, int) const {}

@@ -170,11 +170,11 @@ static __global__ void __launch_bounds__(256) k_ref_weight(const float2* __restr
 // Per-pick factors of the transforms: 1 / a for t = Re IFFT(F1 / a), and the pair
 // coefficient (IoPairNorm) of a map that is to be taken as it is.
 static __global__ void k_ref_factors(const RefineAcc* __restrict__ acc, int n, double cnt, double* __restrict__ inva,
-                                     float4* __restrict__ as_is) {
+                                     float2* __restrict__ as_is) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     inva[p] = cnt / sqrt(acc[p].asum);
-    as_is[p] = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
+    as_is[p] = make_float2(1.0f, 0.0f);
 }
 
 // Source coordinates of rotate_subIMG for output pixel (i, j) and angle e.
