@@ -10,13 +10,18 @@
 // (the detectors' 3838 = 2 19 101, 3710 = 2 5 7 53 and 4092 = 4 3 11 31) with half the
 // multiply-adds of a plain DFT and both operands of most of them in registers.
 //
-// Bound by latency and issue: rows of 5760 values take two CTAs of 256
-// threads to an SM.  The stage code is one function per direction, called by every IO
-// variant of the kernel, so that its radices are compiled once.
+// Bound by latency and issue: three CTAs of 256 threads to an SM (80 registers;
+// rows of 5760 values would leave room for four), issue 60 to 63 % over the units of
+// window 300 and 36 % where a micrograph's rows make 570 CTAs.  The stage code is one
+// function per direction, called by every IO variant of the kernel, so that its
+// radices are compiled once.  Twiddles are table entries: products of two saved 2 %
+// of a search at window 300 and cost up to 6 % more rounding error (512: 1.06e-7
+// rms, 1.00e-7 with entries; the mixed-radix kernel 1.00e-7).
 // Without batching, a thread waits for one load at a time (long scoreboard 8 of
 // 14 stalled cycles per issue at length 300, 27 % issue): with four in flight and
-// 32-bit offsets the 4320 units of 300 x 300 take 5.4 ms instead of 7.5, the
-// preparation of a 4096 x 4096 micrograph 5.0 instead of 6.4 (eight in flight: the same).
+// 32-bit offsets the 4320 units of 300 x 300 take 5.4 ms instead of 7.5 (5.1 now
+// with larger chunks), the preparation of a 4096 x 4096 micrograph 5.0 instead of 6.4
+// (eight in flight: the same).
 #pragma once
 
 #include "regfft.cuh"

@@ -4,8 +4,9 @@
 // taken pixel by pixel (main.cu:530-535); float addition is not associative,
 // so the order is part of the result.  One dependent addition per pixel costs
 // 4 cycles of latency: 73.4 ms for 5760 x 4092 pixels when a single thread does
-// it, with the rest of the GPU waiting; this way it is 1.7 ms (0.5 where the mean
-// is not 0).
+// it, with the rest of the GPU waiting; this way it is 0.7 ms at a mean of 5 and a
+// deviation of 1.2, 1.4 to 2.3 for noise around zero, 18 at a mean of 100 (see
+// k_seq_apply).
 //
 // While the running sum s stays inside one binade [2^e, 2^(e+1)) it is k u with
 // u = 2^(e-23) and an integer k, and rounding to nearest even makes adding q
@@ -157,8 +158,10 @@ __host__ __device__ __forceinline__ bool seq_apply(float& s, unsigned binade, co
 //   shared memory and done 512 terms at a time by one warp: by a run where that
 //   applies, term by term (4 cycles each) where it does not.
 // The last kernel is what is left: its time goes with the number of blocks in
-// which the sum passes a power of two, 12 of 1438 for a mean that is not 0 and
-// 136 for 5760 x 4092 pixels of coloured noise around 0.
+// which the sum passes a power of two, 12 of 1438 for a mean of a few deviations and
+// 136 for 5760 x 4092 pixels of coloured noise around 0, and in which the float sum
+// has drifted into another binade than the exact one: most of them for a mean of a
+// hundred deviations, where all terms of a binade round the same way.
 constexpr int kSeqThreads = 1024;
 constexpr int kSeqTerms = 16;  // per thread
 constexpr int kSeqBlock = kSeqThreads * kSeqTerms;
