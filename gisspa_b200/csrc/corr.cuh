@@ -33,9 +33,11 @@
 // later, so the earliest unpublished item can always proceed.  Every wait is
 // bounded; a wait that gives up raises the error flag (reported as
 // GS_ERR_TIMEOUT) and the item still completes and is published, so no other
-// CTA is left waiting on it.  Units scored once the flag is up get NaN: those whose
-// maps the wait was for, and the launch's later ones (gs_correlate_window_noalloc
-// does not wait for its launches and has no other way to tell).
+// CTA is left waiting on it.  The units whose maps the wait was for score NaN: it
+// adds NaN to their sums (gs_correlate_window_noalloc does not wait for its launches
+// and has no other way to tell).  That part of a wait is a call of its own: within
+// the loop it cost 1.5 % at windows 128 and 512, and looking at the flag where a
+// unit is scored 0.4 % at 720.
 //
 // Memory ordering: producers store the maps bypassing L1 (st.global with an
 // L2 cache hint) and add their accumulator atomics; the CTA barrier that ends
@@ -130,27 +132,18 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
 }
 
 // The calling thread waits until *p >= target (bounded: about a second or
-// more, then it flags the error and gives up).  A barrier must follow before
-// other threads rely on the condition.
-__device__ __forceinline__ void wait_counter(const int* p, int target, int* error) {
-    if (ld_acquire_gpu(p) >= target) return;
+// more, then it flags the error and gives up: false).  A barrier must follow before
+// other threads rely on the condition.  (Its caller has looked; looking once more
+// before sleeping is worth 1.3 % at window 720.)
+__device__ __forceinline__ bool wait_counter(const int* p, int target, int* error) {
+    if (ld_acquire_gpu(p) >= target) return true;
     bool ok = false;
     for (int it = 0; it < (1 << 22) && !ok; ++it) {
         __nanosleep(256);
         ok = ld_acquire_gpu(p) >= target;
     }
-    if (!ok) {
-        atomicExch(error, 1);
-        __threadfence();  // the flag before anything the item overwrites too early
-    }
-}
-
-// The calling warp waits until *p >= target: lane 0 spins (bounded, about a
-// second or more, then flags the error and gives up) and __syncwarp()
-// extends its acquire to the warp.  Every lane must call it.
-__device__ __forceinline__ void wait_counter_warp(const int* p, int target, int* error) {
-    if ((threadIdx.x & 31) == 0) wait_counter(p, target, error);
-    __syncwarp();
+    if (!ok) atomicExch(error, 1);
+    return ok;
 }
 
 // b^-1 mod m for gcd(b, m) = 1 (compile time, m small)
@@ -541,13 +534,32 @@ __host__ __device__ __forceinline__ CorrItem corr_item(const CorrArgs& a, int it
     return CorrItem{a.nu - a.lag + c / T, c % T, false};
 }
 
-// Each warp waits for what an item depends on before working on it: a row
-// tile for its slot's previous unit's column tiles, a column tile for its
-// unit's row tiles.
-template <int T>
+// The rest of a wait whose counter was not there at once.  Where it gives up, units u
+// and v (v < 0: none) are scored NaN.
+static __device__ __noinline__ void corr_wait_slow(const int* p, int target, int* error, UnitAcc* acc, int u, int v) {
+    if (wait_counter(p, target, error) || !acc) return;
+    for (int q = 0; q < 2; ++q) {
+        atomicAdd(&acc[2 * (long long)u + q].s2, __longlong_as_double(0x7ff8000000000000ll));
+        if (v >= 0) atomicAdd(&acc[2 * (long long)v + q].s2, __longlong_as_double(0x7ff8000000000000ll));
+    }
+    __threadfence();  // before anything the item overwrites too early
+}
+
+// Each warp waits for what an item depends on before working on it (lane 0 looks,
+// __syncwarp() extends its acquire to the warp): a row tile for its slot's previous
+// unit's column tiles, a column tile for its unit's row tiles.
+template <int T, CorrEpi kEpi>
 __device__ __forceinline__ void corr_wait_for(const CorrArgs& a, const CorrItem& it) {
-    if (!it.row) wait_counter_warp(a.done_rows + it.u, T, a.error);
-    else if (it.u >= a.S) wait_counter_warp(a.done_cols + (it.u - a.S), T, a.error);
+    UnitAcc* acc = kEpi == kCorrScore ? a.acc : nullptr;
+    if (!it.row) {
+        if ((threadIdx.x & 31) == 0 && ld_acquire_gpu(a.done_rows + it.u) < T)
+            corr_wait_slow(a.done_rows + it.u, T, a.error, acc, it.u, -1);
+        __syncwarp();
+    } else if (it.u >= a.S) {
+        if ((threadIdx.x & 31) == 0 && ld_acquire_gpu(a.done_cols + (it.u - a.S)) < T)
+            corr_wait_slow(a.done_cols + (it.u - a.S), T, a.error, acc, it.u, it.u - a.S);
+        __syncwarp();
+    }
 }
 
 // Count a finished tile; the last count of a unit's column pass computes its
@@ -567,8 +579,6 @@ __device__ __forceinline__ void corr_publish(const CorrArgs& a, const CorrItem& 
     int prev;
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(prev) : "l"(&a.done_cols[u]) : "memory");
     if (prev != F::T - 1) return;
-    const bool gave_up = ld_acquire_gpu(a.error) != 0;
-    const float nan = __int_as_float(0x7fc00000);
     const int2 wp = a.unit_wp[u];
     const UnitAcc* ac = a.acc + 2 * (long long)u;
     // sum of the map c1 + i c2 = L^2 S(0, 0), S = W conj(P)
@@ -585,7 +595,7 @@ __device__ __forceinline__ void corr_publish(const CorrArgs& a, const CorrItem& 
         UnitAcc v;
         v.key = __ldcg(&ac[q].key);
         v.s2 = __ldcg(&ac[q].s2);
-        a.out[o] = gave_up ? UnitOut{nan, 0, nan, nan} : unit_score(v, sums[q], F::L);
+        a.out[o] = unit_score(v, sums[q], F::L);
     }
 }
 
@@ -618,7 +628,7 @@ __global__ void __launch_bounds__(CorrCfg<N2, V>::kThreads, CorrCfg<N2, V>::kCta
         // issued before the dependency wait and overlaps it
         const CorrItem it = corr_item<F::T>(a, item);
         const int2 wp = it.row ? __ldg(a.unit_wp + it.u) : make_int2(0, 0);
-        corr_wait_for<F::T>(a, it);
+        corr_wait_for<F::T, kEpi>(a, it);
         if (it.row) corr_row_tile<N2, V>(a, it.u, it.j, tile, twt, wp);
         else corr_col_tile<N2, V, kEpi>(a, it.u, it.j, tile, twt, ymask);
         // the claim made after the previous barrier enters the ring only now,

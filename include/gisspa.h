@@ -423,7 +423,7 @@ void gs_host_free(void* p);
  * (other streams, other host threads) race.  At some windows the work is one
  * kernel whose parts wait for one another, each wait bounded to a second or
  * more; should one give up, where a search returns GS_ERR_TIMEOUT, the units
- * concerned (and possibly later ones of the call) get NaN scores and sigmas. */
+ * concerned get NaN scores and sigmas. */
 #define GS_NOALLOC_SCRATCH_BYTES (32u << 20)
 #define GS_NOALLOC_MAX_WINDOW 2012
 int gs_correlate_window_noalloc(const float* d_window_spectrum, const float* d_pair_spectra,

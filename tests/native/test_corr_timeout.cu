@@ -1,7 +1,8 @@
 // A dependency wait of the persistent correlation that runs out (its counter
 // starts one short, so the tiles of unit 1 that it stands for never reach the
 // target): the launch ends, raises its flag and scores that unit NaN; the units
-// before it, and the same launch with whole counters, score as they should.
+// before it, and the same launch with whole counters, score as they should.  (CTAs
+// that wait hold items of later units, whose waits may give up as well.)
 #include <cmath>
 #include <cstdio>
 #include <random>
