@@ -282,9 +282,9 @@ DTYPES = {"fp32": "f32", "tc-bf16": "bf16 hi+lo split, f32 accumulate",
 
 
 # DRAM bytes (read + write) of one persistent-kernel launch at window 720 per
-# (window, pair) unit, from an ncu capture of 88 windows x 100 pairs (10.63 GB
-# read + 0.22 GB written for 8800 units), scaled by units in the bench
-TRAFFIC_PER_PAIR_UNIT_L720 = (10629210000 + 223908608) / 8800.0
+# (window, pair) unit, from an ncu capture of 88 windows x 100 pairs (10.52 GB
+# read + 0.10 GB written for 8800 units), scaled by units in the bench
+TRAFFIC_PER_PAIR_UNIT_L720 = (10518360000 + 102855680) / 8800.0
 
 
 def compare_picks(base, other, thres: float) -> dict:
