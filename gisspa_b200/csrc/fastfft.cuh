@@ -12,10 +12,11 @@
 // 16 BP + 1) makes both the step-1 writes and the step-2 reads of a
 // half-warp hit distinct banks.  All twiddles inside the register DFTs are
 // compile-time constants (regfft.cuh).  The W_l^{n2 k1} are entries of the
-// twiddle table, put in shared memory by [k1][n2] once per CTA: products of entries,
-// up to three deep, made twice the transform's rounding error of it (window 320
-// 2.0e-7 against 0.94e-7 rms, 512 2.2e-7 against 1.0e-7; the mixed-radix kernel
-// 0.98e-7 and 1.0e-7) for under 1 % of a search's time.
+// twiddle table, put in shared memory by [k1][n2] once per CTA behind the first data
+// loads (before them it cost the allocation-free call at window 512 1.5 of 26 us):
+// products of entries, up to three deep, made twice the transform's rounding error of
+// it (window 320 2.0e-7 against 0.94e-7 rms, 512 2.2e-7 against 1.0e-7; the
+// mixed-radix kernel 0.98e-7 and 1.0e-7).
 #pragma once
 
 #include <type_traits>
@@ -54,19 +55,35 @@ __global__ void __launch_bounds__(256, 2) k_fft16(const float2* __restrict__ tw,
     const int img = blockIdx.y;
     const int v0 = blockIdx.x * F::V;
     float2* twt = sm16 + F::V * F::VP;  // W_l^{n2 k1} at k1 N2 + n2
-    for (int i = threadIdx.x; i < F::L; i += F::kThreads) {
-        const int k1 = i / N2, n2 = i - k1 * N2;
-        twt[i] = twiddle(tw, n2 * k1, kInv);
+    constexpr int kTw = (F::L + F::kThreads - 1) / F::kThreads;
+    float2 w[kTw];
+#pragma unroll
+    for (int t = 0; t < kTw; ++t) {
+        const int i = min((int)threadIdx.x + t * F::kThreads, F::L - 1), k1 = i / N2, n2 = i - k1 * N2;
+        w[t] = twiddle(tw, n2 * k1, kInv);
     }
-    __syncthreads();
-    // ---- step 1: 16-point DFTs down the stride-N2 columns of each vector
-    for (int task = threadIdx.x; task < F::V * N2; task += F::kThreads) {
+    // ---- step 1: 16-point DFTs down the stride-N2 columns of each vector (every
+    // thread goes round once, with or without a task: the table is stored behind the
+    // first task's loads, so that they overlap its own)
+    bool first = true;
+    for (int task = threadIdx.x; first || task < F::V * N2; task += F::kThreads) {
+        const bool on = N2 >= 16 || task < F::V * N2;
         int v, n2;
         if (kCols) { n2 = task / F::V; v = task - n2 * F::V; }
         else { v = task / N2; n2 = task - v * N2; }
         float2 a[16];
+        if (on) {
 #pragma unroll
-        for (int n1 = 0; n1 < 16; ++n1) a[n1] = io.load(img, v0 + v, N2 * n1 + n2);
+            for (int n1 = 0; n1 < 16; ++n1) a[n1] = io.load(img, v0 + v, N2 * n1 + n2);
+        }
+        if (first) {
+#pragma unroll
+            for (int t = 0; t < kTw; ++t)
+                if ((int)threadIdx.x + t * F::kThreads < F::L) twt[threadIdx.x + t * F::kThreads] = w[t];
+            __syncthreads();
+            first = false;
+        }
+        if (!on) break;
         rf::rfft<16, 1, kInv>(a);
         float2* dst = sm16 + v * F::VP + n2;
         rf::static_for<16>([&](auto kc) {
