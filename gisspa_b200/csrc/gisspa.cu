@@ -242,16 +242,21 @@ int get_plan(gs_ctx* ctx, int n, FftPlan** out) {
         const double a = -2.0 * M_PI * (double)k / (double)n;
         tw[k] = make_float2((float)cos(a), (float)sin(a));
     }
-    CK(cudaMalloc(&pl.tw, sizeof(float2) * n));
-    CK(cudaMemcpy(pl.tw, tw.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
-    pl.d.tw = pl.tw;
     bool dense = false;
     if (plan_factors(n, &pl.plan.A, &pl.plan.B, &pl.plan.C, &dense)) {
         pl.plan.n = n;
         pl.plan.dense = dense ? 1 : 0;
-        pl.plan.tw = pl.tw;
+        const int extra = plan_table_size(pl.plan);
+        for (int i = 0; i < extra; ++i) tw.push_back(tw[plan_table_entry(pl.plan, i)]);
     } else {
         pl.plan.A = 0;
+    }
+    CK(cudaMalloc(&pl.tw, sizeof(float2) * tw.size()));
+    CK(cudaMemcpy(pl.tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
+    pl.d.tw = pl.tw;
+    if (pl.plan.A) {
+        pl.plan.tw = pl.tw;
+        plan_tables(&pl.plan, pl.tw + n);
     }
     auto res = ctx->plans.emplace(n, pl);
     *out = &res.first->second;

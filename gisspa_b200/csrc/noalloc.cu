@@ -128,14 +128,17 @@ struct F16Pass2Last : F16Pass2 {
     }
 };
 
-// tw[k] = exp(-2 pi i k / n), zeroed accumulators and counters.
-__global__ void k_noalloc_prepare(float2* tw, int n, UnitAcc* acc, int* count, int nacc) {
+// tw[k] = exp(-2 pi i k / n) and behind them the plan's tables (plan.A = 0: none),
+// zeroed accumulators and counters.
+__global__ void k_noalloc_prepare(float2* tw, int n, const __grid_constant__ PlanDesc plan, UnitAcc* acc, int* count,
+                                  int nacc) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < nacc) {
         acc[k] = UnitAcc{0ull, 0.0, 0.0};
         count[k] = 0;
     }
-    if (k < n) tw[k] = noalloc_twiddle(k, n);
+    const int extra = plan.A ? plan_table_size(plan) : 0;
+    if (k < n + extra) tw[k] = noalloc_twiddle(k < n ? k : plan_table_entry(plan, k - n), n);
 }
 
 // What the persistent kernel starts from: twiddles, zeroed accumulators and
@@ -294,16 +297,19 @@ extern "C" int gs_correlate_window_noalloc(const float* d_window_spectrum, const
         plan.n = l;
         plan.dense = dense ? 1 : 0;
         plan.tw = tw;
+        plan_tables(&plan, tw + l);
     } else {
         plan.A = 0;
     }
+    const int ntw = l + (plan.A ? plan_table_size(plan) : 0);
+    static_assert(3 * GS_NOALLOC_MAX_WINDOW * sizeof(float2) <= kTwBytes, "three tables of a window's length at most");
     for (int p0 = 0; p0 < npairs; p0 += chunk) {
         const int np = std::min(chunk, npairs - p0);
         const int nt = std::min(n_templates - 2 * p0, 2 * np);
         const float2* P = Pall + (size_t)p0 * l2;
         // accumulators start at zero for every chunk
         int* count = reinterpret_cast<int*>(acc + 2 * (size_t)np);
-        k_noalloc_prepare<<<(std::max(l, 2 * np) + 63) / 64, 64, 0, s>>>(tw, l, acc, count, 2 * np);
+        k_noalloc_prepare<<<(std::max(ntw, 2 * np) + 63) / 64, 64, 0, s>>>(tw, l, plan, acc, count, 2 * np);
         if (cudaGetLastError() != cudaSuccess) return GS_ERR_CUDA;
         cudaError_t e;
         if (fast) {

@@ -14,9 +14,11 @@
 // rows of 5760 values would leave room for four), issue 60 to 63 % over the units of
 // window 300 and 36 % where a micrograph's rows make 570 CTAs.  The stage code is one
 // function per direction, called by every IO variant of the kernel, so that its
-// radices are compiled once.  Twiddles are table entries: products of two saved 2 %
-// of a search at window 300 and cost up to 6 % more rounding error (512: 1.06e-7
-// rms, 1.00e-7 with entries; the mixed-radix kernel 1.00e-7).
+// radices are compiled once.  Twiddles are table entries, of each stage's own table in
+// the order that its butterflies read them: from the one table 2 to 5 % of a search
+// at windows without kernels of their own, and products of two entries, as fast,
+// have up to 6 % more rounding error (512: 1.06e-7 rms, 1.00e-7 with entries; the
+// mixed-radix kernel 1.00e-7).
 // Without batching, a thread waits for one load at a time (long scoreboard 8 of
 // 14 stalled cycles per issue at length 300, 27 % issue): with four in flight and
 // 32-bit offsets the 4320 units of 300 x 300 take 5.4 ms instead of 7.5 (5.1 now
@@ -41,7 +43,29 @@ struct PlanDesc {
     int P1 = 0, P2 = 0, VP = 0;      // pitches of k1, k2 and of a vector
     SmallDiv dA, dB, dC, dBC, dAC, dAB, dn, dtile;
     const float2* tw = nullptr;      // exp(-2 pi i k / n)
+    // the same factors in the order of the stages (plan_tables), or none
+    const float2 *twA = nullptr, *twB = nullptr;
 };
+
+// The factors of stage A (W_n^{q e} at q B C + e, e < B C) and of stage B
+// (W_BC^{q e} at q C + e, e < C) behind one another, so that neighbouring butterflies
+// read neighbouring factors: number of them, and the index k of W_n^k that the
+// i-th one is.
+__host__ __device__ inline int plan_table_size(const PlanDesc& d) {
+    return (d.A > 1 && d.B * d.C > 1 ? d.n : 0) + (d.B > 1 && d.C > 1 ? d.B * d.C : 0);
+}
+__host__ __device__ inline int plan_table_entry(const PlanDesc& d, int i) {
+    const int BC = d.B * d.C;
+    if (d.A > 1 && BC > 1) {
+        if (i < d.n) return (i / BC) * (i % BC);  // below n
+        i -= d.n;
+    }
+    return d.A * (i / d.C) * (i % d.C);
+}
+inline void plan_tables(PlanDesc* d, const float2* table) {
+    d->twA = d->A > 1 && d->B * d->C > 1 ? table : nullptr;
+    d->twB = d->B > 1 && d->C > 1 ? table + (d->twA ? d->n : 0) : nullptr;
+}
 
 // Register DFTs of the stages.
 constexpr bool plan_radix(int r) {
@@ -123,11 +147,15 @@ inline bool plan_strides_fit(const PlanDesc& d, const VecGeom& g, int tile) {
 
 // One stage: per vector `d_count.d` butterflies of radix R; butterfly j starts at
 // (j / split) pa + j % split and steps by `stride`.  kTw: output q is multiplied
-// by W_n^{q e}, e = tw_mul * (tw_low ? j % split : j), a table entry each.
+// by W_n^{q e}, e = tw_mul i, i = tw_low ? j % split : j, a table entry each: the
+// stage's own table at q tab_stride + i where there is one, else tw[q e] (these lie
+// in up to q cache lines per warp).
 struct PlanStage {
     SmallDiv count, split;
     int pa, pb, stride, tw_mul;
     bool tw_low;
+    const float2* tab = nullptr;
+    int tab_stride = 0;
 };
 
 template <int R, bool kInv, bool kTw>
@@ -142,11 +170,13 @@ __device__ __forceinline__ void plan_stage(float2* buf, int nv, int VP, const Pl
         for (int q = 0; q < R; ++q) a[q] = p[q * s.stride];
         if constexpr (R > 1) rf::rfft<R, 1, kInv>(a);
         if constexpr (kTw) {
-            const int e = s.tw_mul * (s.tw_low ? lo : j);
+            const int i = s.tw_low ? lo : j;
+            const float2* w = s.tab ? s.tab + i : tw;
+            const int step = s.tab ? s.tab_stride : s.tw_mul * i;
             rf::static_for<R>([&](auto qc) {
                 constexpr int q = decltype(qc)::value;
                 constexpr int r = rf::rpos<R>(q);
-                p[q * s.stride] = q ? cmul(a[r], twiddle(tw, q * e, kInv)) : a[r];
+                p[q * s.stride] = q ? cmul(a[r], twiddle(w, q * step, kInv)) : a[r];
             });
         } else {
             rf::static_for<R>([&](auto qc) {
@@ -237,12 +267,12 @@ template <bool kInv>
 static __device__ __noinline__ float2* plan_block_fft(float2* buf, float2* alt, float2* tab, int nv, const PlanDesc& D) {
     const int BC = D.B * D.C;
     if (D.A > 1) {
-        PlanStage s{D.dBC, D.dC, D.P2, 1, D.P1, 1, false};
+        PlanStage s{D.dBC, D.dC, D.P2, 1, D.P1, 1, false, D.twA, BC};
         if (BC > 1) plan_dispatch<kInv, true>(D.A, buf, nv, D.VP, s, D.tw);
         else plan_dispatch<kInv, false>(D.A, buf, nv, D.VP, s, D.tw);
     }
     if (D.B > 1) {
-        PlanStage s{D.dAC, D.dC, D.P1, 1, D.P2, D.A, true};
+        PlanStage s{D.dAC, D.dC, D.P1, 1, D.P2, D.A, true, D.twB, D.C};
         if (D.C > 1) plan_dispatch<kInv, true>(D.B, buf, nv, D.VP, s, D.tw);
         else plan_dispatch<kInv, false>(D.B, buf, nv, D.VP, s, D.tw);
     }
