@@ -21,7 +21,7 @@
 // mixed-radix kernel 1.00e-7).
 // Without batching, a thread waits for one load at a time (long scoreboard 8 of
 // 14 stalled cycles per issue at length 300, 27 % issue): with four in flight and
-// 32-bit offsets the 4320 units of 300 x 300 take 5.4 ms instead of 7.5 (5.1 now
+// 32-bit offsets the 4320 units of 300 x 300 take 5.4 ms instead of 7.5 (4.9 now
 // with larger chunks), the preparation of a 4096 x 4096 micrograph 5.0 instead of 6.4
 // (eight in flight: the same).
 #pragma once
